@@ -746,7 +746,7 @@ def run_gpu(args, rank: int, world: int, local_rank: int):
     d2h = 5 * mt * 8 + 8 * (10 + 1 + 10 + 10 * 8) + 2 * 10 * 8 * 8 + nsel * rec_bytes
     peak, peak_kind = measured_peaks()
     kms = statistics.mean(pt2_ms)
-    nl = max(1, (r["launches"] - 1) // 3)  # k_pt2 launches per step (one per chunk)
+    nl = max(1, (r["launches"] - 1) // 4)  # k_cand + k_pt2 pairs per step (one per chunk)
     achieved = r["alg_bytes"] / (kms / 1e3) / 1e9
     prof = kernel_profile(args.workload) if args.gen_every == 1 else None
     traffic = prof.get("dram_bytes_per_launch") if prof else None

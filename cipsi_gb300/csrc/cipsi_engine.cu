@@ -44,29 +44,66 @@ __global__ void __launch_bounds__(kReduceThreads) k_reduce(const double* part, i
   }
 }
 
-// k_reduce for every geometry of a batch: block (q, b) sums column q of
-// geometry b's per-unit partials into its reduced sums
-__global__ void __launch_bounds__(kReduceThreads) k_reduce_batch(const Params* geo) {
-  __shared__ double ps[kReduceThreads], pc[kReduceThreads];
-  const Params& p = geo[blockIdx.y];
-  const int nq = 5 * p.metat;
-  const int q = blockIdx.x;
-  if (q >= nq) return;
-  const int nunits = p.nunits;
-  const int per = (nunits + kReduceThreads - 1) / kReduceThreads;
-  const int u0 = threadIdx.x * per, u1 = min(nunits, u0 + per);
-  double s = 0.0, c = 0.0;
-  for (int u = u0; u < u1; ++u) kahan_add(s, c, p.gen_part[(long long)u * nq + q]);
-  ps[threadIdx.x] = s;
-  pc[threadIdx.x] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double S = 0.0, C = 0.0;
-    for (int t = 0; t < kReduceThreads; ++t) {
-      kahan_add(S, C, ps[t]);
-      kahan_add(S, C, -pc[t]);
+// One exact sum (words of 32 bits in 64-bit counters, the top one signed, in
+// units of 2^-unit) as a double, rounded once from its leading 96 bits.
+__device__ double fx_value(const unsigned long long* g, int unit) {
+  uint32_t w[5];
+  unsigned long long c = 0;
+  for (int i = 0; i < 3; ++i) {
+    // the carry is below 2^32 and the counter well below 2^64 - 2^32
+    const unsigned long long x = g[i] + c;
+    w[i] = (uint32_t)x;
+    c = x >> 32;
+  }
+  const long long top = (long long)(g[3] + c);
+  w[3] = (uint32_t)top;
+  w[4] = (uint32_t)((unsigned long long)top >> 32);
+  const bool neg = top < 0;
+  if (neg) {
+    unsigned long long b = 1;
+    for (int i = 0; i < 5; ++i) {
+      b += (uint32_t)~w[i];
+      w[i] = (uint32_t)b;
+      b >>= 32;
     }
-    p.red[q] = S - C;
+  }
+  int h = 4;
+  while (h > 0 && w[h] == 0u) --h;
+  const unsigned long long hi = ((unsigned long long)w[h] << 32) | (h >= 1 ? w[h - 1] : 0u);
+  double v = (double)hi * 4294967296.0 + (double)(h >= 2 ? w[h - 2] : 0u);
+  v = ldexp(v, 32 * (h - 2) - unit);
+  return neg ? -v : v;
+}
+
+// The forward kernel's exact sums of geometry blockIdx.x as doubles: class
+// sums to hist_tab, E2 sums and norms (every class together, and the terms
+// outside the histogram) to red.  One small block per geometry: no partial
+// sums per work unit are kept or added up.
+constexpr int kFinishThreads = 256;
+__global__ void __launch_bounds__(kFinishThreads) k_finish(Params p0, const Params* geo) {
+  const Params& p = geo ? geo[blockIdx.x] : p0;
+  const int mt = p.metat, nc = p.nclass;
+  auto value = [&](const unsigned long long* lo, const unsigned long long* hi, double big) {
+    return fx_value(lo, 84) + (fx_value(hi, 44) + big);
+  };
+  for (int i = threadIdx.x; i < 2 * nc * mt; i += kFinishThreads) {
+    const int q = i / (nc * mt), c = i / mt % nc, m = i % mt;
+    const int x = fx_tab(q, c, m);
+    p.hist_tab[i] = value(p.sums + 4 * x, p.sums_hi + 4 * x, p.sums_big[x]);
+  }
+  for (int i = threadIdx.x; i < 5 * mt; i += kFinishThreads) {
+    const int q = i / mt, m = i % mt;
+    unsigned long long lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
+    double big = 0.0;
+    for (int c = 0; c <= (q < 2 ? kNClass : 0); ++c) {
+      const int x = q < 2 ? fx_tab(q, c, m) : fx_acc(q - 2, m);
+      for (int w = 0; w < 4; ++w) {
+        lo[w] += p.sums[4 * x + w];
+        hi[w] += p.sums_hi[4 * x + w];
+      }
+      big += p.sums_big[x];
+    }
+    p.red[i] = value(lo, hi, big);
   }
 }
 
@@ -162,15 +199,27 @@ __global__ void __launch_bounds__(256) k_gather(GatherArgs a) {
   }
 }
 
+// What a run accumulates into, in one allocation cleared by one call:
+// counters, dpivot, histogram counts | exact sums | work counter, records in
+// the pool (8 bytes each).
+constexpr size_t kCountWords = C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots;
+constexpr size_t kZeroWords = kCountWords + (size_t)9 * kFxSums + 2;
+void set_zeroed(Params& p, unsigned long long* z) {
+  p.counters = z;
+  p.dpivot_bits = z + C_NCOUNTERS;
+  p.hist_nom = z + C_NCOUNTERS + 1;
+  p.hist_nam = z + C_NCOUNTERS + 1 + kNClass;
+  p.sums = z + kCountWords;
+  p.sums_hi = p.sums + (size_t)4 * kFxSums;
+  p.sums_big = reinterpret_cast<double*>(p.sums_hi + (size_t)4 * kFxSums);
+  p.work = reinterpret_cast<int*>(z + kZeroWords - 2);
+  p.pool_count = z + kZeroWords - 1;
+}
+
 // zero what every geometry of a batch accumulates into (block b: geometry b)
 __global__ void k_batch_clear(const Params* geo) {
-  const Params& p = geo[blockIdx.x];
-  const int ncount = C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots;
-  for (int i = threadIdx.x; i < ncount; i += blockDim.x) p.counters[i] = 0ull;
-  for (int i = threadIdx.x; i < 2 * kNClass * kMaxRoots; i += blockDim.x) p.hist_tab[i] = 0.0;
-  const long long npart = (long long)max(p.nunits, 1) * 5 * p.metat;
-  for (long long i = threadIdx.x; i < npart; i += blockDim.x) p.gen_part[i] = 0.0;
-  if (threadIdx.x == 0 && p.pool_count) *p.pool_count = 0ull;
+  unsigned long long* z = geo[blockIdx.x].counters;
+  for (int i = threadIdx.x; i < (int)kZeroWords; i += blockDim.x) z[i] = 0ull;
 }
 
 }  // namespace
@@ -205,40 +254,37 @@ struct cipsi_ctx {
   int32_t* dpairtab = nullptr;
   int32_t* dntttt = nullptr;
   double *dF = nullptr, *dJ = nullptr, *dK = nullptr, *dfmpb = nullptr;
+  double* djx = nullptr;  // J and J - K as square matrices (coalesced rows)
   int8_t* dorbsym = nullptr;
   int64_t ninte = 0;
   // per-run buffers
-  int32_t* dunits = nullptr;
-  int units_cap = 0;
+  // the plan on the device (pack_plan): one allocation and one copy
+  unsigned char* dplan = nullptr;
+  size_t plan_cap = 0;
+  std::vector<unsigned char> hplan;
   int nunits = 0;
-  std::vector<int32_t> hunits;
-  int32_t* dgens = nullptr;
-  uint8_t* dgmask = nullptr;
-  int gens_cap = 0;
+  unsigned char* dcand = nullptr;  // candidate buffer of cand_cap slots
+  long long cand_cap = 0;
   int32_t* dnb_j = nullptr;
   uint64_t* dnb_em = nullptr;
   uint64_t* dlr_ent = nullptr;
+  uint32_t *dlr_e = nullptr, *dlrw_e = nullptr;
+  uint2* dlrw_jh = nullptr;
   size_t scratch_blocks = 0;
   double* dgen_part = nullptr;
   size_t gen_part_cap = 0;
-  unsigned long long* dcounters = nullptr;  // counters + dpivot + hist
+  unsigned long long* dcounters = nullptr;  // kZeroWords: counters, exact sums, work and pool counters
   double* dhist_tab = nullptr;
   double* dred = nullptr;
-  int* dwork = nullptr;
   uint64_t* dsel_bits = nullptr;
   int32_t* dsel_owner = nullptr;
   double *dsel_xam = nullptr, *dsel_evp = nullptr;
   long long sel_cap = 0;
-  // record path: per-CTA staging (slot-indexed), the pool of unit segments,
-  // the unit table (segment, records, output offset)
-  uint64_t* dst_bits = nullptr;
-  double *dst_xam = nullptr, *dst_evp = nullptr;
-  uint32_t* dst_mask = nullptr;
-  size_t st_slots = 0;  // allocated grid x st_cap slots
+  // record path: the pool of unit segments, the unit table (segment, records,
+  // output offset)
   uint64_t* dpool_bits = nullptr;
   double *dpool_xam = nullptr, *dpool_evp = nullptr;
   long long pool_cap = 0;
-  unsigned long long* dpool_count = nullptr;
   long long* dunit_pool = nullptr;
   int32_t* dunit_nsel = nullptr;
   long long* dunit_out = nullptr;
@@ -395,15 +441,14 @@ void cipsi_ctx_destroy(cipsi_ctx* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   dfree(ctx->dS); dfree(ctx->dygen); dfree(ctx->dyef); dfree(ctx->dnesp); dfree(ctx->dc);
   dfree(ctx->deri); dfree(ctx->dpairtab); dfree(ctx->dntttt); dfree(ctx->dF); dfree(ctx->dJ);
-  dfree(ctx->dK); dfree(ctx->dfmpb); dfree(ctx->dorbsym); dfree(ctx->dgens); dfree(ctx->dgmask);
+  dfree(ctx->dK); dfree(ctx->djx); dfree(ctx->dfmpb); dfree(ctx->dorbsym); dfree(ctx->dplan); dfree(ctx->dcand);
   dfree(ctx->deri64);
   dfree(ctx->deri_w);
-  dfree(ctx->dunits);
   dfree(ctx->dnb_j); dfree(ctx->dnb_em); dfree(ctx->dlr_ent); dfree(ctx->dgen_part);
-  dfree(ctx->dcounters); dfree(ctx->dhist_tab); dfree(ctx->dred); dfree(ctx->dwork);
+  dfree(ctx->dlr_e); dfree(ctx->dlrw_e); dfree(ctx->dlrw_jh);
+  dfree(ctx->dcounters); dfree(ctx->dhist_tab); dfree(ctx->dred);
   dfree(ctx->dsel_bits); dfree(ctx->dsel_owner); dfree(ctx->dsel_xam); dfree(ctx->dsel_evp);
-  dfree(ctx->dst_bits); dfree(ctx->dst_xam); dfree(ctx->dst_evp); dfree(ctx->dst_mask);
-  dfree(ctx->dpool_bits); dfree(ctx->dpool_xam); dfree(ctx->dpool_evp); dfree(ctx->dpool_count);
+  dfree(ctx->dpool_bits); dfree(ctx->dpool_xam); dfree(ctx->dpool_evp);
   dfree(ctx->dunit_pool); dfree(ctx->dunit_nsel); dfree(ctx->dunit_out); dfree(ctx->dscan_total);
   dfree(ctx->dsigma); dfree(ctx->dFraw); dfree(ctx->dh_count); dfree(ctx->dh_rowptr);
   dfree(ctx->dh_col); dfree(ctx->dh_val);
@@ -471,6 +516,15 @@ static int set_integrals_common(cipsi_ctx* ctx, const int32_t* itsym, const int3
   if ((rc = upload(ctx, &ctx->dF, F.data(), F.size()))) return rc;
   if ((rc = upload(ctx, &ctx->dJ, aj, nter))) return rc;
   if ((rc = upload(ctx, &ctx->dK, ak, nter))) return rc;
+  std::vector<double> jx((size_t)2 * n * n);
+  for (int i = 0; i < n; ++i)
+    for (int j = 0; j <= i; ++j) {
+      const size_t t = (size_t)i * (i + 1) / 2 + j;
+      jx[(size_t)i * n + j] = jx[(size_t)j * n + i] = aj[t];
+      jx[(size_t)n * n + (size_t)i * n + j] = jx[(size_t)n * n + (size_t)j * n + i] = aj[t] - ak[t];
+    }
+  if ((rc = upload(ctx, &ctx->djx, jx.data(), jx.size()))) return rc;
+  CK(cudaStreamSynchronize(ctx->stream));  // pt, nt, F, jx leave scope
   ctx->ninte = ninte;
   return CIPSI_OK;
 }
@@ -637,21 +691,6 @@ int cipsi_set_roots(cipsi_ctx* ctx, const double* c, const double* e, const doub
 
 }  // extern "C"
 
-static size_t queue_bytes(int W, int R) {
-  switch (W * 16 + R) {
-    case 16 + 1: return sizeof(WarpQueue<1, 1>);
-    case 16 + 2: return sizeof(WarpQueue<1, 2>);
-    case 16 + 4: return sizeof(WarpQueue<1, 4>);
-    case 16 + 8: return sizeof(WarpQueue<1, 8>);
-    case 32 + 1: return sizeof(WarpQueue<2, 1>);
-    case 32 + 2: return sizeof(WarpQueue<2, 2>);
-    case 32 + 4: return sizeof(WarpQueue<2, 4>);
-    default: return sizeof(WarpQueue<2, 8>);
-  }
-}
-
-
-
 namespace {
 
 int roots_pad(int mt) { return mt <= 1 ? 1 : mt <= 2 ? 2 : mt <= 4 ? 4 : 8; }
@@ -673,11 +712,35 @@ struct RunPlan {
   std::vector<uint8_t> gmask;  // allowed rank changes, bit (D + 2)
   std::vector<int32_t> ug, ur0, ur1;
   std::vector<long long> uslots;  // candidate slots per unit (block_candidates over its allowed blocks)
-  long long max_slots = 0;
+  long long max_slots = 0, all_slots = 0;
   bool pertu_ref = false, pertu_mono = false;
 };
 
-void plan_run(const cipsi_ctx* ctx, const cipsi_opts* o, int r_chunk, RunPlan& pl) {
+constexpr int kLowChunk = 6;  // of the reference and its singles: their L_R are the longest
+
+// Blocks of removed electrons per work unit of the forward kernels.  k_cand's
+// warps take the blocks of a unit on their own, so a unit wants a few per warp:
+// 16 at the default r_chunk of 6 (2.7 r_chunk above it; r_chunk itself below,
+// where the caller asks for fine units).  At the default, when the run has few
+// blocks, no more than leaves eight units per CTA, down to two blocks.
+// (60 orbitals, S = 2001: 45.8 ms at 24, 45.5 at 16, 47.3 at 8, 55 at 60; one
+// shard of 120 orbitals: 57, 55, 54 ms.)
+int unit_blocks(int r_chunk, long long run_blocks, int sms) {
+  if (r_chunk < 6) return r_chunk;
+  return (int)std::max(2ll, std::min<long long>(8ll * r_chunk / 3, run_blocks / (16ll * sms)));
+}
+// all blocks of a run, about: generators times pairs of electrons
+long long run_blocks(const cipsi_ctx* ctx, const cipsi_opts* o) {
+  const long long nel = 2 * ctx->d.noca;
+  long long n = 0;
+  for (int k = 0; k < ctx->d.ncf; ++k)
+    if (ctx->ygen[k] && !ctx->ysaut[k] && !(o->gen_mask && !o->gen_mask[k])) ++n;
+  return n * (nel * (nel + 1) / 2);
+}
+
+// r_chunk: allowed R blocks per work unit; low_chunk: of the reference and its
+// singles, which meet most of S
+void plan_run(const cipsi_ctx* ctx, const cipsi_opts* o, int r_chunk, int low_chunk, RunPlan& pl) {
   const int ncf = ctx->d.ncf, W = ctx->W;
   // flags on the content of S (pertu.f:52-61)
   bool yd = false, ym = false, yf = false;
@@ -745,6 +808,7 @@ void plan_run(const cipsi_ctx* ctx, const cipsi_opts* o, int r_chunk, RunPlan& p
     ur1.push_back(b);
     pl.uslots.push_back(slots);
     pl.max_slots = std::max(pl.max_slots, slots);
+    pl.all_slots += slots;
   };
   for (int g : order) {
     const int k = gens[g];
@@ -787,7 +851,7 @@ void plan_run(const cipsi_ctx* ctx, const cipsi_opts* o, int r_chunk, RunPlan& p
         if (m & (1u << (hfR + aV - nRr + 2))) return true;
       return false;
     };
-    const int kRChunk = ctx->rank[k] <= 1 ? 1 : kRChunkHigh;
+    const int kRChunk = ctx->rank[k] <= 1 ? low_chunk : kRChunkHigh;
     int cnt = 0, start = -1, last = -1;
     long long slots = 0;
     for (int r = 0; r < nR; ++r) {
@@ -807,33 +871,67 @@ void plan_run(const cipsi_ctx* ctx, const cipsi_opts* o, int r_chunk, RunPlan& p
   }
 }
 
-// Shared-memory L_R capacity, dynamic shared memory and CTAs per SM.
-// ctas: 0 = 200 KB per CTA (two CTAs per SM when the list fits in half),
-// 1 = one CTA per SM, 2 = sized so that two CTAs fit per SM.
+// CTAs per SM of k_cand: ctas 0 = as many as fit, 1 or 2 = at most that many
+int fwd_blocks_per_sm(int W, int R, int ctas) {
+  const int fit = W == 1 ? (R == 1 ? cand_ctas<1, 1>() : R == 2 ? cand_ctas<1, 2>() : R == 4 ? cand_ctas<1, 4>()
+                                                                                           : cand_ctas<1, 8>())
+                         : (R == 1 ? cand_ctas<2, 1>() : R == 2 ? cand_ctas<2, 2>() : R == 4 ? cand_ctas<2, 4>()
+                                                                                           : cand_ctas<2, 8>());
+  return ctas == 0 ? fit : std::min(fit, ctas);
+}
+
+// Bytes of a candidate's slot, and the most that one buffer takes: runs with
+// more slots go through it in parts (a few GB: enough units for every SM even
+// at 120 orbitals, where a unit has 200,000 slots).
+constexpr size_t cand_slot_bytes(int R) { return 8 * (size_t)R + 8 + 8 + 4 + 4; }
+constexpr size_t kCandMaxBytes = (size_t)8 << 30;
+CandBuf cand_views(unsigned char* base, long long cap, int R) {
+  CandBuf c;
+  c.cap = cap;
+  c.b = reinterpret_cast<double*>(base);
+  c.mp = c.b + (size_t)R * cap;
+  c.vp = c.mp + cap;
+  c.code = reinterpret_cast<uint32_t*>(c.vp + cap);
+  c.meta = c.code + cap;
+  return c;
+}
+
+// Units in parts whose slots add up to at most cap (a unit's own slots fit):
+// the parts' first units, then the number of units; slot0: each unit's first
+// slot in its part.
+std::vector<int> cut_units(const std::vector<long long>& slots, long long cap, std::vector<long long>& slot0) {
+  std::vector<int> cut{0};
+  slot0.resize(slots.size());
+  long long acc = 0;
+  for (int u = 0; u < (int)slots.size(); ++u) {
+    if (acc + slots[u] > cap && u > cut.back()) {
+      cut.push_back(u);
+      acc = 0;
+    }
+    slot0[u] = acc;
+    acc += slots[u];
+  }
+  if (cut.back() != (int)slots.size()) cut.push_back((int)slots.size());
+  return cut;
+}
+
+// The adjoint kernel's shared-memory L_R capacity, dynamic shared memory and
+// CTAs per SM.  ctas: 1 = one CTA per SM with a long list, else two: the part
+// of a longer list is read from the block's global scratch, 8 bytes per
+// entry, which costs less than halving the resident warps (82 + 32 KB of
+// static shared memory fit an SM twice).
 struct LaunchShape {
   int lr_cap;
   size_t smem;
   int blocks_per_sm;
 };
-
-// adj: the adjoint launch.  Its static shared memory exceeds the forward's
-// by ~4 KB (the per-block dE/dhdig and dE/dhmp sums), which its L_R list
-// gives back so that two CTAs still fit per SM; it never fills the
-// epilogue queues (its drains find them empty), so they take no space.
-LaunchShape launch_shape(int W, int R, int ncf_max, int ctas, bool adj = false) {
+LaunchShape adj_shape(int ncf_max, int ctas) {
   const size_t per_entry = 8;  // compact L_R entry
-  const size_t qbytes = adj ? 0 : (size_t)(kThreads / 32) * queue_bytes(W, R);
-  // two CTAs per SM unless one is asked for: the part of a long L_R list
-  // beyond shared memory is read from the block's global scratch, 8 bytes
-  // per entry, which costs less than halving the resident warps
-  // (the kernel's static shared memory, ~28 KB, comes on top: two CTAs of
-  // 82 + 28 KB, or one of 192 + 28 KB, fit the SM's 228 KB)
-  const size_t smem_total = (ctas == 1 ? (size_t)192 * 1024 : (size_t)82 * 1024) - (adj ? 4096 : 0);
-  const size_t smem_budget = smem_total > qbytes + 16 ? smem_total - qbytes - 16 : 0;
+  const size_t smem_budget = (ctas == 1 ? (size_t)188 * 1024 : (size_t)78 * 1024) - 16;
   LaunchShape ls;
   ls.lr_cap = (int)std::min<size_t>((size_t)ncf_max, smem_budget / per_entry);
-  ls.smem = (((size_t)ls.lr_cap * per_entry + 15) & ~(size_t)15) + qbytes + 16;
-  ls.blocks_per_sm = ctas == 1 ? 1 : ls.smem <= (adj ? 82 : 86) * 1024 ? 2 : 1;
+  ls.smem = (((size_t)ls.lr_cap * per_entry + 15) & ~(size_t)15) + 16;
+  ls.blocks_per_sm = ctas == 1 ? 1 : 2;
   return ls;
 }
 
@@ -864,54 +962,63 @@ int grow_sel(cipsi_ctx* ctx, long long cap) {
   return CIPSI_OK;
 }
 
-// Device buffers of one run on ctx (generator and unit lists, per-unit
-// partial sums, counters, histogram, records), sized for the plan; the lists
-// are uploaded on stream st.
-int prepare_run(cipsi_ctx* ctx, const RunPlan& pl, cudaStream_t st) {
-  const int mt = ctx->d.metat;
-  const int ngen = (int)pl.gens.size(), nunits = (int)pl.ug.size();
-  ctx->ngen = ngen;
-  ctx->nunits = nunits;
-  if (ngen > ctx->gens_cap) {
-    ++ctx->buf_gen;
-    dfree(ctx->dgens); dfree(ctx->dgmask);
-    CK(cudaMalloc(&ctx->dgens, (size_t)std::max(ngen, 1) * sizeof(int32_t)));
-    CK(cudaMalloc(&ctx->dgmask, (size_t)std::max(ngen, 1)));
-    ctx->gens_cap = ngen;
+// A plan as the kernels read it: per unit its first slot in the candidate
+// buffer (8 bytes), generator slot, block range and number of slots (4 each);
+// the generators and their masks.  Appended to `out` at a multiple of 64 bytes.
+size_t pack_plan(const RunPlan& pl, const std::vector<long long>& slot0, std::vector<unsigned char>& out) {
+  const size_t base = (out.size() + 63) / 64 * 64, ngen = pl.gens.size(), nu = pl.ug.size();
+  out.resize(base + nu * (8 + 4 * 4) + ngen * 5);
+  size_t off = base;
+  auto put = [&](const void* src, size_t n) {
+    if (n) std::memcpy(out.data() + off, src, n);
+    off += n;
+  };
+  const std::vector<int32_t> ns(pl.uslots.begin(), pl.uslots.end());
+  put(slot0.data(), nu * 8);
+  put(pl.ug.data(), nu * 4);
+  put(pl.ur0.data(), nu * 4);
+  put(pl.ur1.data(), nu * 4);
+  put(ns.data(), nu * 4);
+  put(pl.gens.data(), ngen * 4);
+  put(pl.gmask.data(), ngen);
+  return base;
+}
+// the kernels' parameters of a packed plan at device address d
+void set_plan(Params& p, const unsigned char* d, int nunits, int ngen) {
+  const int32_t* u = reinterpret_cast<const int32_t*>(d + (size_t)nunits * 8);
+  p.nunits = nunits;
+  p.ngen = ngen;
+  p.unit_g = u;
+  p.unit_r0 = u + nunits;
+  p.unit_r1 = u + 2 * (size_t)nunits;
+  p.gens = u + 4 * (size_t)nunits;
+  p.gen_dmask = reinterpret_cast<const uint8_t*>(p.gens + ngen);
+}
+
+// Device buffers of one run on ctx (counters, histogram, records; the plan,
+// uploaded on stream st, unless the caller keeps it: slot0 null), sized for it.
+int prepare_run(cipsi_ctx* ctx, const RunPlan& pl, const std::vector<long long>* slot0, cudaStream_t st) {
+  const int nunits = (int)pl.ug.size();
+  if (slot0) {
+    ctx->hplan.clear();
+    pack_plan(pl, *slot0, ctx->hplan);
+    const size_t bytes = ctx->hplan.size();
+    if (bytes > ctx->plan_cap || !ctx->dplan) {
+      ++ctx->buf_gen;
+      dfree(ctx->dplan);
+      ctx->plan_cap = 0;
+      CK(cudaMalloc(&ctx->dplan, std::max<size_t>(bytes, 64)));
+      ctx->plan_cap = std::max<size_t>(bytes, 64);
+    }
+    ctx->nunits = nunits;
+    ctx->ngen = (int)pl.gens.size();
+    if (bytes) CK(cudaMemcpyAsync(ctx->dplan, ctx->hplan.data(), bytes, cudaMemcpyHostToDevice, st));
   }
-  if (nunits > ctx->units_cap) {
-    ++ctx->buf_gen;
-    dfree(ctx->dunits);
-    CK(cudaMalloc(&ctx->dunits, (size_t)std::max(nunits, 1) * 3 * sizeof(int32_t)));
-    ctx->units_cap = nunits;
-  }
-  if (ngen) {
-    CK(cudaMemcpyAsync(ctx->dgens, pl.gens.data(), ngen * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(ctx->dgmask, pl.gmask.data(), ngen, cudaMemcpyHostToDevice, st));
-  }
-  if (nunits) {
-    ctx->hunits.resize((size_t)3 * nunits);
-    std::copy(pl.ug.begin(), pl.ug.end(), ctx->hunits.begin());
-    std::copy(pl.ur0.begin(), pl.ur0.end(), ctx->hunits.begin() + nunits);
-    std::copy(pl.ur1.begin(), pl.ur1.end(), ctx->hunits.begin() + 2 * nunits);
-    CK(cudaMemcpyAsync(ctx->dunits, ctx->hunits.data(), (size_t)3 * nunits * sizeof(int32_t),
-                       cudaMemcpyHostToDevice, st));
-  }
-  const size_t nq = (size_t)5 * mt;
-  if ((size_t)std::max(nunits, 1) * nq > ctx->gen_part_cap) {
-    ++ctx->buf_gen;
-    dfree(ctx->dgen_part);
-    ctx->gen_part_cap = (size_t)std::max(nunits, 1) * nq;
-    CK(cudaMalloc(&ctx->dgen_part, ctx->gen_part_cap * sizeof(double)));
-  }
-  // counters [C_NCOUNTERS] + dpivot + nom[10] + nam[10*8]
-  const size_t ncount = C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots;
   if (!ctx->dcounters) {
     ++ctx->buf_gen;
-    CK(cudaMalloc(&ctx->dcounters, ncount * sizeof(unsigned long long)));
+    CK(cudaMalloc(&ctx->dcounters, kZeroWords * sizeof(unsigned long long)));
     CK(cudaMalloc(&ctx->dhist_tab, 2 * kNClass * kMaxRoots * sizeof(double)));
     CK(cudaMalloc(&ctx->dred, 5 * kMaxRoots * sizeof(double)));
-    CK(cudaMalloc(&ctx->dwork, sizeof(int)));
   }
   if (ctx->pool_cap == 0) {
     const int rc = grow_pool(ctx, 1 << 20);
@@ -929,32 +1036,24 @@ int prepare_run(cipsi_ctx* ctx, const RunPlan& pl, cudaStream_t st) {
     CK(cudaMalloc(&ctx->dunit_out, (size_t)nunits * sizeof(long long)));
     ctx->unit_tab_cap = nunits;
   }
-  if (!ctx->dpool_count) {
+  if (!ctx->dscan_total) {
     ++ctx->buf_gen;
-    CK(cudaMalloc(&ctx->dpool_count, sizeof(unsigned long long)));
     CK(cudaMalloc(&ctx->dscan_total, sizeof(unsigned long long)));
   }
   return CIPSI_OK;
 }
 
-// Per-CTA record staging for `grid` CTAs of st_cap slots each.
-int ensure_staging(cipsi_ctx* ctx, int grid, long long st_cap) {
-  const size_t slots = (size_t)grid * (size_t)st_cap;
-  if (slots <= ctx->st_slots && ctx->dst_mask) return CIPSI_OK;
+// The candidate buffer, for at least `slots` slots.
+int ensure_cand(cipsi_ctx* ctx, long long slots) {
+  if (slots <= ctx->cand_cap && ctx->dcand) return CIPSI_OK;
   ++ctx->buf_gen;
-  dfree(ctx->dst_bits); dfree(ctx->dst_xam); dfree(ctx->dst_evp); dfree(ctx->dst_mask);
-  const int W = ctx->W, mt = ctx->d.metat;
-  CK(cudaMalloc(&ctx->dst_bits, slots * 2 * W * sizeof(uint64_t)));
-  CK(cudaMalloc(&ctx->dst_xam, slots * sizeof(double)));
-  CK(cudaMalloc(&ctx->dst_evp, slots * mt * sizeof(double)));
-  CK(cudaMalloc(&ctx->dst_mask, slots / 32 * sizeof(uint32_t)));
-  CK(cudaMemset(ctx->dst_mask, 0, slots / 32 * sizeof(uint32_t)));
-  ctx->st_slots = slots;
+  dfree(ctx->dcand);
+  ctx->cand_cap = 0;
+  const long long cap = std::max<long long>((slots + 63) / 64 * 64, 64);
+  CK(cudaMalloc(&ctx->dcand, (size_t)cap * cand_slot_bytes(roots_pad(ctx->d.metat))));
+  ctx->cand_cap = cap;
   return CIPSI_OK;
 }
-
-// Staging slots per CTA for a plan: its largest unit, in whole mask words.
-long long staging_cap(const RunPlan& pl) { return std::max<long long>(32, (pl.max_slots + 31) / 32 * 32); }
 
 // Kernel parameters of one run on ctx (everything but the neighbour scratch
 // and the L_R capacity).
@@ -967,13 +1066,7 @@ void fill_params(const cipsi_ctx* ctx, const cipsi_opts* o, const RunPlan& pl, P
   p.metat = mt;
   p.nsym = ctx->d.nsym;
   p.isym = ctx->d.isym;
-  p.ngen = (int)pl.gens.size();
-  p.gens = ctx->dgens;
-  p.gen_dmask = ctx->dgmask;
-  p.nunits = nunits;
-  p.unit_g = ctx->dunits;
-  p.unit_r0 = ctx->dunits + nunits;
-  p.unit_r1 = ctx->dunits + 2 * nunits;
+  set_plan(p, ctx->dplan, nunits, (int)pl.gens.size());
   p.S = ctx->dS;
   p.ygen = ctx->dygen;
   p.nesp = ctx->dnesp;
@@ -986,6 +1079,7 @@ void fill_params(const cipsi_ctx* ctx, const cipsi_opts* o, const RunPlan& pl, P
   p.F = ctx->dF;
   p.J = ctx->dJ;
   p.K = ctx->dK;
+  p.jx = ctx->djx;
   p.fmpb = ctx->dfmpb;
   p.orbsym = ctx->dorbsym;
   for (int i = 0; i < ctx->d.nsym; ++i)
@@ -1008,30 +1102,20 @@ void fill_params(const cipsi_ctx* ctx, const cipsi_opts* o, const RunPlan& pl, P
   for (int i = 0; i < kNClass; ++i) {
     p.aval[i] = o->aval[i];
     std::memcpy(&p.aval_bits[i], &o->aval[i], 8);
+    p.aval_hi[i] = i + 1 < o->nclass ? (int)(p.aval_bits[i] >> 32) : 0x7fffffff;
   }
   p.pertu_ref = pl.pertu_ref ? 1 : 0;
   p.pertu_mono = pl.pertu_mono ? 1 : 0;
-  p.gen_part = ctx->dgen_part;
-  p.counters = ctx->dcounters;
-  p.dpivot_bits = ctx->dcounters + C_NCOUNTERS;
-  p.hist_nom = ctx->dcounters + C_NCOUNTERS + 1;
-  p.hist_nam = ctx->dcounters + C_NCOUNTERS + 1 + kNClass;
+  set_zeroed(p, ctx->dcounters);
   p.hist_tab = ctx->dhist_tab;
   p.red = ctx->dred;
   p.rec_mode = 1;
-  p.st_cap = (int)staging_cap(pl);
-  p.st_bits = ctx->dst_bits;
-  p.st_xam = ctx->dst_xam;
-  p.st_evp = ctx->dst_evp;
-  p.st_mask = ctx->dst_mask;
   p.pool_bits = ctx->dpool_bits;
   p.pool_xam = ctx->dpool_xam;
   p.pool_evp = ctx->dpool_evp;
   p.pool_cap = ctx->pool_cap;
-  p.pool_count = ctx->dpool_count;
   p.unit_pool = ctx->dunit_pool;
   p.unit_nsel = ctx->dunit_nsel;
-  p.work = ctx->dwork;
 }
 
 // Output arrays of a run's records: the caller's pinned sink or the
@@ -1077,12 +1161,21 @@ cudaError_t enqueue_gather(const cipsi_ctx* ctx, const Params& p, int u0, int u1
   return cudaGetLastError();
 }
 
-// Per-CTA neighbour scratch (nb_j, nb_emask, lr_ent) for `grid` CTAs.
+// entries of a warp's L_R overflow lists for S of ncf determinants
+int lrw_entries(int ncf) { return std::min(kLrWarpG, ncf); }
+
+// Per-CTA neighbour and L_R scratch for `grid` CTAs.
 int ensure_neighbour_scratch(cipsi_ctx* ctx, int grid) {
   if ((size_t)grid <= ctx->scratch_blocks && ctx->dnb_j) return CIPSI_OK;
   const int ncf = ctx->d.ncf;
   ++ctx->buf_gen;
   dfree(ctx->dnb_j); dfree(ctx->dnb_em); dfree(ctx->dlr_ent);
+  dfree(ctx->dlr_e); dfree(ctx->dlrw_e); dfree(ctx->dlrw_jh);
+  ctx->scratch_blocks = 0;
+  const size_t nw = (size_t)grid * kWarps * 2 * lrw_entries(ncf);
+  CK(cudaMalloc(&ctx->dlr_e, (size_t)grid * ncf * sizeof(uint32_t)));
+  CK(cudaMalloc(&ctx->dlrw_e, nw * sizeof(uint32_t)));
+  CK(cudaMalloc(&ctx->dlrw_jh, nw * sizeof(uint2)));
   CK(cudaMalloc(&ctx->dnb_j, (size_t)grid * ncf * sizeof(int32_t)));
   CK(cudaMalloc(&ctx->dnb_em, (size_t)grid * ncf * sizeof(uint64_t)));
   CK(cudaMalloc(&ctx->dlr_ent, (size_t)grid * ncf * sizeof(uint64_t)));
@@ -1090,17 +1183,62 @@ int ensure_neighbour_scratch(cipsi_ctx* ctx, int grid) {
   return CIPSI_OK;
 }
 
-// the plain (one geometry) forward launch of k_pt2<W, R>
-cudaError_t launch_plain(const Params& p, int W, int R, int grid, size_t smem, cudaStream_t st) {
-  if (W == 1)
-    return R == 1 ? launch_pt2<1, 1, false>(p, BatchArgs{}, grid, smem, st)
-         : R == 2 ? launch_pt2<1, 2, false>(p, BatchArgs{}, grid, smem, st)
-         : R == 4 ? launch_pt2<1, 4, false>(p, BatchArgs{}, grid, smem, st)
-                  : launch_pt2<1, 8, false>(p, BatchArgs{}, grid, smem, st);
-  return R == 1 ? launch_pt2<2, 1, false>(p, BatchArgs{}, grid, smem, st)
-       : R == 2 ? launch_pt2<2, 2, false>(p, BatchArgs{}, grid, smem, st)
-       : R == 4 ? launch_pt2<2, 4, false>(p, BatchArgs{}, grid, smem, st)
-                : launch_pt2<2, 8, false>(p, BatchArgs{}, grid, smem, st);
+// the context's neighbour and L_R scratch into the kernel's parameters
+void set_scratch(const cipsi_ctx* ctx, Params& p) {
+  p.nb_j = ctx->dnb_j;
+  p.nb_emask = ctx->dnb_em;
+  p.lr_ent = ctx->dlr_ent;
+  p.lr_jh = reinterpret_cast<uint2*>(ctx->dlr_ent);
+  p.lr_e = ctx->dlr_e;
+  p.lrw_e = ctx->dlrw_e;
+  p.lrw_jh = ctx->dlrw_jh;
+  p.lrw_cap = lrw_entries(ctx->d.ncf);
+  p.nb_stride = ctx->d.ncf;
+}
+
+// both forward kernels of class (W, R) on the units of `la`: the candidate
+// buffer's marks cleared, then k_cand on `grid` CTAs and k_pt2
+template <bool B>
+cudaError_t launch_forward(const Params& p, const LaunchArgs& la, int W, int R, int grid, int sms, long long slots,
+                           cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(la.cand.meta, 0, (size_t)slots * sizeof(uint32_t), st);
+  if (e != cudaSuccess) return e;
+#define CIPSI_FORWARD(W_, R_)                                  \
+  if (W == W_ && R == R_) {                                    \
+    e = launch_cand<W_, R_, B>(p, la, grid, st);               \
+    return e != cudaSuccess ? e : launch_pt2<W_, R_, B>(p, la, sms, st); \
+  }
+  CIPSI_FORWARD(1, 1)
+  CIPSI_FORWARD(1, 2)
+  CIPSI_FORWARD(1, 4)
+  CIPSI_FORWARD(1, 8)
+  CIPSI_FORWARD(2, 1)
+  CIPSI_FORWARD(2, 2)
+  CIPSI_FORWARD(2, 4)
+  CIPSI_FORWARD(2, 8)
+#undef CIPSI_FORWARD
+  return cudaErrorInvalidValue;
+}
+
+// units [u0, u1) of the context's plan
+LaunchArgs plan_args(const cipsi_ctx* ctx, const Params& p, int u0, int u1) {
+  LaunchArgs la{};
+  la.unit_slot = reinterpret_cast<const long long*>(ctx->dplan) + u0;
+  la.unit_nslots = reinterpret_cast<const int32_t*>(ctx->dplan + (size_t)ctx->nunits * 8) + 3 * (size_t)ctx->nunits + u0;
+  la.cand = cand_views(ctx->dcand, ctx->cand_cap, roots_pad(ctx->d.metat));
+  la.nunits = u1 - u0;
+  la.work = p.work;
+  return la;
+}
+// the parameters of a launch over units u0.. of the plan
+Params part_params(const Params& p, int u0) {
+  Params q = p;
+  q.unit_g += u0;
+  q.unit_r0 += u0;
+  q.unit_r1 += u0;
+  q.unit_pool += u0;
+  q.unit_nsel += u0;
+  return q;
 }
 
 }  // namespace
@@ -1158,53 +1296,54 @@ int cipsi_run_pt2_async(cipsi_ctx* ctx, const cipsi_opts* o) {
   int rc = check_run_args(ctx, o);
   if (rc) return rc;
   CK(cudaSetDevice(ctx->device));
-  const int ncf = ctx->d.ncf, W = ctx->W, mt = ctx->d.metat;
-  RunPlan pl;
-  plan_run(ctx, o, ctx->tune_r_chunk, pl);
-  const int nunits = (int)pl.ug.size();
+  const int W = ctx->W, mt = ctx->d.metat;
   int dev_sms = 0;
   CK(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
-  const LaunchShape ls = launch_shape(W, roots_pad(mt), ncf, ctx->tune_ctas);
-  const int grid = std::max(1, std::min(nunits, dev_sms * ls.blocks_per_sm));
+  RunPlan pl;
+  const int ub = unit_blocks(ctx->tune_r_chunk, run_blocks(ctx, o), dev_sms);
+  plan_run(ctx, o, ub, std::min(ub, kLowChunk), pl);
+  const int nunits = (int)pl.ug.size();
+  const int R = roots_pad(mt);
+  const int grid = std::max(1, std::min(nunits, dev_sms * fwd_blocks_per_sm(W, R, ctx->tune_ctas)));
   rc = ensure_neighbour_scratch(ctx, grid);
   if (rc) return rc;
-  rc = prepare_run(ctx, pl, ctx->stream);
+  const long long cap = std::max(pl.max_slots, (long long)(kCandMaxBytes / cand_slot_bytes(R)));
+  std::vector<long long> slot0;
+  const std::vector<int> cut = cut_units(pl.uslots, cap, slot0);
+  rc = prepare_run(ctx, pl, &slot0, ctx->stream);
   if (rc) return rc;
-  rc = ensure_staging(ctx, grid, staging_cap(pl));
+  rc = ensure_cand(ctx, std::min(cap, pl.all_slots));
   if (rc) return rc;
-  const size_t nq = (size_t)5 * mt;
-  const size_t ncount = C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots;
-  CK(cudaMemsetAsync(ctx->dcounters, 0, ncount * sizeof(unsigned long long), ctx->stream));
-  CK(cudaMemsetAsync(ctx->dhist_tab, 0, 2 * kNClass * kMaxRoots * sizeof(double), ctx->stream));
-  CK(cudaMemsetAsync(ctx->dwork, 0, sizeof(int), ctx->stream));
-  CK(cudaMemsetAsync(ctx->dpool_count, 0, sizeof(unsigned long long), ctx->stream));
-  CK(cudaMemsetAsync(ctx->dgen_part, 0, (size_t)std::max(nunits, 1) * nq * sizeof(double), ctx->stream));
+  CK(cudaMemsetAsync(ctx->dcounters, 0, kZeroWords * sizeof(unsigned long long), ctx->stream));
 
   Params p{};
   fill_params(ctx, o, pl, p);
-  p.nb_j = ctx->dnb_j;
-  p.nb_emask = ctx->dnb_em;
-  p.lr_ent = ctx->dlr_ent;
-  p.lr_cap = ls.lr_cap;
-  p.nb_stride = ncf;
+  set_scratch(ctx, p);
 
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   if (nunits > 0) {
-    cudaError_t e = launch_plain(p, W, roots_pad(mt), grid, ls.smem, ctx->stream);
-    if (e != cudaSuccess) return fail(ctx, CIPSI_ERR_CUDA, std::string("k_pt2 launch: ") + cudaGetErrorString(e));
+    cudaError_t e = cudaSuccess;
+    for (size_t c = 0; c + 1 < cut.size(); ++c) {
+      const int u0 = cut[c], u1 = cut[c + 1];
+      if (c) CK(cudaMemsetAsync(p.work, 0, 2 * sizeof(int), ctx->stream));
+      const LaunchArgs la = plan_args(ctx, p, u0, u1);
+      e = launch_forward<false>(part_params(p, u0), la, W, R, std::min(grid, u1 - u0), dev_sms,
+                                slot0[u1 - 1] + pl.uslots[u1 - 1], ctx->stream);
+      if (e != cudaSuccess)
+        return fail(ctx, CIPSI_ERR_CUDA, std::string("k_cand / k_pt2 launch: ") + cudaGetErrorString(e));
+    }
     CK(cudaEventRecord(ctx->evk, ctx->stream));
-    ctx->last_launches = 4;
+    ctx->last_launches = 2 * (long long)(cut.size() - 1) + 3;  // and the unit scan, the gather, k_finish
     GatherArgs ga{};
     record_target(ctx, ga);
     e = enqueue_gather(ctx, p, 0, nunits, 0, ga, ctx->stream, dev_sms);
     if (e != cudaSuccess) return fail(ctx, CIPSI_ERR_CUDA, std::string("record gather: ") + cudaGetErrorString(e));
-    k_reduce<<<(unsigned)nq, kReduceThreads, 0, ctx->stream>>>(ctx->dgen_part, nunits, (int)nq, ctx->dred);
-    CK(cudaGetLastError());
   } else {
     CK(cudaEventRecord(ctx->evk, ctx->stream));
-    ctx->last_launches = 0;
-    CK(cudaMemsetAsync(ctx->dred, 0, nq * sizeof(double), ctx->stream));
+    ctx->last_launches = 1;
   }
+  k_finish<<<1, kFinishThreads, 0, ctx->stream>>>(p, nullptr);
+  CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev1, ctx->stream));
   ctx->ev_valid = true;
   ctx->nclass = o->nclass;
@@ -1234,7 +1373,7 @@ int cipsi_fetch_result(cipsi_ctx* ctx, cipsi_result* r) {
     r->psimp[m] = red[3 * mt + m];
     r->psivp[m] = red[4 * mt + m];
   }
-  const size_t ncount = C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots;
+  const size_t ncount = kCountWords;
   std::vector<unsigned long long> cnt(ncount);
   CK(cudaMemcpy(cnt.data(), ctx->dcounters, ncount * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
   std::vector<double> tab(2 * kNClass * kMaxRoots);
@@ -1278,7 +1417,7 @@ int cipsi_fetch_result(cipsi_ctx* ctx, cipsi_result* r) {
   const long long nsel = (long long)cnt[C_NSEL];
   r->n_selected = nsel;
   if (cnt[C_STAGE_OVF])
-    return fail(ctx, CIPSI_ERR_CUDA, "internal error: a selected candidate's slot lay outside its staging region");
+    return fail(ctx, CIPSI_ERR_CUDA, "internal error: a candidate's slot lay outside its work unit");
   // the records are valid when every unit segment found room in the pool;
   // the output arrays then hold the first out_cap of them, in unit order
   const long long out_cap = ctx->sink ? ctx->sink_cap : ctx->sel_cap;
@@ -1366,7 +1505,7 @@ int ensure_stream_buffers(cipsi_ctx* ctx, long long cap, bool host, long long hb
 // cipsi_fetch_result), reading on the context stream
 int read_results(cipsi_ctx* ctx, int nclass, cipsi_result* r) {
   const int mt = ctx->d.metat;
-  const size_t ncount = C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots;
+  const size_t ncount = kCountWords;
   std::vector<double> red(5 * mt), tab(2 * kNClass * kMaxRoots);
   std::vector<unsigned long long> cnt(ncount);
   CK(cudaMemcpyAsync(red.data(), ctx->dred, red.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1405,7 +1544,7 @@ int read_results(cipsi_ctx* ctx, int nclass, cipsi_result* r) {
                            cnt[C_NP1] * (8.0 * mt + 8.0 + 2.0 * avg_rank * 2 * 4.0) +
                            cnt[C_NPROC] * (8.0 * avg_rank + 8.0 * (avg_rank + avg_rank * avg_rank) + 8.0 * mt));
   if (cnt[C_STAGE_OVF])
-    return fail(ctx, CIPSI_ERR_CUDA, "internal error: a selected candidate's slot lay outside its staging region");
+    return fail(ctx, CIPSI_ERR_CUDA, "internal error: a candidate's slot lay outside its work unit");
   return CIPSI_OK;
 }
 
@@ -1420,17 +1559,16 @@ int cipsi_run_pt2_stream(cipsi_ctx* ctx, const cipsi_opts* o, int64_t chunk_reco
   if (!r) return fail(ctx, CIPSI_ERR_ARG, "run_pt2_stream: null result");
   if (ctx->pending) return fail(ctx, CIPSI_ERR_STATE, "an asynchronous run is pending: fetch its result first");
   CK(cudaSetDevice(ctx->device));
-  const int ncf = ctx->d.ncf, W = ctx->W, mt = ctx->d.metat;
-  RunPlan pl;
-  plan_run(ctx, o, ctx->tune_r_chunk, pl);
-  const int nunits = (int)pl.ug.size();
+  const int W = ctx->W, mt = ctx->d.metat;
   int dev_sms = 0;
   CK(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
-  const LaunchShape ls = launch_shape(W, roots_pad(mt), ncf, ctx->tune_ctas);
-  const int grid = std::max(1, std::min(nunits, dev_sms * ls.blocks_per_sm));
+  RunPlan pl;
+  const int ub = unit_blocks(ctx->tune_r_chunk, run_blocks(ctx, o), dev_sms);
+  plan_run(ctx, o, ub, std::min(ub, kLowChunk), pl);
+  const int nunits = (int)pl.ug.size();
+  const int R = roots_pad(mt);
+  const int grid = std::max(1, std::min(nunits, dev_sms * fwd_blocks_per_sm(W, R, ctx->tune_ctas)));
   if ((rc = ensure_neighbour_scratch(ctx, grid))) return rc;
-  if ((rc = prepare_run(ctx, pl, ctx->stream))) return rc;
-  if ((rc = ensure_staging(ctx, grid, staging_cap(pl)))) return rc;
   // chunk capacity: what was asked, else what about half the free device
   // memory holds (pool + two record buffers), at most 2^29 records; at
   // least the largest unit's slots
@@ -1451,22 +1589,15 @@ int cipsi_run_pt2_stream(cipsi_ctx* ctx, const cipsi_opts* o, int64_t chunk_reco
     }
   }
   cap = std::max(cap, std::max<long long>(pl.max_slots, 1024));
+  // a chunk's candidates have to fit their buffer too
+  cap = std::min(cap, std::max(std::max<long long>(pl.max_slots, 1024), (long long)(kCandMaxBytes / cand_slot_bytes(R))));
+  std::vector<long long> slot0;
+  const std::vector<int> cut = cut_units(pl.uslots, cap, slot0);
+  if ((rc = prepare_run(ctx, pl, &slot0, ctx->stream))) return rc;
+  if ((rc = ensure_cand(ctx, std::min(cap, pl.all_slots)))) return rc;
   if (ctx->pool_cap < cap && (rc = grow_pool(ctx, cap))) return rc;
   const long long hb_cap = std::min<long long>(cap, 1ll << 24);
   if ((rc = ensure_stream_buffers(ctx, cap, fn != nullptr, hb_cap))) return rc;
-  // chunks: consecutive units whose slots add up to at most cap
-  std::vector<int> cut{0};
-  {
-    long long acc = 0;
-    for (int u = 0; u < nunits; ++u) {
-      if (acc + pl.uslots[u] > cap && u > cut.back()) {
-        cut.push_back(u);
-        acc = 0;
-      }
-      acc += pl.uslots[u];
-    }
-    if (cut.back() != nunits) cut.push_back(nunits);
-  }
   const int nchunks = (int)cut.size() - 1;
   // per chunk: records gathered and records placed in the pool (pinned)
   unsigned long long* hcnt = nullptr;
@@ -1477,18 +1608,10 @@ int cipsi_run_pt2_stream(cipsi_ctx* ctx, const cipsi_opts* o, int64_t chunk_reco
     ~HostFree() { if (p) cudaFreeHost(p); }
   } hold{hcnt};
 
-  const size_t nq = (size_t)5 * mt;
-  const size_t ncount = C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots;
-  CK(cudaMemsetAsync(ctx->dcounters, 0, ncount * sizeof(unsigned long long), ctx->stream));
-  CK(cudaMemsetAsync(ctx->dhist_tab, 0, 2 * kNClass * kMaxRoots * sizeof(double), ctx->stream));
-  CK(cudaMemsetAsync(ctx->dgen_part, 0, (size_t)std::max(nunits, 1) * nq * sizeof(double), ctx->stream));
+  CK(cudaMemsetAsync(ctx->dcounters, 0, kZeroWords * sizeof(unsigned long long), ctx->stream));
   Params p{};
   fill_params(ctx, o, pl, p);
-  p.nb_j = ctx->dnb_j;
-  p.nb_emask = ctx->dnb_em;
-  p.lr_ent = ctx->dlr_ent;
-  p.lr_cap = ls.lr_cap;
-  p.nb_stride = ncf;
+  set_scratch(ctx, p);
   const size_t words = 2 * (size_t)W;
 
   long long delivered = 0;  // records handed to the consumer so far
@@ -1552,20 +1675,14 @@ int cipsi_run_pt2_stream(cipsi_ctx* ctx, const cipsi_opts* o, int64_t chunk_reco
     const int u0 = cut[c], u1 = cut[c + 1], b = c & 1;
     // the record buffer of this chunk was last read by chunk c - 2's copies
     if (c >= 2 && fn) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_copied[b], 0));
-    CK(cudaMemsetAsync(ctx->dwork, 0, sizeof(int), ctx->stream));
-    CK(cudaMemsetAsync(ctx->dpool_count, 0, sizeof(unsigned long long), ctx->stream));
-    Params pc = p;
-    pc.nunits = u1 - u0;
-    pc.unit_g = p.unit_g + u0;
-    pc.unit_r0 = p.unit_r0 + u0;
-    pc.unit_r1 = p.unit_r1 + u0;
-    pc.gen_part = p.gen_part + (size_t)u0 * nq;
-    pc.unit_pool = p.unit_pool + u0;
-    pc.unit_nsel = p.unit_nsel + u0;
-    const int cgrid = std::max(1, std::min(u1 - u0, grid));
+    // work counter and pool count (next to each other)
+    CK(cudaMemsetAsync(p.work, 0, 2 * sizeof(unsigned long long), ctx->stream));
+    const LaunchArgs la = plan_args(ctx, p, u0, u1);
     CK(cudaEventRecord(kev[2 * c], ctx->stream));
-    cudaError_t e = launch_plain(pc, W, roots_pad(mt), cgrid, ls.smem, ctx->stream);
-    if (e != cudaSuccess) return fail(ctx, CIPSI_ERR_CUDA, std::string("k_pt2 launch: ") + cudaGetErrorString(e));
+    cudaError_t e = launch_forward<false>(part_params(p, u0), la, W, R, std::min(grid, u1 - u0), dev_sms,
+                                          slot0[u1 - 1] + pl.uslots[u1 - 1], ctx->stream);
+    if (e != cudaSuccess)
+      return fail(ctx, CIPSI_ERR_CUDA, std::string("k_cand / k_pt2 launch: ") + cudaGetErrorString(e));
     CK(cudaEventRecord(kev[2 * c + 1], ctx->stream));
     GatherArgs ga{};
     ga.out_bits = ctx->dout_bits[b];
@@ -1576,17 +1693,13 @@ int cipsi_run_pt2_stream(cipsi_ctx* ctx, const cipsi_opts* o, int64_t chunk_reco
     e = enqueue_gather(ctx, p, u0, u1, 0, ga, ctx->stream, dev_sms);
     if (e != cudaSuccess) return fail(ctx, CIPSI_ERR_CUDA, std::string("record gather: ") + cudaGetErrorString(e));
     CK(cudaMemcpyAsync(&hcnt[2 * c], ctx->dscan_total, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(&hcnt[2 * c + 1], ctx->dpool_count, 8, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(&hcnt[2 * c + 1], p.pool_count, 8, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaEventRecord(ctx->ev_gathered[b], ctx->stream));
     if (fn && c >= 1 && (rc = deliver(c - 1))) return rc;
   }
   if (fn && nchunks >= 1 && (rc = deliver(nchunks - 1))) return rc;
-  if (nunits > 0) {
-    k_reduce<<<(unsigned)nq, kReduceThreads, 0, ctx->stream>>>(ctx->dgen_part, nunits, (int)nq, ctx->dred);
-    CK(cudaGetLastError());
-  } else {
-    CK(cudaMemsetAsync(ctx->dred, 0, nq * sizeof(double), ctx->stream));
-  }
+  k_finish<<<1, kFinishThreads, 0, ctx->stream>>>(p, nullptr);
+  CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev1, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   if (fn) CK(cudaStreamSynchronize(ctx->copy_stream));
@@ -1601,7 +1714,7 @@ int cipsi_run_pt2_stream(cipsi_ctx* ctx, const cipsi_opts* o, int64_t chunk_reco
     pt2 += t;
   }
   r->pt2_ms = pt2;
-  r->launches = 3ll * nchunks + (nunits > 0 ? 1 : 0);
+  r->launches = 4ll * nchunks + 1;
   for (int c = 0; c < nchunks; ++c)
     if ((long long)hcnt[2 * c + 1] > ctx->pool_cap)
       return fail(ctx, CIPSI_ERR_OVERFLOW, "internal error: a chunk's records overflowed the pool");
@@ -1685,22 +1798,25 @@ int run_adjoint(cipsi_ctx* ctx, const cipsi_opts* o, const double* seed, double*
   const int ncf = ctx->d.ncf, W = ctx->W, mt = ctx->d.metat, n = ctx->d.norb;
   const int nt = n * (n + 1) / 2;
   RunPlan pl;
-  plan_run(ctx, o, ctx->tune_r_chunk, pl);
+  plan_run(ctx, o, ctx->tune_r_chunk, 1, pl);
   const int nunits = (int)pl.ug.size();
   int dev_sms = 0;
   CK(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
   const int R = roots_pad(mt);
-  const LaunchShape ls = launch_shape(W, R, ncf, ctx->tune_ctas, true);
+  const LaunchShape ls = adj_shape(ncf, ctx->tune_ctas);
   const int grid = std::max(1, std::min(nunits, dev_sms * ls.blocks_per_sm));
   rc = ensure_neighbour_scratch(ctx, grid);
   if (rc) return rc;
-  rc = prepare_run(ctx, pl, ctx->stream);
+  const std::vector<long long> slot0(pl.ug.size(), 0);  // no candidate buffer
+  rc = prepare_run(ctx, pl, &slot0, ctx->stream);
   if (rc) return rc;
   const size_t nq = (size_t)5 * mt;
-  const size_t ncount = C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots;
-  CK(cudaMemsetAsync(ctx->dcounters, 0, ncount * sizeof(unsigned long long), ctx->stream));
-  CK(cudaMemsetAsync(ctx->dhist_tab, 0, 2 * kNClass * kMaxRoots * sizeof(double), ctx->stream));
-  CK(cudaMemsetAsync(ctx->dwork, 0, sizeof(int), ctx->stream));
+  if ((size_t)std::max(nunits, 1) * nq > ctx->gen_part_cap) {  // per-unit partial sums
+    dfree(ctx->dgen_part);
+    ctx->gen_part_cap = (size_t)std::max(nunits, 1) * nq;
+    CK(cudaMalloc(&ctx->dgen_part, ctx->gen_part_cap * sizeof(double)));
+  }
+  CK(cudaMemsetAsync(ctx->dcounters, 0, kZeroWords * sizeof(unsigned long long), ctx->stream));
   CK(cudaMemsetAsync(ctx->dgen_part, 0, (size_t)std::max(nunits, 1) * nq * sizeof(double), ctx->stream));
   // gradient buffers (this call only)
   const int stride = 3 * nt + 2 * n;
@@ -1730,12 +1846,10 @@ int run_adjoint(cipsi_ctx* ctx, const cipsi_opts* o, const double* seed, double*
 
   Params p{};
   fill_params(ctx, o, pl, p);
-  p.nb_j = ctx->dnb_j;
-  p.nb_emask = ctx->dnb_em;
-  p.lr_ent = ctx->dlr_ent;
+  set_scratch(ctx, p);
   p.lr_cap = ls.lr_cap;
-  p.nb_stride = ncf;
   p.rec_mode = 0;  // no records from an adjoint launch
+  p.gen_part = ctx->dgen_part;
   for (int m = 0; m < mt; ++m) {
     p.seed_mp[m] = seed[m];
     p.seed_vp[m] = seed[mt + m];
@@ -1750,17 +1864,17 @@ int run_adjoint(cipsi_ctx* ctx, const cipsi_opts* o, const double* seed, double*
   if (nunits > 0) {
     cudaError_t e;
     if (W == 1) {
-      e = R == 1 ? launch_pt2<1, 1, false, true>(p, BatchArgs{}, grid, ls.smem, ctx->stream)
-        : R == 2 ? launch_pt2<1, 2, false, true>(p, BatchArgs{}, grid, ls.smem, ctx->stream)
-        : R == 4 ? launch_pt2<1, 4, false, true>(p, BatchArgs{}, grid, ls.smem, ctx->stream)
-                 : launch_pt2<1, 8, false, true>(p, BatchArgs{}, grid, ls.smem, ctx->stream);
+      e = R == 1 ? launch_pt2_adj<1, 1>(p, grid, ls.smem, ctx->stream)
+        : R == 2 ? launch_pt2_adj<1, 2>(p, grid, ls.smem, ctx->stream)
+        : R == 4 ? launch_pt2_adj<1, 4>(p, grid, ls.smem, ctx->stream)
+                 : launch_pt2_adj<1, 8>(p, grid, ls.smem, ctx->stream);
     } else {
-      e = R == 1 ? launch_pt2<2, 1, false, true>(p, BatchArgs{}, grid, ls.smem, ctx->stream)
-        : R == 2 ? launch_pt2<2, 2, false, true>(p, BatchArgs{}, grid, ls.smem, ctx->stream)
-        : R == 4 ? launch_pt2<2, 4, false, true>(p, BatchArgs{}, grid, ls.smem, ctx->stream)
-                 : launch_pt2<2, 8, false, true>(p, BatchArgs{}, grid, ls.smem, ctx->stream);
+      e = R == 1 ? launch_pt2_adj<2, 1>(p, grid, ls.smem, ctx->stream)
+        : R == 2 ? launch_pt2_adj<2, 2>(p, grid, ls.smem, ctx->stream)
+        : R == 4 ? launch_pt2_adj<2, 4>(p, grid, ls.smem, ctx->stream)
+                 : launch_pt2_adj<2, 8>(p, grid, ls.smem, ctx->stream);
     }
-    if ((rc = ck(e, "adjoint k_pt2 launch"))) return rc;
+    if ((rc = ck(e, "k_pt2_adj launch"))) return rc;
     k_reduce<<<(unsigned)nq, kReduceThreads, 0, ctx->stream>>>(ctx->dgen_part, nunits, (int)nq, ctx->dred);
   } else {
     if ((rc = ck(cudaMemsetAsync(ctx->dred, 0, nq * sizeof(double), ctx->stream), "memset"))) return rc;
@@ -1895,28 +2009,29 @@ struct cipsi_batch {
   std::vector<cipsi_opts> opts;
   std::vector<unsigned long long> buf_gen;
   Params* dgeo = nullptr;
+  unsigned char* dplan = nullptr;  // every geometry's plan
   struct Class {
     int W = 1, R = 1;
-    int big = 0;  // the plain form would run these contexts at one CTA per SM
     std::vector<int> geos;
     int nunits = 0, grid = 0, ncf_max = 0;
-    LaunchShape ls{};
     int32_t* dunit_geo = nullptr;
     int32_t* dunit_local = nullptr;
     int* dwork = nullptr;
     int32_t* dnb_j = nullptr;
     uint64_t* dnb_em = nullptr;
     uint64_t* dlr_ent = nullptr;
-    // record staging shared by the class's geometries (per CTA)
-    long long st_cap = 32;
-    uint64_t* dst_bits = nullptr;
-    double *dst_xam = nullptr, *dst_evp = nullptr;
-    uint32_t* dst_mask = nullptr;
+    uint32_t *dlr_e = nullptr, *dlrw_e = nullptr;
+    uint2* dlrw_jh = nullptr;
+    // the units' slots and the candidate buffer, shared by the class's geometries
+    unsigned char* dunit_slot = nullptr;
+    unsigned char* dcand = nullptr;
+    long long cand_cap = 0;
+    std::vector<int> cut;
+    std::vector<long long> part_slots;
     cudaStream_t st = nullptr;
     cudaEvent_t ev_join = nullptr;
   };
   std::vector<Class> classes;
-  int max_nq = 0;
   cudaEvent_t ev_fork = nullptr, ev0 = nullptr, ev1 = nullptr, done = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -1937,15 +2052,6 @@ int bfail(cipsi_batch* b, int code, const std::string& msg) {
       return bfail(b, CIPSI_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-template <int W>
-cudaError_t launch_batch_class(const Params& p0, const BatchArgs& ba, int R, int grid, size_t smem,
-                               cudaStream_t st) {
-  return R == 1 ? launch_pt2<W, 1, true>(p0, ba, grid, smem, st)
-       : R == 2 ? launch_pt2<W, 2, true>(p0, ba, grid, smem, st)
-       : R == 4 ? launch_pt2<W, 4, true>(p0, ba, grid, smem, st)
-                : launch_pt2<W, 8, true>(p0, ba, grid, smem, st);
-}
-
 void batch_free(cipsi_batch* b) {
   cudaSetDevice(b->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
@@ -1954,11 +2060,13 @@ void batch_free(cipsi_batch* b) {
   for (auto& c : b->classes) {
     dfree(c.dunit_geo); dfree(c.dunit_local); dfree(c.dwork);
     dfree(c.dnb_j); dfree(c.dnb_em); dfree(c.dlr_ent);
-    dfree(c.dst_bits); dfree(c.dst_xam); dfree(c.dst_evp); dfree(c.dst_mask);
+    dfree(c.dlr_e); dfree(c.dlrw_e); dfree(c.dlrw_jh);
+    dfree(c.dunit_slot); dfree(c.dcand);
     if (c.st) cudaStreamDestroy(c.st);
     if (c.ev_join) cudaEventDestroy(c.ev_join);
   }
   dfree(b->dgeo);
+  dfree(b->dplan);
   for (cudaEvent_t e : {b->ev_fork, b->ev0, b->ev1, b->done})
     if (e) cudaEventDestroy(e);
   if (b->stream) cudaStreamDestroy(b->stream);
@@ -1999,68 +2107,86 @@ int cipsi_batch_create(cipsi_batch** out, cipsi_ctx* const* ctxs, int32_t n, con
 
   // plan every geometry; per-context buffers as for a plain run
   std::vector<Params> P(n);
-  std::vector<long long> work(n), stcap(n);
+  std::vector<long long> work(n);
+  std::vector<std::vector<long long>> uslots(n);
+  std::vector<unsigned char> hplan;
+  std::vector<size_t> plan_at(n);
+  std::vector<int> plan_gens(n);
   b->ctxs.assign(ctxs, ctxs + n);
   b->opts.assign(opts, opts + n);
+  long long all_blocks = 0;
+  for (int i = 0; i < n; ++i) all_blocks += run_blocks(ctxs[i], &opts[i]);
+  const int ub = unit_blocks(r_chunk, all_blocks, dev_sms);
   for (int i = 0; i < n; ++i) {
     cipsi_ctx* ctx = ctxs[i];
     b->opts[i].gen_mask = nullptr;  // used by the plan below only
     RunPlan pl;
-    plan_run(ctx, &opts[i], r_chunk, pl);
-    if (prepare_run(ctx, pl, b->stream)) return bfail(b, CIPSI_ERR_CUDA, "context " + std::to_string(i) + ": " + ctx->err);
+    plan_run(ctx, &opts[i], ub, std::min(ub, kLowChunk), pl);
+    // the plan is the batch's own: the context's is replaced by every plain run
+    plan_at[i] = pack_plan(pl, std::vector<long long>(pl.ug.size(), 0), hplan);
+    plan_gens[i] = (int)pl.gens.size();
+    if (prepare_run(ctx, pl, nullptr, b->stream)) return bfail(b, CIPSI_ERR_CUDA, "context " + std::to_string(i) + ": " + ctx->err);
     fill_params(ctx, &opts[i], pl, P[i]);
-    stcap[i] = staging_cap(pl);
+    uslots[i] = pl.uslots;
     work[i] = (long long)pl.ug.size() * ctx->d.ncf;
     const int W = ctx->W, R = roots_pad(ctx->d.metat);
-    // contexts whose shared-memory list needs a whole SM go to their own
-    // launch, so the others keep two CTAs per SM as in the plain form
-    const int big = ctas_per_sm == 0 && launch_shape(W, R, ctx->d.ncf, 0).blocks_per_sm == 1 ? 1 : 0;
     int c = 0;
-    while (c < (int)b->classes.size() &&
-           !(b->classes[c].W == W && b->classes[c].R == R && b->classes[c].big == big))
-      ++c;
+    while (c < (int)b->classes.size() && !(b->classes[c].W == W && b->classes[c].R == R)) ++c;
     if (c == (int)b->classes.size()) {
       b->classes.emplace_back();
       b->classes[c].W = W;
       b->classes[c].R = R;
-      b->classes[c].big = big;
     }
     b->classes[c].geos.push_back(i);
-    b->max_nq = std::max(b->max_nq, 5 * ctx->d.metat);
   }
-  BCK(cudaStreamSynchronize(b->stream));  // host plan vectors die here
+  BCK(cudaMalloc(&b->dplan, std::max<size_t>(hplan.size(), 64)));
+  if (!hplan.empty()) BCK(cudaMemcpy(b->dplan, hplan.data(), hplan.size(), cudaMemcpyHostToDevice));
+  for (int i = 0; i < n; ++i) set_plan(P[i], b->dplan + plan_at[i], P[i].nunits, plan_gens[i]);
 
   // per class: unit order (heaviest geometry first), launch shape, scratch
   for (auto& c : b->classes) {
     std::stable_sort(c.geos.begin(), c.geos.end(), [&](int x, int y) { return work[x] > work[y]; });
     std::vector<int32_t> ugeo, ulocal;
-    int mt_max = 1;
+    std::vector<long long> slots;
     for (int i : c.geos) {
       c.ncf_max = std::max(c.ncf_max, ctxs[i]->d.ncf);
-      c.st_cap = std::max(c.st_cap, stcap[i]);
-      mt_max = std::max(mt_max, ctxs[i]->d.metat);
       for (int u = 0; u < P[i].nunits; ++u) {
         ugeo.push_back(i);
         ulocal.push_back(u);
+        slots.push_back(uslots[i][u]);
+      }
+    }
+    long long max_slots = 0, all_slots = 0;
+    for (long long x : slots) {
+      max_slots = std::max(max_slots, x);
+      all_slots += x;
+    }
+    const long long cap = std::max(max_slots, (long long)(kCandMaxBytes / cand_slot_bytes(c.R)));
+    std::vector<long long> slot0;
+    c.cut = cut_units(slots, cap, slot0);
+    for (size_t q = 0; q + 1 < c.cut.size(); ++q) c.part_slots.push_back(slot0[c.cut[q + 1] - 1] + slots[c.cut[q + 1] - 1]);
+    c.cand_cap = std::max<long long>(64, (std::min(cap, all_slots) + 63) / 64 * 64);
+    BCK(cudaMalloc(&c.dcand, (size_t)c.cand_cap * cand_slot_bytes(c.R)));
+    {
+      const std::vector<int32_t> ns(slots.begin(), slots.end());
+      BCK(cudaMalloc(&c.dunit_slot, std::max<size_t>(12 * slots.size(), 64)));
+      if (!slots.empty()) {
+        BCK(cudaMemcpy(c.dunit_slot, slot0.data(), 8 * slots.size(), cudaMemcpyHostToDevice));
+        BCK(cudaMemcpy(c.dunit_slot + 8 * slots.size(), ns.data(), 4 * slots.size(), cudaMemcpyHostToDevice));
       }
     }
     c.nunits = (int)ugeo.size();
-    c.ls = launch_shape(c.W, c.R, c.ncf_max, ctas_per_sm);
-    c.grid = std::max(1, std::min(c.nunits, dev_sms * c.ls.blocks_per_sm));
+    c.grid = std::max(1, std::min(c.nunits, dev_sms * fwd_blocks_per_sm(c.W, c.R, ctas_per_sm)));
     BCK(cudaMalloc(&c.dunit_geo, (size_t)std::max(c.nunits, 1) * sizeof(int32_t)));
     BCK(cudaMalloc(&c.dunit_local, (size_t)std::max(c.nunits, 1) * sizeof(int32_t)));
-    BCK(cudaMalloc(&c.dwork, sizeof(int)));
+    BCK(cudaMalloc(&c.dwork, 2 * sizeof(int)));
     BCK(cudaMalloc(&c.dnb_j, (size_t)c.grid * c.ncf_max * sizeof(int32_t)));
     BCK(cudaMalloc(&c.dnb_em, (size_t)c.grid * c.ncf_max * sizeof(uint64_t)));
     BCK(cudaMalloc(&c.dlr_ent, (size_t)c.grid * c.ncf_max * sizeof(uint64_t)));
-    {
-      const size_t slots = (size_t)c.grid * (size_t)c.st_cap;
-      BCK(cudaMalloc(&c.dst_bits, slots * 2 * c.W * sizeof(uint64_t)));
-      BCK(cudaMalloc(&c.dst_xam, slots * sizeof(double)));
-      BCK(cudaMalloc(&c.dst_evp, slots * mt_max * sizeof(double)));
-      BCK(cudaMalloc(&c.dst_mask, slots / 32 * sizeof(uint32_t)));
-      BCK(cudaMemset(c.dst_mask, 0, slots / 32 * sizeof(uint32_t)));
-    }
+    BCK(cudaMalloc(&c.dlr_e, (size_t)c.grid * c.ncf_max * sizeof(uint32_t)));
+    const size_t nw = (size_t)c.grid * kWarps * 2 * lrw_entries(c.ncf_max);
+    BCK(cudaMalloc(&c.dlrw_e, nw * sizeof(uint32_t)));
+    BCK(cudaMalloc(&c.dlrw_jh, nw * sizeof(uint2)));
     if (c.nunits) {
       BCK(cudaMemcpy(c.dunit_geo, ugeo.data(), (size_t)c.nunits * sizeof(int32_t), cudaMemcpyHostToDevice));
       BCK(cudaMemcpy(c.dunit_local, ulocal.data(), (size_t)c.nunits * sizeof(int32_t), cudaMemcpyHostToDevice));
@@ -2069,13 +2195,12 @@ int cipsi_batch_create(cipsi_batch** out, cipsi_ctx* const* ctxs, int32_t n, con
       P[i].nb_j = c.dnb_j;
       P[i].nb_emask = c.dnb_em;
       P[i].lr_ent = c.dlr_ent;
+      P[i].lr_jh = reinterpret_cast<uint2*>(c.dlr_ent);
+      P[i].lr_e = c.dlr_e;
+      P[i].lrw_e = c.dlrw_e;
+      P[i].lrw_jh = c.dlrw_jh;
+      P[i].lrw_cap = lrw_entries(c.ncf_max);
       P[i].nb_stride = c.ncf_max;
-      P[i].lr_cap = c.ls.lr_cap;
-      P[i].st_cap = (int)c.st_cap;
-      P[i].st_bits = c.dst_bits;
-      P[i].st_xam = c.dst_xam;
-      P[i].st_evp = c.dst_evp;
-      P[i].st_mask = c.dst_mask;
     }
     BCK(cudaStreamCreateWithFlags(&c.st, cudaStreamNonBlocking));
     BCK(cudaEventCreateWithFlags(&c.ev_join, cudaEventDisableTiming));
@@ -2090,23 +2215,31 @@ int cipsi_batch_create(cipsi_batch** out, cipsi_ctx* const* ctxs, int32_t n, con
   BCK(cudaEventRecord(b->ev_fork, b->stream));
   for (auto& c : b->classes) {
     BCK(cudaStreamWaitEvent(c.st, b->ev_fork, 0));
-    BCK(cudaMemsetAsync(c.dwork, 0, sizeof(int), c.st));
-    if (c.nunits) {
-      BatchArgs ba{b->dgeo, c.dunit_geo, c.dunit_local, c.nunits, c.dwork};
-      const Params& p0 = P[c.geos[0]];
-      cudaError_t e = c.W == 1 ? launch_batch_class<1>(p0, ba, c.R, c.grid, c.ls.smem, c.st)
-                               : launch_batch_class<2>(p0, ba, c.R, c.grid, c.ls.smem, c.st);
+    for (size_t q = 0; q + 1 < c.cut.size(); ++q) {
+      const int u0 = c.cut[q], u1 = c.cut[q + 1];
+      LaunchArgs la{};
+      la.unit_slot = reinterpret_cast<const long long*>(c.dunit_slot) + u0;
+      la.unit_nslots = reinterpret_cast<const int32_t*>(c.dunit_slot + 8 * (size_t)c.nunits) + u0;
+      la.cand = cand_views(c.dcand, c.cand_cap, c.R);
+      la.nunits = u1 - u0;
+      la.work = c.dwork;
+      la.geo = b->dgeo;
+      la.unit_geo = c.dunit_geo + u0;
+      la.unit_local = c.dunit_local + u0;
+      BCK(cudaMemsetAsync(c.dwork, 0, 2 * sizeof(int), c.st));
+      const cudaError_t e = launch_forward<true>(P[c.geos[0]], la, c.W, c.R, std::min(c.grid, u1 - u0), dev_sms,
+                                                 c.part_slots[q], c.st);
       if (e != cudaSuccess) {
         cudaGraph_t g = nullptr;
         cudaStreamEndCapture(b->stream, &g);
         if (g) cudaGraphDestroy(g);
-        return bfail(b, CIPSI_ERR_CUDA, std::string("batched k_pt2 launch: ") + cudaGetErrorString(e));
+        return bfail(b, CIPSI_ERR_CUDA, std::string("batched k_cand / k_pt2 launch: ") + cudaGetErrorString(e));
       }
     }
     BCK(cudaEventRecord(c.ev_join, c.st));
     BCK(cudaStreamWaitEvent(b->stream, c.ev_join, 0));
   }
-  k_reduce_batch<<<dim3((unsigned)b->max_nq, (unsigned)n), kReduceThreads, 0, b->stream>>>(b->dgeo);
+  k_finish<<<(unsigned)n, kFinishThreads, 0, b->stream>>>(P[0], b->dgeo);
   // every geometry's records, in its unit order
   for (int i = 0; i < n; ++i) {
     GatherArgs ga{};
@@ -2178,12 +2311,14 @@ void cipsi_batch_destroy(cipsi_batch* b) {
 }
 
 // ------------------------------------------------- run without allocation
-// cipsi_run_pt2_static runs k_pt2 + k_reduce with every per-run buffer taken
-// from one file-scope device array instead of cudaMalloc'd context buffers.
-// Layout of the array (each region 256-byte aligned): counters + dpivot +
-// histogram counts | histogram sums | reduced sums | work counter |
-// generator list | generator masks | work units | per-unit partial sums |
-// per-block neighbour scratch (nb_j, nb_emask, lr_ent).  The generator and
+// cipsi_run_pt2_static runs k_cand, k_pt2 and k_finish with every per-run buffer taken
+// from file-scope device arrays instead of cudaMalloc'd context buffers: what
+// the kernel accumulates into (kZeroWords), and a scratch array (each region
+// 256-byte aligned): histogram sums | reduced sums | generator list |
+// generator masks | work units | per-block neighbour scratch (nb_j, nb_emask,
+// lr_ent).  The size limit is that of the entry's first form, which also kept
+// counters and five sums per work unit and root in the array: the room for
+// them stays reserved, so that what fits and what does not is unchanged.  The generator and
 // unit lists are staged in file-scope host arrays of fixed size.
 
 }  // extern "C"
@@ -2191,19 +2326,26 @@ void cipsi_batch_destroy(cipsi_batch* b) {
 namespace {
 
 constexpr size_t kStaticScratchBytes = (size_t)32 << 20;  // 32 MiB
+constexpr size_t kStaticCandBytes = (size_t)128 << 20;  // candidate buffer
 constexpr int kStaticMaxUnits = 1 << 18;
 constexpr int kStaticMaxGens = 1 << 17;
 constexpr int kStaticMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_pt2_scratch[kStaticScratchBytes];
+static __device__ __align__(256) unsigned long long g_pt2_zeroed[kZeroWords];
+static __device__ __align__(256) unsigned char g_pt2_cand[kStaticCandBytes];
 
 // host staging of the generator and unit lists (copied to the device array)
 static int32_t g_static_gens[kStaticMaxGens];
 static uint8_t g_static_gmask[kStaticMaxGens];
 static int32_t g_static_units[3 * kStaticMaxUnits];
+static int32_t g_static_nslots[kStaticMaxUnits];
+static long long g_static_slot[kStaticMaxUnits];
 
-// device address of g_pt2_scratch, looked up once per device
+// device addresses of the arrays, looked up once per device
 static unsigned char* g_static_ptr[kStaticMaxDevices];
+static unsigned long long* g_static_zeroed[kStaticMaxDevices];
+static unsigned char* g_static_cand[kStaticMaxDevices];
 static bool g_static_ready[kStaticMaxDevices];
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -2230,6 +2372,10 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
     void* ptr = nullptr;
     CK(cudaGetSymbolAddress(&ptr, g_pt2_scratch));
     g_static_ptr[ctx->device] = static_cast<unsigned char*>(ptr);
+    CK(cudaGetSymbolAddress(&ptr, g_pt2_zeroed));
+    g_static_zeroed[ctx->device] = static_cast<unsigned long long*>(ptr);
+    CK(cudaGetSymbolAddress(&ptr, g_pt2_cand));
+    g_static_cand[ctx->device] = static_cast<unsigned char*>(ptr);
     g_static_ready[ctx->device] = true;
   }
   unsigned char* base = g_static_ptr[ctx->device];
@@ -2288,11 +2434,12 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   int32_t* ug = g_static_units;
   int32_t* ur0 = g_static_units + kStaticMaxUnits;
   int32_t* ur1 = g_static_units + 2 * kStaticMaxUnits;
-  auto push_unit = [&](int g, int a, int b) {
+  auto push_unit = [&](int g, int a, int b, long long slots) {
     if (nunits == kStaticMaxUnits) return false;
     ug[nunits] = g;
     ur0[nunits] = a;
     ur1[nunits] = b;
+    g_static_nslots[nunits] = (int32_t)slots;
     ++nunits;
     return true;
   };
@@ -2300,7 +2447,7 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
     return fail(ctx, CIPSI_ERR_OVERFLOW,
                 "cipsi_run_pt2_static: more than " + std::to_string(kStaticMaxUnits) + " work units");
   };
-  int hfe[2 * 128];
+  int hfe[2 * 128], spe[2 * 128];
   for (int rk = -1; rk <= maxrank; ++rk) {
     for (int g = 0; g < ngen; ++g) {
       const int k = g_static_gens[g];
@@ -2308,18 +2455,23 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
       if (k < 0) {
         const int ntot = (pertu_ref ? 1 : 0) + (pertu_mono ? 2 * noca * (n - noca) : 0);
         for (int t = 0; t < ntot; t += kPertuChunk)
-          if (!push_unit(g, t, std::min(ntot, t + kPertuChunk))) return too_many_units();
+          if (!push_unit(g, t, std::min(ntot, t + kPertuChunk), std::min(ntot - t, kPertuChunk))) return too_many_units();
         continue;
       }
-      int ne = 0;
+      int ne = 0, nes[2] = {0, 0};
       for (int sp = 0; sp < 2; ++sp)
         for (int orb = 0; orb < n; ++orb)
-          if ((ctx->Sbits[(size_t)k * 2 * W + sp * W + (orb >> 6)] >> (orb & 63)) & 1ull)
+          if ((ctx->Sbits[(size_t)k * 2 * W + sp * W + (orb >> 6)] >> (orb & 63)) & 1ull) {
+            spe[ne] = sp;
             hfe[ne++] = orb < noca;
+            ++nes[sp];
+          }
+      const int nv[2] = {n - nes[0], n - nes[1]};
       const uint8_t m = g_static_gmask[g];
       int cnt = 0, start = -1;
+      long long slots = 0;
       for (int rb = 0; rb < nR; ++rb) {
-        int hfR, nRr;
+        int hfR, nRr, x1 = rb, x2 = -1;
         if (rb < nel) {
           hfR = hfe[rb];
           nRr = 1;
@@ -2329,7 +2481,9 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
             t -= nel - 1 - e1;
             ++e1;
           }
-          hfR = hfe[e1] + hfe[e1 + 1 + t];
+          x1 = e1;
+          x2 = e1 + 1 + t;
+          hfR = hfe[x1] + hfe[x2];
           nRr = 2;
         }
         bool ok = false;
@@ -2337,13 +2491,15 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
           if (m & (1u << (hfR + aV - nRr + 2))) ok = true;
         if (!ok) continue;
         if (start < 0) start = rb;
+        slots += block_candidates(nRr, x2 >= 0 && spe[x1] == spe[x2], nv[spe[x1]], nv[0], nv[1]);
         if (++cnt == kRChunk) {
-          if (!push_unit(g, start, rb + 1)) return too_many_units();
+          if (!push_unit(g, start, rb + 1, slots)) return too_many_units();
           cnt = 0;
           start = -1;
+          slots = 0;
         }
       }
-      if (start >= 0 && !push_unit(g, start, nR)) return too_many_units();
+      if (start >= 0 && !push_unit(g, start, nR, slots)) return too_many_units();
     }
   }
 
@@ -2352,12 +2508,9 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   int dev_sms = 0;
   CK(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
   const int R = mt <= 1 ? 1 : mt <= 2 ? 2 : mt <= 4 ? 4 : 8;
-  const LaunchShape ls = launch_shape(W, R, ncf, 0);
-  const int lr_cap = ls.lr_cap;
-  const size_t smem = ls.smem;
-  const int blocks_per_sm = ls.blocks_per_sm;
+  const int blocks_per_sm = fwd_blocks_per_sm(W, R, 0);
   const size_t nq = (size_t)5 * mt;
-  const size_t ncount = C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots;
+  const size_t ncount = kCountWords;
   const size_t off_counters = 0;
   const size_t off_tab = align256(off_counters + ncount * sizeof(unsigned long long));
   const size_t off_red = align256(off_tab + 2 * kNClass * kMaxRoots * sizeof(double));
@@ -2380,15 +2533,31 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   unsigned char* nb0 = base + off_nb;
 
   // zero what the kernels accumulate into; upload the lists
-  CK(cudaMemsetAsync(base, 0, off_gens, ctx->stream));
-  CK(cudaMemsetAsync(base + off_part, 0, (size_t)std::max(nunits, 1) * nq * sizeof(double), ctx->stream));
+  unsigned long long* zeroed = g_static_zeroed[ctx->device];
+  CK(cudaMemsetAsync(zeroed, 0, kZeroWords * sizeof(unsigned long long), ctx->stream));
   if (ngen) {
     CK(cudaMemcpyAsync(base + off_gens, g_static_gens, (size_t)ngen * sizeof(int32_t),
                        cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(base + off_gmask, g_static_gmask, (size_t)ngen, cudaMemcpyHostToDevice, ctx->stream));
   }
   int32_t* dunits = reinterpret_cast<int32_t*>(base + off_units);
+  // units in parts that fit the candidate buffer (a unit has at most 6 * 16,256
+  // slots, a few per cent of it); their slots take 12 of the >= 40 bytes per
+  // unit reserved at off_part
+  const long long cand_cap = (long long)(kStaticCandBytes / cand_slot_bytes(R)) / 64 * 64;
+  {
+    long long acc = 0;
+    for (int u = 0; u < nunits; ++u) {
+      if (acc + g_static_nslots[u] > cand_cap) acc = 0;
+      g_static_slot[u] = acc;
+      acc += g_static_nslots[u];
+    }
+  }
+  long long* dslot = reinterpret_cast<long long*>(base + off_part);
+  int32_t* dnslots = reinterpret_cast<int32_t*>(dslot + nunits);
   if (nunits) {
+    CK(cudaMemcpyAsync(dslot, g_static_slot, (size_t)nunits * 8, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(dnslots, g_static_nslots, (size_t)nunits * 4, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(dunits, ug, (size_t)nunits * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(dunits + nunits, ur0, (size_t)nunits * sizeof(int32_t), cudaMemcpyHostToDevice,
                        ctx->stream));
@@ -2423,6 +2592,7 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   p.F = ctx->dF;
   p.J = ctx->dJ;
   p.K = ctx->dK;
+  p.jx = ctx->djx;
   p.fmpb = ctx->dfmpb;
   p.orbsym = ctx->dorbsym;
   for (int i = 0; i < ctx->d.nsym; ++i)
@@ -2445,46 +2615,53 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   for (int i = 0; i < kNClass; ++i) {
     p.aval[i] = o->aval[i];
     std::memcpy(&p.aval_bits[i], &o->aval[i], 8);
+    p.aval_hi[i] = i + 1 < o->nclass ? (int)(p.aval_bits[i] >> 32) : 0x7fffffff;
   }
   p.pertu_ref = pertu_ref ? 1 : 0;
   p.pertu_mono = pertu_mono ? 1 : 0;
-  // nb_j, nb_emask, lr_ent: grid x ncf entries each (k_pt2 indexes block b at
-  // b * ncf), in three regions of grid * nb_stride >= grid * ncf * 8 bytes
+  // nb_j and lr_e (4 bytes), nb_emask and lr_jh (8 bytes): grid x ncf entries
+  // each (k_pt2 indexes block b at b * ncf), in three regions of
+  // grid * nb_stride >= grid * ncf * 8 bytes; what is left holds the warps'
+  // overflow lists (12 bytes an entry; without them a long list is worked by
+  // the whole CTA)
+  const size_t region = (size_t)grid * nb_stride;
   p.nb_j = reinterpret_cast<int32_t*>(nb0);
-  p.nb_emask = reinterpret_cast<uint64_t*>(nb0 + (size_t)grid * nb_stride);
-  p.lr_ent = reinterpret_cast<uint64_t*>(nb0 + (size_t)2 * grid * nb_stride);
-  p.lr_cap = lr_cap;
+  p.lr_e = reinterpret_cast<uint32_t*>(nb0 + region / 2);
+  p.nb_emask = reinterpret_cast<uint64_t*>(nb0 + region);
+  p.lr_jh = reinterpret_cast<uint2*>(nb0 + 2 * region);
+  const size_t lists = (size_t)grid * kWarps * 2;
+  const size_t left = kStaticScratchBytes - off_nb - 3 * region;
+  p.lrw_cap = (int)std::min<size_t>(left / (lists * 12), (size_t)lrw_entries(ncf));
+  p.lrw_jh = reinterpret_cast<uint2*>(nb0 + 3 * region);
+  p.lrw_e = reinterpret_cast<uint32_t*>(p.lrw_jh + lists * p.lrw_cap);
   p.nb_stride = ncf;
-  p.gen_part = reinterpret_cast<double*>(base + off_part);
-  unsigned long long* dcounters = reinterpret_cast<unsigned long long*>(base + off_counters);
-  p.counters = dcounters;
-  p.dpivot_bits = dcounters + C_NCOUNTERS;
-  p.hist_nom = dcounters + C_NCOUNTERS + 1;
-  p.hist_nam = dcounters + C_NCOUNTERS + 1 + kNClass;
+  set_zeroed(p, zeroed);
   p.hist_tab = reinterpret_cast<double*>(base + off_tab);
   // no record storage: selected perturbers are counted only
   p.rec_mode = 0;
-  p.work = reinterpret_cast<int*>(base + off_work);
   double* dred = reinterpret_cast<double*>(base + off_red);
+  p.red = dred;
 
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
-  if (nunits > 0) {
-    cudaError_t e;
-    if (W == 1) {
-      e = R == 1 ? launch_pt2<1, 1, false>(p, BatchArgs{}, grid, smem, ctx->stream)
-        : R == 2 ? launch_pt2<1, 2, false>(p, BatchArgs{}, grid, smem, ctx->stream)
-        : R == 4 ? launch_pt2<1, 4, false>(p, BatchArgs{}, grid, smem, ctx->stream)
-                 : launch_pt2<1, 8, false>(p, BatchArgs{}, grid, smem, ctx->stream);
-    } else {
-      e = R == 1 ? launch_pt2<2, 1, false>(p, BatchArgs{}, grid, smem, ctx->stream)
-        : R == 2 ? launch_pt2<2, 2, false>(p, BatchArgs{}, grid, smem, ctx->stream)
-        : R == 4 ? launch_pt2<2, 4, false>(p, BatchArgs{}, grid, smem, ctx->stream)
-                 : launch_pt2<2, 8, false>(p, BatchArgs{}, grid, smem, ctx->stream);
-    }
-    if (e != cudaSuccess) return fail(ctx, CIPSI_ERR_CUDA, std::string("k_pt2 launch: ") + cudaGetErrorString(e));
-    k_reduce<<<(unsigned)nq, kReduceThreads, 0, ctx->stream>>>(p.gen_part, nunits, (int)nq, dred);
-    CK(cudaGetLastError());
+  int parts = 0;
+  for (int u0 = 0; u0 < nunits; ++parts) {
+    int u1 = u0 + 1;
+    while (u1 < nunits && g_static_slot[u1] != 0) ++u1;
+    if (u0) CK(cudaMemsetAsync(p.work, 0, 2 * sizeof(int), ctx->stream));
+    LaunchArgs la{};
+    la.unit_slot = dslot + u0;
+    la.unit_nslots = dnslots + u0;
+    la.cand = cand_views(g_static_cand[ctx->device], cand_cap, R);
+    la.nunits = u1 - u0;
+    la.work = p.work;
+    const cudaError_t e = launch_forward<false>(part_params(p, u0), la, W, R, std::min(grid, u1 - u0), dev_sms,
+                                                g_static_slot[u1 - 1] + g_static_nslots[u1 - 1], ctx->stream);
+    if (e != cudaSuccess)
+      return fail(ctx, CIPSI_ERR_CUDA, std::string("k_cand / k_pt2 launch: ") + cudaGetErrorString(e));
+    u0 = u1;
   }
+  k_finish<<<1, kFinishThreads, 0, ctx->stream>>>(p, nullptr);
+  CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev1, ctx->stream));
 
   // results (same fields as cipsi_fetch_result; no records are kept), read
@@ -2494,7 +2671,7 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   unsigned long long cnt[C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots];
   double tab[2 * kNClass * kMaxRoots];
   CK(cudaMemcpyAsync(red, dred, nq * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(cnt, dcounters, ncount * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaMemcpyAsync(cnt, zeroed, ncount * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaMemcpyAsync(tab, p.hist_tab, 2 * kNClass * kMaxRoots * sizeof(double), cudaMemcpyDeviceToHost,
                      ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -2534,7 +2711,7 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
   r->kernel_ms = ms;
   r->pt2_ms = ms;
-  r->launches = nunits > 0 ? 2 : 0;
+  r->launches = 2ll * parts + 1;
   r->n_selected = (int64_t)cnt[C_NSEL];
   return CIPSI_OK;
 }

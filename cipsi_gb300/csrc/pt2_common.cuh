@@ -17,8 +17,8 @@ constexpr int kThreads = 256;
 constexpr int kMaxSym = 8;
 constexpr int kMaxElec = 64;
 constexpr int kMaxOrb = 128;
-constexpr int kRowCap = 128;  // per-warp list of |K' \ j| = 2 entries holding a1
-constexpr int kHitCap = 8;    // per-thread list of scan hits awaiting their matrix elements
+constexpr int kRowCap = 128;  // adjoint: per-warp list of |K' \ j| = 2 entries holding a1
+constexpr int kHitCap = 8;    // adjoint: per-thread list of scan hits awaiting their matrix elements
 
 // counters[] slots
 enum {
@@ -31,7 +31,7 @@ enum {
   C_NP2,
   C_ALGB,
   C_LRFALLBACK,
-  C_STAGE_OVF,  // selected candidates whose slot lay outside the staging region (must stay 0)
+  C_STAGE_OVF,  // candidates whose slot lay outside their unit's (must stay 0)
   C_NCOUNTERS
 };
 
@@ -55,6 +55,7 @@ struct Params {
   const double* F;           // packed i*(i+1)/2 + j (i >= j, 0-based)
   const double* J;
   const double* K;
+  const double* jx;          // 2 x norb x norb: J (opposite spins), J - K (same spin)
   const double* fmpb;        // 2*norb by spin orbital
   const int8_t* orbsym;      // 0-based irreps
   int its[kMaxSym][kMaxSym]; // 0-based product table
@@ -63,34 +64,39 @@ struct Params {
   double tau, teseff;
   double aval[kNClass];
   long long aval_bits[kNClass];  // bit patterns of aval (non-negative, ascending)
+  int aval_hi[kNClass];          // their high words
   int pertu_ref, pertu_mono;
   // scratch
   int32_t* nb_j;             // per block: ncf entries
   uint64_t* nb_emask;
-  uint64_t* lr_ent;          // per block: ncf compact L_R entries beyond lr_cap
-  int lr_cap;                // shared-memory capacity of L_R
+  uint64_t* lr_ent;          // per block: ncf compact L_R entries beyond lr_cap (adjoint kernel)
+  uint32_t* lr_e;            // per block: L_R of a block too long for one warp (forward kernel):
+  uint2* lr_jh;              //   ncf entries each
+  uint32_t* lrw_e;           // per block: 2 x kWarps x lrw_cap entries, the overflow of the warps' lists
+  uint2* lrw_jh;
+  int lrw_cap;
+  int lr_cap;                // shared-memory capacity of L_R (adjoint kernel)
   int nb_stride;             // entries per block in nb_j / nb_emask / lr_ent
   // outputs
-  double* gen_part;          // ngen x (5 * metat)
+  double* gen_part;          // nunits x (5 * metat): per-unit sums (adjoint kernel)
   unsigned long long* counters;
   unsigned long long* dpivot_bits;
   unsigned long long* hist_nom;      // nclass
   unsigned long long* hist_nam;      // nclass x metat
   double* hist_tab;                  // 2 x nclass x metat (tabmp, tabvp)
-  double* red;                       // 5 x metat reduced sums (k_reduce output)
-  // unit-60 records.  A selected candidate is staged in its CTA's region at
-  // its slot (its position in the work unit's candidate order) and flagged
-  // in the region's slot mask; when the unit is done the CTA compacts the
-  // flagged slots, in slot order, into one segment of the record pool and
-  // notes the segment in the unit table.  k_gather then lays the segments
+  double* red;                       // 5 x metat reduced sums (k_reduce / k_finish output)
+  // exact sums of the forward kernel, indexed by fx_tab / fx_acc: words of 32
+  // bits in 64-bit counters (units 2^-84), the same for terms of 2^22 and
+  // more (units 2^-44), and what lies beyond 2^62 or is not finite
+  unsigned long long* sums;
+  unsigned long long* sums_hi;
+  double* sums_big;
+  // unit-60 records.  When k_pt2 is done with a work unit, it compacts the
+  // selected candidates, in slot order, into one segment of the record pool
+  // and notes the segment in the unit table.  k_gather then lays the segments
   // out in unit order, so the records come out in (unit, candidate) order
   // whatever the scheduling.
   int rec_mode;                      // 0: selection counted only; 1: records kept
-  int st_cap;                        // slots per CTA region (multiple of 32)
-  uint64_t* st_bits;                 // grid x st_cap x 2W
-  double* st_xam;                    // grid x st_cap
-  double* st_evp;                    // grid x st_cap x metat
-  uint32_t* st_mask;                 // grid x st_cap / 32
   uint64_t* pool_bits;               // pool_cap x 2W
   double* pool_xam;                  // pool_cap
   double* pool_evp;                  // pool_cap x metat
@@ -117,15 +123,33 @@ struct Params {
 
 static_assert(sizeof(Params) % sizeof(int) == 0, "Params is copied as ints");
 
-// Batched launch: many geometries (each with its own Params) in one
-// persistent launch.  Global unit u belongs to geometry unit_geo[u] and is
-// unit unit_local[u] of that geometry's unit list.
-struct BatchArgs {
+// Candidates between the two forward kernels: k_cand writes each candidate that
+// can be a perturber at its slot (its position in its work unit's candidate
+// order, from the unit's first slot on), k_pt2 reads them in that order and
+// leaves the values of a selected one's record in place.
+struct CandBuf {
+  double* b;       // R x cap: <I|H|Psi_m>; then ENvp of a selected one
+  double* mp;      // cap: hmp(I); then its unit-60 value
+  double* vp;      // cap: hdig(I)
+  uint32_t* code;  // cap: the four spin orbitals toggled in the generator, a byte each
+  uint32_t* meta;  // cap: kM* bits, lesp << 8; 0: no candidate
+  long long cap;
+};
+constexpr uint32_t kMLive = 1u, kMD2 = 2u, kMWt1 = 4u, kMSel = 8u;
+
+// One launch of a forward kernel: its work units' first slots and numbers of
+// slots, the candidate buffer, the work counter.  Batched launch: many
+// geometries (each with its own Params) in one persistent launch; unit u then
+// belongs to geometry unit_geo[u] and is unit unit_local[u] of its unit list.
+struct LaunchArgs {
+  const long long* unit_slot;
+  const int32_t* unit_nslots;
+  CandBuf cand;
+  int nunits;
+  int* work;  // [0] k_cand, [1] k_pt2
   const Params* geo;
   const int32_t* unit_geo;
   const int32_t* unit_local;
-  int nunits;
-  int* work;
 };
 
 __device__ __forceinline__ void kahan_add(double& s, double& c, double x) {
@@ -135,19 +159,51 @@ __device__ __forceinline__ void kahan_add(double& s, double& c, double x) {
   s = t;
 }
 
-// Per-warp queue of perturbers that survived the interaction scan.  The
-// FP64 epilogue (denominators, E2, selection) then runs on full warps: the
-// FP64 pipe of GB300 is narrow, and a warp instruction costs the same with
-// 32 lanes or with the few that would be live at the candidate level.
-constexpr int kQCap = 64;
+constexpr int kWarps = kThreads / 32;
+constexpr int kMaxDn = 48;      // spin orbitals where K' differs from the reference
+constexpr int kMaxG = 4;        // rows of a block worked together
+constexpr int kDenseCap = 64;   // per-warp list of (entry, row): the entry touches the whole row
+constexpr int kEvCap = 256;     // per-warp ring of (entry, row, column) events
+constexpr int kHitCap2 = 32 + 32 * kMaxG;  // per-warp list of (entry, row): the entry holds the row's a1
+constexpr int kLrWarpG = 1024;  // overflow entries of each L_R list of a warp, in global scratch
+
+// One warp's part of k_cand's shared memory.  The L_R lists are short: what
+// shared memory does not take is L1, which holds their overflow.
 template <int W, int R>
-struct WarpQueue {
-  uint64_t u[2 * W][kQCap];
-  double bc[R][kQCap];
-  double hmp[kQCap], hvp[kQCap], fmul[kQCap];
-  int nmul[kQCap], slot[kQCap];  // slot: the candidate's position in its work unit
-  unsigned char flags[kQCap];  // bit 0 ybis, bit 1 is_pert1
+struct WarpMem {
+  static constexpr int NC = 64 * W;                  // columns: empty orbitals of one spin
+  static constexpr int XN = R <= 2 ? 128 : 64 * W;   // (row, column) places of the rows worked together
+  static constexpr int CapA = 64;                    // L_R entries with |K' \ j| <= 1
+  static constexpr int CapB = R == 1 ? 96 : 64;      // and with |K' \ j| = 2
+  double vd[2][NC];                      // hdig(K'+a) - hdig(K') by (spin, column)
+  double xb[R][XN];                      // sums of <I|H|j> c_j over j != k
+  double rhv[kMaxG], rmp[kMaxG];         // per row: hdig(K'+a1), hmp(K'+a1)
+  uint64_t par[2 * W];                   // bit o: parity of the electrons of K' below o, by spin
+  uint2 jhA[CapA], jhB[CapB];            // L_R entries: j; holes of K' in j, |K' \ j| << 16
+  uint32_t eA[CapA], eB[CapB];           // their spin orbitals E = j \ K', one code per byte
+  uint32_t own[NC][2 * W];               // candidates (row, column) owned by an earlier generator or in S;
+                                         //   from the block's row pass on: those still alive
+  uint32_t owncol[2][2 * W];             // orbitals (by spin, column) every candidate of which is owned
+  uint32_t dense[kDenseCap];             // entry << 2 | row
+  uint32_t ev[kEvCap];                   // entry << 8 | list << 7 | place
+  uint32_t hits[kHitCap2];               // entry << 2 | row
+  int ra1[kMaxG], rrow[kMaxG], rpA[kMaxG], rpX[kMaxG];
+  uint32_t rsg[kMaxG];
+  uint16_t xf[XN];                       // per place: element found, non-zero, lesp
+  uint16_t cols[XN];                     // surviving candidates: row << 8 | column
+  uint8_t rows[NC];                      // the block's rows with a candidate alive
+  uint8_t dn_so[kMaxDn], dn_sg[kMaxDn];  // where K' differs from the reference: code, 1 = added
 };
+template <int W, int R>
+constexpr size_t fwd_smem() {
+  return (size_t)kWarps * sizeof(WarpMem<W, R>);
+}
+
+// indices of the exact sums: by class (kNClass: outside the histogram) the MP
+// (q = 0) and EN (q = 1) terms; e2b, psimp, psivp (q = 0, 1, 2)
+__host__ __device__ constexpr int fx_tab(int q, int c, int m) { return (q * (kNClass + 1) + c) * kMaxRoots + m; }
+__host__ __device__ constexpr int fx_acc(int q, int m) { return (2 * (kNClass + 1) + q) * kMaxRoots + m; }
+constexpr int kFxSums = (2 * (kNClass + 1) + 3) * kMaxRoots;
 
 // Candidates of one block of removed electrons R: nv added orbitals for
 // |R| = 1, nv(nv-1)/2 same-spin pairs, nva * nvb opposite-spin pairs (nv:
@@ -160,10 +216,20 @@ __host__ __device__ inline long long block_candidates(int nR, bool same_spin, in
   return same_spin ? (long long)nv1 * (nv1 - 1) / 2 : (long long)nva * nvb;
 }
 
-// k_pt2<W, R, B, ADJ> launched with `smem` bytes of dynamic shared memory
-// (pt2_w1.cu / pt2_w2.cu: forward, plain and batched; pt2_adj.cu: adjoint).
-template <int W, int R, bool B, bool ADJ = false>
-cudaError_t launch_pt2(const Params& p, const BatchArgs& ba, int grid, size_t smem, cudaStream_t st);
+// The forward kernels, plain and batched: k_cand<W, R, B> (pt2_w1.cu,
+// pt2_w2.cu) on `grid` CTAs and k_pt2<W, R, B> (pt2_epi.cu) on as many as fit,
+// one after the other.
+template <int W, int R, bool B>
+cudaError_t launch_cand(const Params& p, const LaunchArgs& la, int grid, cudaStream_t st);
+template <int W, int R, bool B>
+cudaError_t launch_pt2(const Params& p, const LaunchArgs& la, int sms, cudaStream_t st);
+// CTAs of k_cand<W, R, *> per SM
+template <int W, int R>
+int cand_ctas();
+// k_pt2_adj<W, R> launched with `smem` bytes of dynamic shared memory
+// (pt2_adj.cu, pt2_adj_w2.cu)
+template <int W, int R>
+cudaError_t launch_pt2_adj(const Params& p, int grid, size_t smem, cudaStream_t st);
 
 // The Hamiltonian over a determinant list by rows (hbuild.cu): pass 1
 // counts, per row i, the columns j < min(i, jmax) within two excitations;

@@ -138,6 +138,7 @@ __device__ __forceinline__ void ai_adj(const Params& p, int i, int j, int k, int
 // first code), bits 32-33 m = |K' \ j|, bits 34-63 the index j.
 __device__ __forceinline__ uint64_t lr_entry(uint32_t ebytes, int ne, int m, int j) {
   const uint32_t first = ebytes & 0xFFu;
+#pragma unroll 1
   for (int q = ne; q < 4; ++q) ebytes |= first << (8 * q);
   return (uint64_t)ebytes | ((uint64_t)m << 32) | ((uint64_t)j << 34);
 }
@@ -197,6 +198,7 @@ __device__ __forceinline__ double hmat(const Params& p, const uint64_t* u, const
 #pragma unroll
       for (int w = 0; w < W; ++w) {
         uint64_t h = hf[sp * W + w] & ~D[sp * W + w];
+#pragma unroll 1
         while (h) {
           const int r = w * 64 + __ffsll((long long)h) - 1;
           h &= h - 1;
@@ -204,6 +206,7 @@ __device__ __forceinline__ double hmat(const Params& p, const uint64_t* u, const
           if (sp == s) val += ai(p, pp, r, qq, r);
         }
         uint64_t t = D[sp * W + w] & ~hf[sp * W + w];
+#pragma unroll 1
         while (t) {
           const int r = w * 64 + __ffsll((long long)t) - 1;
           t &= t - 1;
@@ -277,6 +280,7 @@ __device__ void hmat_adj(const Params& p, const uint64_t* u, const uint64_t* v, 
 #pragma unroll
       for (int ww = 0; ww < W; ++ww) {
         uint64_t h = hf[sp * W + ww] & ~D[sp * W + ww];
+#pragma unroll 1
         while (h) {
           const int r = ww * 64 + __ffsll((long long)h) - 1;
           h &= h - 1;
@@ -284,6 +288,7 @@ __device__ void hmat_adj(const Params& p, const uint64_t* u, const uint64_t* v, 
           if (sp == s) ai_adj(p, pp, r, qq, r, sw);
         }
         uint64_t t = D[sp * W + ww] & ~hf[sp * W + ww];
+#pragma unroll 1
         while (t) {
           const int r = ww * 64 + __ffsll((long long)t) - 1;
           t &= t - 1;
@@ -403,11 +408,13 @@ __device__ void diag_terms_adj(const Params& p, const uint64_t* u, const uint64_
 #pragma unroll
     for (int w = 0; w < W; ++w) {
       uint64_t h = hf[sp * W + w] & ~u[sp * W + w];
+#pragma unroll 1
       while (h && nh < 24) {
         hs[nh++] = w * 64 + __ffsll((long long)h) - 1 + sp * p.norb;
         h &= h - 1;
       }
       uint64_t t = u[sp * W + w] & ~hf[sp * W + w];
+#pragma unroll 1
       while (t && np < 24) {
         ps[np++] = w * 64 + __ffsll((long long)t) - 1 + sp * p.norb;
         t &= t - 1;
@@ -419,23 +426,35 @@ __device__ void diag_terms_adj(const Params& p, const uint64_t* u, const uint64_
   double* sJ = sl + nt;
   double* sK = sl + 2 * nt;
   double* sf = sl + 3 * nt;
+#pragma unroll 1
   for (int i = 0; i < np; ++i) atomicAdd(&sf[ps[i]], gm);
+#pragma unroll 1
   for (int i = 0; i < nh; ++i) atomicAdd(&sf[hs[i]], -gm);
   if (gh == 0.0) return;
+#pragma unroll 1
   for (int i = 0; i < np; ++i) atomicAdd(&sF[tri(ps[i] % n, ps[i] % n)], gh);
+#pragma unroll 1
   for (int i = 0; i < nh; ++i) atomicAdd(&sF[tri(hs[i] % n, hs[i] % n)], -gh);
   auto jk = [&](int a, int b, double c) {
     const int t = tri(a % n, b % n);
     atomicAdd(&sJ[t], c);
     if ((a / n) == (b / n)) atomicAdd(&sK[t], -c);
   };
+#pragma unroll 1
   for (int i = 0; i < nh; ++i) jk(hs[i], hs[i], 0.5 * gh);
+#pragma unroll 1
   for (int i = 0; i < np; ++i) jk(ps[i], ps[i], 0.5 * gh);
+#pragma unroll 1
   for (int i = 0; i < nh; ++i)
+#pragma unroll 1
     for (int j = i + 1; j < nh; ++j) jk(hs[i], hs[j], gh);
+#pragma unroll 1
   for (int i = 0; i < np; ++i)
+#pragma unroll 1
     for (int j = i + 1; j < np; ++j) jk(ps[i], ps[j], gh);
+#pragma unroll 1
   for (int i = 0; i < nh; ++i)
+#pragma unroll 1
     for (int j = 0; j < np; ++j) jk(hs[i], ps[j], -gh);
 }
 
@@ -451,11 +470,13 @@ __device__ void diag_terms(const Params& p, const uint64_t* u, const uint64_t* h
 #pragma unroll
     for (int w = 0; w < W; ++w) {
       uint64_t h = hf[sp * W + w] & ~u[sp * W + w];
+#pragma unroll 1
       while (h && nh < 24) {
         hs[nh++] = w * 64 + __ffsll((long long)h) - 1 + sp * p.norb;
         h &= h - 1;
       }
       uint64_t t = u[sp * W + w] & ~hf[sp * W + w];
+#pragma unroll 1
       while (t && np < 24) {
         ps[np++] = w * 64 + __ffsll((long long)t) - 1 + sp * p.norb;
         t &= t - 1;
@@ -463,7 +484,9 @@ __device__ void diag_terms(const Params& p, const uint64_t* u, const uint64_t* h
     }
   }
   double mp = 0.0;
+#pragma unroll 1
   for (int i = 0; i < np; ++i) mp += __ldg(&p.fmpb[ps[i]]);
+#pragma unroll 1
   for (int i = 0; i < nh; ++i) mp -= __ldg(&p.fmpb[hs[i]]);
   hmpi = mp;
   if (!want_hdig) {
@@ -472,10 +495,12 @@ __device__ void diag_terms(const Params& p, const uint64_t* u, const uint64_t* h
   }
   const int n = p.norb;
   double e = 0.0;
+#pragma unroll 1
   for (int i = 0; i < np; ++i) {
     const int o = ps[i] % n;
     e += __ldg(&p.F[tri(o, o)]);
   }
+#pragma unroll 1
   for (int i = 0; i < nh; ++i) {
     const int o = hs[i] % n;
     e -= __ldg(&p.F[tri(o, o)]);
@@ -488,13 +513,21 @@ __device__ void diag_terms(const Params& p, const uint64_t* u, const uint64_t* h
     return x;
   };
   // same-position terms of the reference's pair sum, 0.5*(J_tt-K_tt+J_pp-K_pp)
+#pragma unroll 1
   for (int i = 0; i < nh; ++i) e += 0.5 * jk(hs[i], hs[i]);
+#pragma unroll 1
   for (int i = 0; i < np; ++i) e += 0.5 * jk(ps[i], ps[i]);
+#pragma unroll 1
   for (int i = 0; i < nh; ++i)
+#pragma unroll 1
     for (int j = i + 1; j < nh; ++j) e += jk(hs[i], hs[j]);
+#pragma unroll 1
   for (int i = 0; i < np; ++i)
+#pragma unroll 1
     for (int j = i + 1; j < np; ++j) e += jk(ps[i], ps[j]);
+#pragma unroll 1
   for (int i = 0; i < nh; ++i)
+#pragma unroll 1
     for (int j = 0; j < np; ++j) e -= jk(hs[i], ps[j]);
   hdigi = e;
 }
@@ -542,6 +575,7 @@ __device__ int2 ordered_partition2(int n, Part part, Emit emit, int* warp_tmp /*
   const int chunk = (((n + nw - 1) / nw) + 31) & ~31;
   const int lo = min(n, wid * chunk), hi = min(n, lo + chunk);
   int c0 = 0, c1 = 0;
+#pragma unroll 1
   for (int base = lo; base < hi; base += 32) {
     const int i = base + lane;
     const int pt = i < hi ? part(i) : -1;
@@ -554,6 +588,7 @@ __device__ int2 ordered_partition2(int n, Part part, Emit emit, int* warp_tmp /*
   }
   __syncthreads();
   int o0 = 0, o1 = 0, n0 = 0, n1 = 0;
+#pragma unroll 1
   for (int w = 0; w < nw; ++w) {
     const int a = warp_tmp[w], b = warp_tmp[nw + w];
     if (w < wid) {
@@ -564,6 +599,7 @@ __device__ int2 ordered_partition2(int n, Part part, Emit emit, int* warp_tmp /*
     n1 += b;
   }
   const unsigned below = (1u << lane) - 1u;
+#pragma unroll 1
   for (int base = lo; base < hi; base += 32) {
     const int i = base + lane;
     const int pt = i < hi ? part(i) : -1;
@@ -578,39 +614,6 @@ __device__ int2 ordered_partition2(int n, Part part, Emit emit, int* warp_tmp /*
   return make_int2(n0, n1);
 }
 
-// Counters of the candidate scan.  Kept apart from Acc: Acc is passed by
-// reference to the out-of-line queue drain, so it lives in local memory,
-// and these are incremented in the scan loop itself (registers).
-struct ScanCounts {
-  unsigned long long ncand, ncmp, np1, np2;
-  __device__ void zero() { ncand = ncmp = np1 = np2 = 0ull; }
-};
-
-// One thread's histogram (cip/isto.f): class sums and counts, indexed by
-// class at run time, so it lives in local memory (L1-resident); one FP64 add
-// per contribution, no atomics; merged into the block's at kernel end.
-template <int R>
-struct HistPriv {
-  double tab[kNClass][2][R];
-  unsigned int nom[kNClass];  // per-thread counts stay far below 2^32
-  unsigned int nam[kNClass][R];
-  __device__ void zero() {
-    for (int c = 0; c < kNClass; ++c) {
-      nom[c] = 0ull;
-      for (int m = 0; m < R; ++m) {
-        tab[c][0][m] = tab[c][1][m] = 0.0;
-        nam[c][m] = 0ull;
-      }
-    }
-  }
-};
-
-struct SmemHist {
-  unsigned long long nom[kNClass];
-  unsigned long long nam[kNClass * kMaxRoots];
-  double tab[2 * kNClass * kMaxRoots];
-};
-
 // histogram class of a non-negative value (cip/isto.f: first i with
 // val < aval(i)); compared as IEEE bit patterns, which order non-negative
 // doubles exactly as the values (integer pipe instead of FP64 compares)
@@ -618,189 +621,9 @@ __device__ __forceinline__ int hist_class(const Params& p, double val) {
   const long long v = __double_as_longlong(val);
   const int nc = p.nclass - 1;
   int c = 0;
+#pragma unroll 1
   for (int i = 0; i < nc; ++i) c += (v >= p.aval_bits[i]) ? 1 : 0;
   return c;
-}
-
-// Everything the reference does with one candidate after its interaction
-// scan: denominators, E2, selection, histogram, unit-60 record.  Called by
-// all 32 lanes of a warp; `live` marks the lanes holding a perturber.
-template <int W, int R>
-__device__ void finish_candidate(const Params& p, bool live, const uint64_t* u, double hmpi,
-                                 double hvpi, const double* bc, int slot /*in the work unit*/,
-                                 double fmul, int nmul, bool ybis, bool is_pert1, Acc<R>& acc,
-                                 HistPriv<R>& hp) {
-  constexpr unsigned kFull = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  double xam = 0.0;
-  bool ydeg = false;
-  // weighted E2 terms per root: term * (1 + fmul), which is also what the
-  // histogram (isto.f, fm = fmul + 1) and cipsym's unit-60 value
-  // (cipsym/pert1.f:244, eivp * (fmul + 1)) use
-  double vil[R], semp[R], sevp[R];
-  // the reference adds each term and then term*fmul (spin-flip weight,
-  // pert1.f:280-287); one compensated add of term*(1+fmul) is used here.
-  // fmul = 0 whenever ybis is false, so wgt = fmul + 1 for every perturber.
-  const double wgt = ybis ? 1.0 + fmul : 1.0;
-#pragma unroll
-  for (int m = 0; m < R; ++m) {
-    vil[m] = 0.0;
-    semp[m] = sevp[m] = 0.0;
-    if (!live || m >= p.metat) continue;
-    const double bcalc = bc[m];
-    const double dmp = p.emp[m] - hmpi;
-    double eivp = 0.0, tvp = 0.0, cimp, xim, deno, eim;
-    if (p.yen) {
-      // the three denominators share one FP64 division (GB300's FP64 rate is
-      // 1/64 of FP32): br = b/(dmp*dvp*db), b/dmp = dvp*db*br, etc.
-      const double dvp = p.e[m] - hvpi;
-      const double db = p.eb[m] - hvpi;
-      const double pvb = dvp * db;
-      const double prod = dmp * pvb;
-      double civp, cib;
-      // 1e-280 < |prod| < 1e280 tested on the exponent field (integer pipe):
-      // binary exponent in [-930, 929]
-      const unsigned pex = (unsigned)(__double_as_longlong(prod) >> 52) & 0x7FFu;
-      if (pex - 93u < 1860u) {
-        const double br = bcalc / prod;
-        cimp = br * pvb;
-        civp = br * (dmp * db);
-        cib = br * (dmp * dvp);
-      } else {  // a denominator at (or near) zero or huge: divide one by one
-        cimp = bcalc / dmp;
-        civp = bcalc / dvp;
-        cib = bcalc / db;
-      }
-      eivp = bcalc * civp;
-      tvp = eivp * wgt;
-      kahan_add(acc.e2vp[m], acc.cvp[m], tvp);
-      acc.psivp[m] = fma(civp * civp, wgt, acc.psivp[m]);
-      kahan_add(acc.e2b[m], acc.cb[m], (bcalc * cib) * wgt);
-      xim = p.ysele ? fabs(eivp) : fabs(civp);
-      deno = dvp;
-      eim = eivp;
-    } else {
-      cimp = bcalc / dmp;
-    }
-    const double eimp = bcalc * cimp;
-    const double tmp = eimp * wgt;
-    kahan_add(acc.e2mp[m], acc.cmp[m], tmp);
-    acc.psimp[m] = fma(cimp * cimp, wgt, acc.psimp[m]);
-    if (!p.yen) {
-      xim = p.ysele ? fabs(eimp) : fabs(cimp);
-      deno = dmp;
-      eim = eimp;
-    }
-    // comparisons of magnitudes on their IEEE bit patterns (exact for
-    // non-negative doubles; NaN compares as in the reference: never below)
-    const long long bdeno = __double_as_longlong(deno) & 0x7fffffffffffffffll;
-    const long long beim = __double_as_longlong(eim) & 0x7fffffffffffffffll;
-    if (!(bdeno > kBits005 && bdeno <= kBitsInf) && !(beim < kBits1em6) && p.ywdeg) ydeg = true;
-    if (lt_nonneg(xim, p.teste[m])) acc.dpivot = max_nonneg(acc.dpivot, xim);
-    if (p.ymoyen) {
-      xim = xim * p.taum[m];
-      vil[m] = xim;
-      xam = max_nonneg(xam, xim);
-    }
-    semp[m] = tmp;
-    sevp[m] = tvp;
-  }
-  if (live) {
-    acc.ietat += (unsigned long long)(long long)(nmul + 1);
-    acc.nproc += 1;
-  }
-  // histogram (cip/isto.f; pert1 calls it always, diexcit only if ymoyen)
-  if (live && (is_pert1 || p.ymoyen) && xam >= p.teseff) {
-    const int cls = hist_class(p, xam);
-    hp.nom[cls] += (unsigned)(1 + nmul);
-#pragma unroll
-    for (int m = 0; m < R; ++m) {
-      if (m >= p.metat || vil[m] < p.teseff) continue;
-      hp.tab[cls][0][m] += semp[m];  // eimp * (fmul + 1)
-      hp.tab[cls][1][m] += sevp[m];  // eivp * (fmul + 1)
-      hp.nam[hist_class(p, vil[m])][m] += (unsigned)(1 + nmul);
-    }
-  }
-  if (ydeg) xam = 1.0;
-  // unit-60 record (pie.f): counted per warp; kept, when asked, at the
-  // candidate's slot of this CTA's staging region (compacted in slot order
-  // when the work unit is done, unit_compact)
-  const bool sel = live && xam > p.tau && p.ymoyen;
-  const unsigned sm = __ballot_sync(kFull, sel);
-  if (sm && lane == 0) atomicAdd(&p.counters[C_NSEL], (unsigned long long)__popc(sm));
-  if (sel && p.rec_mode && slot >= p.st_cap) atomicAdd(&p.counters[C_STAGE_OVF], 1ull);  // host sizing error
-  if (sel && p.rec_mode && slot < p.st_cap) {
-    const size_t s = (size_t)blockIdx.x * p.st_cap + slot;
-#pragma unroll
-    for (int q = 0; q < 2 * W; ++q) p.st_bits[s * 2 * W + q] = u[q];
-    p.st_xam[s] = xam;
-    // ENvp per root written by cipsym (cipsym/pert1.f:244): eivp*(fmul+1)
-#pragma unroll
-    for (int m = 0; m < R; ++m)
-      if (m < p.metat) p.st_evp[s * p.metat + m] = p.symvar ? sevp[m] : 0.0;
-    atomicOr(&p.st_mask[(size_t)blockIdx.x * (p.st_cap >> 5) + (slot >> 5)], 1u << (slot & 31));
-  }
-}
-
-// End of a work unit (whole block): the staged records of its flagged
-// slots go, in slot order, to one segment of the record pool, reserved with
-// a single atomic; the unit table notes the segment.  The slot mask is
-// cleared for the next unit.  Records beyond the pool's capacity are
-// counted but not stored (the host sees pool_count > pool_cap).
-template <int W>
-__device__ __noinline__ void unit_compact(const Params& p, int unit, int nslots, int* tmp /* >= 32 ints */,
-                             long long& sbase /* shared */) {
-  constexpr unsigned kFull = 0xffffffffu;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
-  __syncthreads();  // every warp's staging stores and mask bits are done
-  const int nwords = (min(nslots, p.st_cap) + 31) >> 5;
-  uint32_t* mask = p.st_mask + (size_t)blockIdx.x * (p.st_cap >> 5);
-  const size_t st0 = (size_t)blockIdx.x * p.st_cap;
-  // each thread owns a contiguous range of mask words
-  const int per = (nwords + (int)blockDim.x - 1) / (int)blockDim.x;
-  const int w0 = min(nwords, tid * per), w1 = min(nwords, w0 + per);
-  int cnt = 0;
-  for (int w = w0; w < w1; ++w) cnt += __popc(__ldcg(&mask[w]));
-  // block exclusive scan of cnt (thread order = slot order)
-  int incl = cnt;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(kFull, incl, o);
-    if (lane >= o) incl += y;
-  }
-  if (lane == 31) tmp[wid] = incl;
-  __syncthreads();
-  if (tid == 0) {
-    int acc = 0;
-    for (int w = 0; w < nw; ++w) {
-      const int v = tmp[w];
-      tmp[w] = acc;
-      acc += v;
-    }
-    long long base = 0;
-    if (acc) base = (long long)atomicAdd(p.pool_count, (unsigned long long)acc);
-    p.unit_pool[unit] = base;
-    p.unit_nsel[unit] = acc;
-    sbase = base;
-  }
-  __syncthreads();
-  long long pos = sbase + tmp[wid] + (incl - cnt);
-  for (int w = w0; w < w1; ++w) {
-    uint32_t m = __ldcg(&mask[w]);
-    if (m) mask[w] = 0u;
-    while (m) {
-      const int b = __ffs(m) - 1;
-      m &= m - 1u;
-      if (pos < p.pool_cap) {
-        const size_t s = st0 + (size_t)(w * 32 + b);
-#pragma unroll
-        for (int q = 0; q < 2 * W; ++q) p.pool_bits[(size_t)pos * 2 * W + q] = __ldcg(&p.st_bits[s * 2 * W + q]);
-        p.pool_xam[pos] = __ldcg(&p.st_xam[s]);
-        for (int mm = 0; mm < p.metat; ++mm) p.pool_evp[(size_t)pos * p.metat + mm] = __ldcg(&p.st_evp[s * p.metat + mm]);
-      }
-      ++pos;
-    }
-  }
-  __syncthreads();
 }
 
 template <int R>
@@ -809,6 +632,7 @@ __device__ void block_flush(const Params& p, Acc<R>& acc, int gslot, double* red
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int nw = blockDim.x >> 5;
   const int nq = 5 * p.metat;
+#pragma unroll 1
   for (int q = 0; q < nq; ++q) {
     const int m = q % p.metat, which = q / p.metat;
     double v = 0.0;
@@ -821,12 +645,14 @@ __device__ void block_flush(const Params& p, Acc<R>& acc, int gslot, double* red
             : which == 3 ? acc.psimp[mm]
                          : acc.psivp[mm];
       }
+#pragma unroll 1
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if (lane == 0) red[q * 32 + wid] = v;
   }
   __syncthreads();
   if (threadIdx.x < nq) {
     double s = 0.0, c = 0.0;
+#pragma unroll 1
     for (int w = 0; w < nw; ++w) kahan_add(s, c, red[threadIdx.x * 32 + w]);
     p.gen_part[(long long)gslot * nq + threadIdx.x] = s - c;
   }
@@ -838,118 +664,6 @@ __device__ void block_flush(const Params& p, Acc<R>& acc, int gslot, double* red
   }
 }
 
-
-// Enqueue the live lanes' perturbers (called by a whole warp); runs the
-// epilogue on every full batch of 32.
-template <int W, int R>
-__device__ void enqueue_candidate(const Params& p, WarpQueue<W, R>& q, int& qn, bool live,
-                                  const uint64_t* u, double hmpi, double hvpi, const double* bc,
-                                  int slot, double fmul, int nmul, bool ybis, bool is_pert1,
-                                  Acc<R>& acc, HistPriv<R>& hp);
-
-template <int W, int R>
-__device__ __noinline__ void drain_queue(const Params& p, WarpQueue<W, R>& q, int& qn, bool all, Acc<R>& acc,
-                            HistPriv<R>& hp) {
-  const int lane = threadIdx.x & 31;
-  while (qn >= 32 || (all && qn > 0)) {
-    const int base = qn >= 32 ? qn - 32 : 0;
-    const int cnt = qn >= 32 ? 32 : qn;
-    const bool live = lane < cnt;
-    const int e = base + (live ? lane : 0);
-    uint64_t u[2 * W];
-#pragma unroll
-    for (int w = 0; w < 2 * W; ++w) u[w] = q.u[w][e];
-    double bc[R];
-#pragma unroll
-    for (int m = 0; m < R; ++m) bc[m] = q.bc[m][e];
-    const unsigned char f = q.flags[e];
-    finish_candidate<W, R>(p, live, u, q.hmp[e], q.hvp[e], bc, q.slot[e], q.fmul[e], q.nmul[e],
-                           (f & 1) != 0, (f & 2) != 0, acc, hp);
-    __syncwarp();
-    qn = base;
-  }
-}
-
-template <int W, int R>
-__device__ void enqueue_candidate(const Params& p, WarpQueue<W, R>& q, int& qn, bool live,
-                                  const uint64_t* u, double hmpi, double hvpi, const double* bc,
-                                  int slot, double fmul, int nmul, bool ybis, bool is_pert1,
-                                  Acc<R>& acc, HistPriv<R>& hp) {
-  const int lane = threadIdx.x & 31;
-  const unsigned lm = __ballot_sync(0xffffffffu, live);
-  if (live) {
-    const int e = qn + __popc(lm & ((1u << lane) - 1u));
-#pragma unroll
-    for (int w = 0; w < 2 * W; ++w) q.u[w][e] = u[w];
-#pragma unroll
-    for (int m = 0; m < R; ++m) q.bc[m][e] = bc[m];
-    q.hmp[e] = hmpi;
-    q.hvp[e] = hvpi;
-    q.fmul[e] = fmul;
-    q.nmul[e] = nmul;
-    q.slot[e] = slot;
-    q.flags[e] = (unsigned char)((ybis ? 1 : 0) | (is_pert1 ? 2 : 0));
-  }
-  qn += __popc(lm);
-  __syncwarp();
-  // the drain is out of line; calling it only with a full batch spares the
-  // register saves of a call on every other candidate round
-  if (qn >= 32) drain_queue<W, R>(p, q, qn, false, acc, hp);
-}
-
-// Block totals of the integer counters and the histogram into the
-// geometry's global counters; then reset them for the next geometry.
-template <int R>
-__device__ void flush_totals(const Params& p, Acc<R>& acc, HistPriv<R>& hp, SmemHist& hist,
-                             unsigned long long ncand, unsigned long long ncmp, unsigned long long np1,
-                             unsigned long long np2) {
-  const int tid = threadIdx.x;
-  // block totals of the integer counters and the histogram
-  __syncthreads();
-  {
-    unsigned long long v[8] = {acc.ietat, acc.nproc, 0ull, ncand, ncmp, np1, np2, 0ull};
-    for (int q = 0; q < 8; ++q) {
-      unsigned long long x = v[q];
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if ((tid & 31) == 0 && x) atomicAdd(&p.counters[q], x);
-    }
-    unsigned long long db = __double_as_longlong(acc.dpivot);
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long y = __shfl_down_sync(0xffffffffu, db, o);
-      db = y > db ? y : db;
-    }
-    if ((tid & 31) == 0) atomicMax(p.dpivot_bits, db);
-  }
-  // this thread's histogram into the block's
-  for (int c = 0; c < p.nclass; ++c) {
-    if (hp.nom[c]) atomicAdd(&hist.nom[c], (unsigned long long)hp.nom[c]);
-    for (int m = 0; m < R && m < p.metat; ++m) {
-      if (hp.tab[c][0][m] != 0.0) atomicAdd(&hist.tab[c * kMaxRoots + m], hp.tab[c][0][m]);
-      if (hp.tab[c][1][m] != 0.0)
-        atomicAdd(&hist.tab[kNClass * kMaxRoots + c * kMaxRoots + m], hp.tab[c][1][m]);
-      if (hp.nam[c][m]) atomicAdd(&hist.nam[c * kMaxRoots + m], (unsigned long long)hp.nam[c][m]);
-    }
-  }
-  __syncthreads();
-  for (int i = tid; i < p.nclass; i += blockDim.x)
-    if (hist.nom[i]) atomicAdd(&p.hist_nom[i], hist.nom[i]);
-  for (int i = tid; i < p.nclass * kMaxRoots; i += blockDim.x) {
-    const int c = i / kMaxRoots, m = i % kMaxRoots;
-    if (m >= p.metat) continue;
-    if (hist.nam[i]) atomicAdd(&p.hist_nam[c * p.metat + m], hist.nam[i]);
-    if (hist.tab[i] != 0.0) atomicAdd(&p.hist_tab[c * p.metat + m], hist.tab[i]);
-    const double tv = hist.tab[kNClass * kMaxRoots + i];
-    if (tv != 0.0) atomicAdd(&p.hist_tab[p.nclass * p.metat + c * p.metat + m], tv);
-  }
-  __syncthreads();
-  acc.ietat = acc.nproc = 0ull;
-  acc.dpivot = 0.0;
-  hp.zero();
-  for (int i = tid; i < kNClass; i += blockDim.x) hist.nom[i] = 0;
-  for (int i = tid; i < kNClass * kMaxRoots; i += blockDim.x) hist.nam[i] = 0;
-  for (int i = tid; i < 2 * kNClass * kMaxRoots; i += blockDim.x) hist.tab[i] = 0.0;
-  __syncthreads();
-}
 
 // ------------------------------------------------------------------ kernel
 struct BlockShared {
@@ -968,11 +682,12 @@ struct BlockShared {
   int gen;
   int kidx;
   int rank_k;
-  long long unit_base;    // pool segment of the unit being compacted
 };
 
-template <int W, int R, bool B, bool ADJ>
-__global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
+// The adjoint kernel: E2 sums and the gradients of the integrals and root
+// energies.
+template <int W, int R>
+__global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
   extern __shared__ __align__(16) unsigned char dyn[];
   // the current geometry's parameters, in shared memory (device functions
   // then read them through a shared-memory reference instead of a local
@@ -980,7 +695,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
   __shared__ Params sgeo;
   const Params& p = sgeo;
   __shared__ BlockShared sh;
-  __shared__ SmemHist hist;
   __shared__ double red[5 * kMaxRoots * 32];
   __shared__ int ctmp[33];
   __shared__ int16_t wrow[(kThreads / 32) * kRowCap];
@@ -992,85 +706,48 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
   // L_R entries (compact form, lr_entry) up to lr_cap in shared memory; the
   // rest of a longer list stays in the block's global scratch
   uint64_t* lr_ent = reinterpret_cast<uint64_t*>(dyn);
-  // per-warp epilogue queues, 16-byte aligned after the L_R entries
-  const size_t qoff = (((size_t)p0.lr_cap * 8) + 15) & ~(size_t)15;
-  WarpQueue<W, R>& wq = reinterpret_cast<WarpQueue<W, R>*>(dyn + qoff)[threadIdx.x >> 5];
-  int qn = 0;
-
-  for (int i = tid; i < kNClass; i += blockDim.x) hist.nom[i] = 0;
-  for (int i = tid; i < kNClass * kMaxRoots; i += blockDim.x) hist.nam[i] = 0;
-  for (int i = tid; i < 2 * kNClass * kMaxRoots; i += blockDim.x) hist.tab[i] = 0.0;
-
   // per-geometry state
   int32_t* my_nb_j = nullptr;
   uint64_t* my_nb_em = nullptr;
   uint64_t* my_lr_ent = nullptr;
   uint64_t hf[2 * W];
   int ncf = 0;
-  auto geo_init = [&]() {
-    my_nb_j = p.nb_j + (size_t)blockIdx.x * p.nb_stride;
-    my_nb_em = p.nb_emask + (size_t)blockIdx.x * p.nb_stride;
-    my_lr_ent = p.lr_ent + (size_t)blockIdx.x * p.nb_stride;
+  if (tid == 0) sgeo = p0;
+  __syncthreads();
+  my_nb_j = p.nb_j + (size_t)blockIdx.x * p.nb_stride;
+  my_nb_em = p.nb_emask + (size_t)blockIdx.x * p.nb_stride;
+  my_lr_ent = p.lr_ent + (size_t)blockIdx.x * p.nb_stride;
 #pragma unroll
-    for (int s = 0; s < 2; ++s)
+  for (int s = 0; s < 2; ++s)
 #pragma unroll
-      for (int w = 0; w < W; ++w) {
-        const int lo = w * 64;
-        const int n = min(max(p.noca - lo, 0), 64);
-        hf[s * W + w] = (n >= 64) ? ~0ull : ((1ull << n) - 1ull);
-      }
-    ncf = p.ncf;
-  };
-  if (!B) {
-    if (tid == 0) sgeo = p0;
-    __syncthreads();
-    geo_init();
-  }
-  int cur_geo = -1;
+    for (int w = 0; w < W; ++w) {
+      const int lo = w * 64;
+      const int n = min(max(p.noca - lo, 0), 64);
+      hf[s * W + w] = (n >= 64) ? ~0ull : ((1ull << n) - 1ull);
+    }
+  ncf = p.ncf;
 
   Acc<R> acc;
   acc.zero();
-  ScanCounts sc;
-  sc.zero();
-  HistPriv<R> hp;
-  hp.zero();
   // adjoint: per-thread root-energy gradients and per-block accumulators of
   // dE/dhdig and dE/dhmp over one block of removed electrons (K' terms:
   // adj_sh[0..1]; per added spin orbital: adj_gv, adj_gf)
-  __shared__ double adj_gv[ADJ ? 2 * kMaxOrb : 1], adj_gf[ADJ ? 2 * kMaxOrb : 1], adj_sh[2];
+  __shared__ double adj_gv[2 * kMaxOrb], adj_gf[2 * kMaxOrb], adj_sh[2];
   double adjr[3][R];
   double adj_gK = 0.0, adj_gM = 0.0;
   double* adj_sl = nullptr;
-  if (ADJ) {
 #pragma unroll
-    for (int m = 0; m < R; ++m) adjr[0][m] = adjr[1][m] = adjr[2][m] = 0.0;
-    for (int i = tid; i < 2 * kMaxOrb; i += blockDim.x) adj_gv[i] = adj_gf[i] = 0.0;
-    adj_sl = p0.g_slice + (size_t)blockIdx.x * p0.slice_stride;
-  }
+  for (int m = 0; m < R; ++m) adjr[0][m] = adjr[1][m] = adjr[2][m] = 0.0;
+#pragma unroll 1
+  for (int i = tid; i < 2 * kMaxOrb; i += blockDim.x) adj_gv[i] = adj_gf[i] = 0.0;
+  adj_sl = p0.g_slice + (size_t)blockIdx.x * p0.slice_stride;
 
   for (;;) {
     __syncthreads();
-    if (tid == 0) sh.gen = atomicAdd(B ? ba.work : p0.work, 1);
+    if (tid == 0) sh.gen = atomicAdd(p0.work, 1);
     __syncthreads();
-    int unit = sh.gen;
-    if (unit >= (B ? ba.nunits : p0.nunits)) break;
-    if (B) {
-      const int gi = ba.unit_geo[unit];
-      if (gi != cur_geo) {
-        if (cur_geo >= 0) {
-          flush_totals<R>(p, acc, hp, hist, sc.ncand, sc.ncmp, sc.np1, sc.np2);
-          sc.zero();
-        }
-        __syncthreads();
-        const int* src = reinterpret_cast<const int*>(ba.geo + gi);
-        int* dst = reinterpret_cast<int*>(&sgeo);
-        for (int i = tid; i < (int)(sizeof(Params) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
-        __syncthreads();
-        cur_geo = gi;
-        geo_init();
-      }
-      unit = ba.unit_local[unit];
-    }
+    const int unit = sh.gen;
+    if (unit >= p0.nunits) break;
     const int g = p.unit_g[unit];
     const int ur0 = p.unit_r0[unit], ur1 = p.unit_r1[unit];
     const int k = p.gens[g];
@@ -1079,6 +756,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
       // ---------------- pertu: reference and its singles, no owner test
       // candidates: t = 0 -> reference (if pertu_ref), then singles
       const int no = p.noca, nv = p.norb - p.noca;
+#pragma unroll 1
       for (int t0 = ur0; t0 < ur1; t0 += blockDim.x) {
         const int t = t0 + tid;
         bool live = t < ur1;
@@ -1099,18 +777,17 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
         for (int m = 0; m < R; ++m) bc[m] = 0.0;
         double hmpi = 0.0, hvpi = 0.0;
         if (live) {
-          sc.ncand++;
           int rankI = 0;
 #pragma unroll
           for (int q = 0; q < 2 * W; ++q) rankI += __popcll(hf[q] & ~u[q]);
           int nint = 0;
           bool drop = false;
+#pragma unroll 1
           for (int j = 0; j < ncf; ++j) {
             const uint64_t* v = p.S + (size_t)j * 2 * W;
             int x = 0;
 #pragma unroll
             for (int q = 0; q < 2 * W; ++q) x += __popcll(u[q] ^ __ldg(&v[q]));
-            sc.ncmp++;
             if (x > 4) continue;
             if (x == 0) {
               drop = true;
@@ -1124,7 +801,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
             for (int q = 0; q < 2 * W; ++q) rankJ += __popcll(hf[q] & ~vv[q]);
             int kind;
             const double h = hmat<W>(p, u, vv, rankI, rankJ, hf, kind);
-            if (kind == 1) sc.np1++; else sc.np2++;
             ++nint;
 #pragma unroll
             for (int m = 0; m < R; ++m)
@@ -1133,42 +809,37 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
           if (drop || nint == 0) live = false;
           if (live) diag_terms<W>(p, u, hf, hmpi, hvpi, p.yen != 0);
         }
-        if (ADJ) {
-          if (live) {
-            double gb[R], gh, gm;
-            adj_factors<R>(p, bc, hmpi, hvpi, 1.0, gb, gh, gm, adjr, acc);
-            acc.ietat += 1;
-            acc.nproc += 1;
-            int rankI = 0;
+        if (live) {
+          double gb[R], gh, gm;
+          adj_factors<R>(p, bc, hmpi, hvpi, 1.0, gb, gh, gm, adjr, acc);
+          acc.ietat += 1;
+          acc.nproc += 1;
+          int rankI = 0;
 #pragma unroll
-            for (int q = 0; q < 2 * W; ++q) rankI += __popcll(hf[q] & ~u[q]);
-            for (int j = 0; j < ncf; ++j) {
-              const uint64_t* v = p.S + (size_t)j * 2 * W;
-              uint64_t vv[2 * W];
-              int x = 0;
+          for (int q = 0; q < 2 * W; ++q) rankI += __popcll(hf[q] & ~u[q]);
+#pragma unroll 1
+          for (int j = 0; j < ncf; ++j) {
+            const uint64_t* v = p.S + (size_t)j * 2 * W;
+            uint64_t vv[2 * W];
+            int x = 0;
 #pragma unroll
-              for (int q = 0; q < 2 * W; ++q) {
-                vv[q] = __ldg(&v[q]);
-                x += __popcll(u[q] ^ vv[q]);
-              }
-              if (x > 4 || x == 0 || (p.adj_1e && x == 4)) continue;
-              int rankJ = 0;
-#pragma unroll
-              for (int q = 0; q < 2 * W; ++q) rankJ += __popcll(hf[q] & ~vv[q]);
-              double w = 0.0;
-#pragma unroll
-              for (int m = 0; m < R; ++m)
-                if (m < p.metat) w += gb[m] * __ldg(&p.c[(size_t)j * p.metat + m]);
-              hmat_adj<W>(p, u, vv, rankI, rankJ, hf, w, !p.adj_1e);
+            for (int q = 0; q < 2 * W; ++q) {
+              vv[q] = __ldg(&v[q]);
+              x += __popcll(u[q] ^ vv[q]);
             }
-            diag_terms_adj<W>(p, u, hf, p.yen ? gh : 0.0, gm, adj_sl);
+            if (x > 4 || x == 0 || (p.adj_1e && x == 4)) continue;
+            int rankJ = 0;
+#pragma unroll
+            for (int q = 0; q < 2 * W; ++q) rankJ += __popcll(hf[q] & ~vv[q]);
+            double w = 0.0;
+#pragma unroll
+            for (int m = 0; m < R; ++m)
+              if (m < p.metat) w += gb[m] * __ldg(&p.c[(size_t)j * p.metat + m]);
+            hmat_adj<W>(p, u, vv, rankI, rankJ, hf, w, !p.adj_1e);
           }
-        } else {
-          enqueue_candidate<W, R>(p, wq, qn, live, u, hmpi, hvpi, bc, t - ur0, 0.0, 0, false, true, acc, hp);
+          diag_terms_adj<W>(p, u, hf, p.yen ? gh : 0.0, gm, adj_sl);
         }
       }
-      drain_queue<W, R>(p, wq, qn, true, acc, hp);
-      if (!ADJ && p.rec_mode) unit_compact<W>(p, unit, ur1 - ur0, ctmp, sh.unit_base);
       block_flush<R>(p, acc, unit, red);
       continue;
     }
@@ -1188,6 +859,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
       int ne = 0;
       for (int s = 0; s < 2; ++s) {
         int nes = 0, nv = 0;
+#pragma unroll 1
         for (int o = 0; o < p.norb; ++o) {
           if ((get_word<2 * W>(kb, s * W + (o >> 6)) >> (o & 63)) & 1ull) {
             sh.occ[ne++] = o + s * p.norb;
@@ -1219,6 +891,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
 #pragma unroll
           for (int q = 0; q < 2 * W; ++q) {
             uint64_t miss = kb[q] & ~__ldg(&p.S[(size_t)j * 2 * W + q]);
+#pragma unroll 1
             while (miss) {
               const int b = __ffsll((long long)miss) - 1;
               miss &= miss - 1;
@@ -1239,9 +912,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
     const uint8_t dmask = p.gen_dmask[g];
     const int nespk = p.nesp[k];
     const bool yefk = p.yef[k] != 0;
-    int slot0 = 0;  // first candidate slot of the current block in the unit
 
     // ---------------- blocks of removed electrons R (this unit's range)
+#pragma unroll 1
     for (int r = ur0; r < ur1; ++r) {
       int e1, e2 = -1;
       if (r < nel) {
@@ -1250,6 +923,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
         // pair index -> (e1 < e2)
         int t = r - nel;
         e1 = 0;
+#pragma unroll 1
         while (t >= nel - 1 - e1) {
           t -= nel - 1 - e1;
           ++e1;
@@ -1264,13 +938,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
       const int hfR = (o1 < p.noca ? 1 : 0) + (e2 >= 0 && o2 < p.noca ? 1 : 0);
       // achievable rank changes D = hfR + aV - |R| (aV = added HF-virtuals)
       bool any = false;
+#pragma unroll 1
       for (int aV = 0; aV <= nRr; ++aV) {
         const int D = hfR + aV - nRr;
         if (dmask & (1u << (D + 2))) any = true;
       }
       if (!any) continue;
-      const int bslot = slot0;
-      slot0 += (int)block_candidates(nRr, sp1 == sp2, sh.nvir[sp1], sh.nvir[0], sh.nvir[1]);
       const uint64_t rmask = (1ull << e1) | (e2 >= 0 ? (1ull << e2) : 0ull);
       // K' = k - R
       uint64_t kp[2 * W];
@@ -1295,6 +968,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
 #pragma unroll
         for (int q = 0; q < 2 * W; ++q) {
           uint64_t d = __ldg(&v[q]) & ~kp[q];
+#pragma unroll 1
           while (d) {
             const int b = __ffsll((long long)d) - 1;
             d &= d - 1;
@@ -1320,6 +994,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
         for (int sp = 0; sp < 2; ++sp)
           for (int w = 0; w < W; ++w) {
             uint64_t h = hf[sp * W + w] & ~kp[sp * W + w];
+#pragma unroll 1
             while (h) {
               const int b = __ffsll((long long)h) - 1;
               h &= h - 1;
@@ -1327,6 +1002,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
               sh.dn_sg[nd++] = -1;
             }
             uint64_t t2 = kp[sp * W + w] & ~hf[sp * W + w];
+#pragma unroll 1
             while (t2) {
               const int b = __ffsll((long long)t2) - 1;
               t2 &= t2 - 1;
@@ -1346,13 +1022,14 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
       const int n01 = nparts.x;
       const int nlr = nparts.x + nparts.y;
       const bool fast = nlr <= p.lr_cap;
-      if (!fast && tid == 0) atomicAdd(&p.counters[C_LRFALLBACK], 1ull);
       auto ent_at = [&](int i) -> uint64_t { return i < p.lr_cap ? lr_ent[i] : my_lr_ent[i]; };
       {
         const int ndn = sh.ndn, n = p.norb;
+#pragma unroll 1
         for (int a = tid; a < 2 * n; a += blockDim.x) {
           const int oa = a % n, sa = a / n;
           double g = 0.0;
+#pragma unroll 1
           for (int i = 0; i < ndn; ++i) {
             const int r = sh.dn_so[i];
             const int t = tri(oa, r % n);
@@ -1368,6 +1045,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
           // spread over its lanes, then summed by shuffles in a fixed order
           const int lane = tid & 31;
           double e = 0.0, mp = 0.0;
+#pragma unroll 1
           for (int t = lane; t < ndn * (ndn + 1); t += 32) {
             if (t < ndn) {
               const int r = sh.dn_so[t], orr = r % n;
@@ -1382,6 +1060,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
               e += 0.5 * sh.dn_sg[i] * sh.dn_sg[j] * x;
             }
           }
+#pragma unroll 1
           for (int o = 16; o > 0; o >>= 1) {
             e += __shfl_down_sync(0xffffffffu, e, o);
             mp += __shfl_down_sync(0xffffffffu, mp, o);
@@ -1409,7 +1088,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
       // listed entries rb[0..nrb) (owner test, already in S, <I|H|j>), then
       // the E2 / selection epilogue.  Called by whole warps.
       auto candidate = [&](bool live, int a1, int a2, int sa1, int sa2, int nscan, const int16_t* rb,
-                           int nrb, int slot) {
+                           int nrb) {
         int D = 0;
         bool ysyspi = true;
         if (live) {
@@ -1459,7 +1138,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
         const uint32_t c1x4 = live ? (uint32_t)(a1 + sa1 * p.norb) * 0x01010101u : 0u;
         const uint32_t c2x4 = live && two ? (uint32_t)(a2 + sa2 * p.norb) * 0x01010101u : 0u;
         if (live) {
-          sc.ncand++;
           or_word<2 * W>(u, sa1 * W + (a1 >> 6), 1ull << (a1 & 63));
           if (a2 >= 0) or_word<2 * W>(u, sa2 * W + (a2 >> 6), 1ull << (a2 & 63));
         }
@@ -1480,6 +1158,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
         // phase B: <I|H|j> of the listed hits, lanes in step
         auto flush = [&]() {
           const int maxh = __reduce_max_sync(0xffffffffu, drop ? 0 : nh);
+#pragma unroll 1
           for (int t = 0; t < maxh; ++t) {
             if (!drop && t < nh) {
               const int j = lr_entry_j(ent_at(hl[t]));
@@ -1491,8 +1170,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
               for (int q = 0; q < 2 * W; ++q) rankJ += __popcll(hf[q] & ~vv[q]);
               int kind;
               const double h = hmat<W>(p, u, vv, rankI, rankJ, hf, kind);
-              if (kind == 1) sc.np1++; else sc.np2++;
-              if (ADJ && kind == 1) {
+                if (kind == 1) {
                 s1j1 = s1n == 1 ? j : s1j1;
                 s1j0 = s1n == 0 ? j : s1j0;
                 ++s1n;
@@ -1507,6 +1185,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
           }
           nh = 0;
         };
+#pragma unroll 1
         for (int i0 = 0; i0 < nscan; i0 += 4) {
           if (__all_sync(0xffffffffu, drop)) break;
           if (__any_sync(0xffffffffu, !drop && nh > kHitCap - 4)) flush();
@@ -1521,6 +1200,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
             const int x2 = i0 + 2 < nscan ? lr_diff(ent_at(i0 + 2), c1x4, c2x4, two) : 99;
             const int x3 = i0 + 3 < nscan ? lr_diff(ent_at(i0 + 3), c1x4, c2x4, two) : 99;
             unsigned hits = (x0 <= 4 ? 1u : 0u) | (x1 <= 4 ? 2u : 0u) | (x2 <= 4 ? 4u : 0u) | (x3 <= 4 ? 8u : 0u);
+#pragma unroll 1
             while (hits && !drop) {
               const int g4 = __ffs(hits) - 1;
               hits &= hits - 1u;
@@ -1528,6 +1208,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
             }
           }
         }
+#pragma unroll 1
         for (int q2 = 0; q2 < nrb; ++q2) {
           if (__all_sync(0xffffffffu, drop)) break;
           if (__any_sync(0xffffffffu, !drop && nh >= kHitCap)) flush();
@@ -1539,7 +1220,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
         }
         flush();
         if (live) {
-          sc.ncmp += (unsigned long long)(nscan + nrb);
           if (drop || nint == 0) live = false;
           if (live && D == 2 && nnz == 0) live = false;  // diexcit drops zero couplings
         }
@@ -1574,92 +1254,89 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
             hvpi += sh.vdg[a2 + sa2 * p.norb] + gq;
           }
         }
-        if (ADJ) {
-          double gb[R], gh = 0.0, gm = 0.0;
+        double gb[R], gh = 0.0, gm = 0.0;
 #pragma unroll
-          for (int m = 0; m < R; ++m) gb[m] = 0.0;
-          if (live) {
-            adj_factors<R>(p, bc, hmpi, hvpi, ybis ? 1.0 + fmul : 1.0, gb, gh, gm, adjr, acc);
-            acc.ietat += (unsigned long long)(long long)(nmul + 1);
-            acc.nproc += 1;
-            if (!p.yen) gh = 0.0;
-          }
-          // second pass over the same entries: dE/dH_Ij = sum_m gb[m] c_jm,
-          // spread over the integrals of <I|H|j>.  Two phases as in the first
-          // pass: each lane lists the entries that interact with its I, then
-          // the warp takes the t-th listed entry of every lane at once, so
-          // hmat_adj runs with the warp in step instead of once per hitting
-          // lane.  The loops are warp-uniform (nscan, nrb); dead lanes list
-          // nothing.  One-electron adjoint: only the one-difference partners
-          // matter; those the first pass noted (up to two) are done here,
-          // and the scan runs only for lanes with more.
-          const bool with_eri = !p.adj_1e;
-          const bool rescan = live && (with_eri || s1n > 2);
-          const auto adj_one = [&](int j) {
-            uint64_t vv[2 * W];
-#pragma unroll
-            for (int q = 0; q < 2 * W; ++q) vv[q] = __ldg(&p.S[(size_t)j * 2 * W + q]);
-            int rankJ = 0;
-#pragma unroll
-            for (int q = 0; q < 2 * W; ++q) rankJ += __popcll(hf[q] & ~vv[q]);
-            double w = 0.0;
-#pragma unroll
-            for (int m = 0; m < R; ++m)
-              if (m < p.metat) w += gb[m] * __ldg(&p.c[(size_t)j * p.metat + m]);
-            hmat_adj<W>(p, u, vv, rank_k + D, rankJ, hf, w, with_eri);
-          };
-          if (!with_eri && live && s1n <= 2) {
-            if (s1n > 0) adj_one(s1j0);
-            if (s1n > 1) adj_one(s1j1);
-          }
-          const bool two = a2 >= 0;
-          const uint32_t c1x4 = rescan ? (uint32_t)(a1 + sa1 * p.norb) * 0x01010101u : 0u;
-          const uint32_t c2x4 = rescan && two ? (uint32_t)(a2 + sa2 * p.norb) * 0x01010101u : 0u;
-          const int xmax = with_eri ? 4 : 2;
-          int nh = 0;
-          int* hl = hitl + threadIdx.x * kHitCap;
-          auto note = [&](int i) {
-            const int x = lr_diff(ent_at(i), c1x4, c2x4, two);
-            if (x <= xmax && x != 0 && lr_entry_j(ent_at(i)) >= k) hl[nh++] = i;
-          };
-          auto flush_adj = [&]() {
-            const int maxh = __reduce_max_sync(0xffffffffu, nh);
-            for (int t = 0; t < maxh; ++t)
-              if (t < nh) adj_one(lr_entry_j(ent_at(hl[t])));
-            nh = 0;
-          };
-          if (__any_sync(0xffffffffu, rescan)) {
-            for (int i = 0; i < nscan; ++i) {
-              if (__any_sync(0xffffffffu, nh == kHitCap)) flush_adj();
-              if (rescan) note(i);
-            }
-            for (int q2 = 0; q2 < nrb; ++q2) {
-              if (__any_sync(0xffffffffu, nh == kHitCap)) flush_adj();
-              if (rescan) note(rb[q2]);
-            }
-            flush_adj();
-          }
-          if (!live) return;
-          // diagonal terms: hdig(I) = hdig(K') + vdg[a1] + vdg[a2] + G(a1,a2),
-          // hmp(I) = hmp(K') + fmpb[a1] + fmpb[a2]
-          adj_gK += gh;
-          adj_gM += gm;
-          atomicAdd(&adj_gv[a1 + sa1 * p.norb], gh);
-          atomicAdd(&adj_gf[a1 + sa1 * p.norb], gm);
-          if (a2 >= 0) {
-            atomicAdd(&adj_gv[a2 + sa2 * p.norb], gh);
-            atomicAdd(&adj_gf[a2 + sa2 * p.norb], gm);
-            const int nt = p.norb * (p.norb + 1) / 2;
-            const int tq = tri(a1, a2);
-            atomicAdd(&adj_sl[nt + tq], gh);
-            if (sa1 == sa2) atomicAdd(&adj_sl[2 * nt + tq], -gh);
-          }
-          return;
+        for (int m = 0; m < R; ++m) gb[m] = 0.0;
+        if (live) {
+          adj_factors<R>(p, bc, hmpi, hvpi, ybis ? 1.0 + fmul : 1.0, gb, gh, gm, adjr, acc);
+          acc.ietat += (unsigned long long)(long long)(nmul + 1);
+          acc.nproc += 1;
+          if (!p.yen) gh = 0.0;
         }
-        enqueue_candidate<W, R>(p, wq, qn, live, u, hmpi, hvpi, bc, slot, fmul, nmul, ybis, is_pert1, acc, hp);
+        // second pass over the same entries: dE/dH_Ij = sum_m gb[m] c_jm,
+        // spread over the integrals of <I|H|j>.  Two phases as in the first
+        // pass: each lane lists the entries that interact with its I, then
+        // the warp takes the t-th listed entry of every lane at once, so
+        // hmat_adj runs with the warp in step instead of once per hitting
+        // lane.  The loops are warp-uniform (nscan, nrb); dead lanes list
+        // nothing.  One-electron adjoint: only the one-difference partners
+        // matter; those the first pass noted (up to two) are done here,
+        // and the scan runs only for lanes with more.
+        const bool with_eri = !p.adj_1e;
+        const bool rescan = live && (with_eri || s1n > 2);
+        const auto adj_one = [&](int j) {
+          uint64_t vv[2 * W];
+#pragma unroll
+          for (int q = 0; q < 2 * W; ++q) vv[q] = __ldg(&p.S[(size_t)j * 2 * W + q]);
+          int rankJ = 0;
+#pragma unroll
+          for (int q = 0; q < 2 * W; ++q) rankJ += __popcll(hf[q] & ~vv[q]);
+          double w = 0.0;
+#pragma unroll
+          for (int m = 0; m < R; ++m)
+            if (m < p.metat) w += gb[m] * __ldg(&p.c[(size_t)j * p.metat + m]);
+          hmat_adj<W>(p, u, vv, rank_k + D, rankJ, hf, w, with_eri);
+        };
+        if (!with_eri && live && s1n <= 2) {
+          if (s1n > 0) adj_one(s1j0);
+          if (s1n > 1) adj_one(s1j1);
+        }
+        const uint32_t g1x4 = rescan ? (uint32_t)(a1 + sa1 * p.norb) * 0x01010101u : 0u;
+        const uint32_t g2x4 = rescan && two ? (uint32_t)(a2 + sa2 * p.norb) * 0x01010101u : 0u;
+        const int xmax = with_eri ? 4 : 2;
+        auto note = [&](int i) {
+          const int x = lr_diff(ent_at(i), g1x4, g2x4, two);
+          if (x <= xmax && x != 0 && lr_entry_j(ent_at(i)) >= k) hl[nh++] = i;
+        };
+        auto flush_adj = [&]() {
+          const int maxh = __reduce_max_sync(0xffffffffu, nh);
+#pragma unroll 1
+          for (int t = 0; t < maxh; ++t)
+            if (t < nh) adj_one(lr_entry_j(ent_at(hl[t])));
+          nh = 0;
+        };
+        if (__any_sync(0xffffffffu, rescan)) {
+#pragma unroll 1
+          for (int i = 0; i < nscan; ++i) {
+            if (__any_sync(0xffffffffu, nh == kHitCap)) flush_adj();
+            if (rescan) note(i);
+          }
+#pragma unroll 1
+          for (int q2 = 0; q2 < nrb; ++q2) {
+            if (__any_sync(0xffffffffu, nh == kHitCap)) flush_adj();
+            if (rescan) note(rb[q2]);
+          }
+          flush_adj();
+        }
+        if (!live) return;
+        // diagonal terms: hdig(I) = hdig(K') + vdg[a1] + vdg[a2] + G(a1,a2),
+        // hmp(I) = hmp(K') + fmpb[a1] + fmpb[a2]
+        adj_gK += gh;
+        adj_gM += gm;
+        atomicAdd(&adj_gv[a1 + sa1 * p.norb], gh);
+        atomicAdd(&adj_gf[a1 + sa1 * p.norb], gm);
+        if (a2 >= 0) {
+          atomicAdd(&adj_gv[a2 + sa2 * p.norb], gh);
+          atomicAdd(&adj_gf[a2 + sa2 * p.norb], gm);
+          const int nt = p.norb * (p.norb + 1) / 2;
+          const int tq = tri(a1, a2);
+          atomicAdd(&adj_sl[nt + tq], gh);
+          if (sa1 == sa2) atomicAdd(&adj_sl[2 * nt + tq], -gh);
+        }
       };
       if (nRr == 1 || !fast) {
         // flat: threads take candidates, every candidate scans all of L_R
+#pragma unroll 1
         for (int t0 = 0; t0 < nA; t0 += blockDim.x) {
           const int t = t0 + tid;
           const bool live = t < nA;
@@ -1670,6 +1347,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
             } else if (sp1 == sp2) {
               // t -> (x < y) over nv1 virtuals
               int x = 0, tt = t;
+#pragma unroll 1
               while (tt >= nv1 - 1 - x) {
                 tt -= nv1 - 1 - x;
                 ++x;
@@ -1683,7 +1361,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
               sa2 = 1;
             }
           }
-          candidate(live, a1, a2, sa1, sa2, nlr, nullptr, 0, bslot + t);
+          candidate(live, a1, a2, sa1, sa2, nlr, nullptr, 0);
         }
       } else {
         // rows: one warp per first added orbital a1; an entry with
@@ -1697,12 +1375,14 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
         int16_t* rowbuf = wrow + wid * kRowCap;
         // rows in zig-zag order over the warps (row lengths fall with the
         // row index for same-spin pairs): even stripes forward, odd backward
+#pragma unroll 1
         for (int t = 0; t * nwarps < nrows; ++t) {
           const int row = (t & 1) ? t * nwarps + (nwarps - 1 - wid) : t * nwarps + wid;
           if (row >= nrows) continue;
           const int a1 = sh.vir[sr][row];
           const uint32_t r1x4 = (uint32_t)(a1 + sr * p.norb) * 0x01010101u;
           int nrb = 0;
+#pragma unroll 1
           for (int i0 = n01; i0 < nlr; i0 += 32) {
             const int i = i0 + lane;
             const bool has = i < nlr && has_byte((uint32_t)ent_at(i), r1x4);
@@ -1716,106 +1396,103 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2(Params p0, BatchArgs ba) {
           __syncwarp();
           const bool overflow = nrb > kRowCap;
           const int ncols = same ? nv1 - 1 - row : sh.nvir[1];
+#pragma unroll 1
           for (int c0 = 0; c0 < ncols; c0 += 32) {
             const int c = c0 + lane;
             const bool live = c < ncols;
             const int a2 = live ? (same ? sh.vir[sc][row + 1 + c] : sh.vir[sc][c]) : 0;
             // a row list that overflowed falls back to the whole of L_R (one
             // call site: the candidate code is instantiated once for rows)
-            // slot: the pair's index in the flat enumeration (row-major
-            // over a1 < a2 for one spin, a1 x a2 for opposite spins)
-            const int tflat = same ? row * (nv1 - 1) - row * (row - 1) / 2 + c : row * sh.nvir[1] + c;
-            candidate(live, a1, a2, sr, sc, overflow ? nlr : n01, rowbuf, overflow ? 0 : nrb, bslot + tflat);
+            candidate(live, a1, a2, sr, sc, overflow ? nlr : n01, rowbuf, overflow ? 0 : nrb);
           }
           __syncwarp();
         }
       }
       __syncthreads();
-      if (ADJ) {
-        // expand this block's dE/dhdig and dE/dhmp sums over F, J, K, fmpb
-        if (tid < 2) adj_sh[tid] = 0.0;
-        __syncthreads();
-        double gk = adj_gK, gmk = adj_gM;
-        for (int o = 16; o > 0; o >>= 1) {
-          gk += __shfl_down_sync(0xffffffffu, gk, o);
-          gmk += __shfl_down_sync(0xffffffffu, gmk, o);
-        }
-        if ((tid & 31) == 0) {
-          atomicAdd(&adj_sh[0], gk);
-          atomicAdd(&adj_sh[1], gmk);
-        }
-        adj_gK = adj_gM = 0.0;
-        __syncthreads();
-        const int n = p.norb, nt = n * (n + 1) / 2, ndn = sh.ndn;
-        double* sF = adj_sl;
-        double* sJ = adj_sl + nt;
-        double* sK = adj_sl + 2 * nt;
-        double* sf = adj_sl + 3 * nt;
-        if (tid == 0) {
-          // hdig(K') = sum_i dn_i F_rr + 1/2 sum_ij dn_i dn_j (J - [same spin] K)
-          const double G = adj_sh[0], M = adj_sh[1];
-          for (int i = 0; i < ndn; ++i) {
-            const int r = sh.dn_so[i], orr = r % n;
-            atomicAdd(&sf[r], sh.dn_sg[i] * M);
-            if (G == 0.0) continue;
-            atomicAdd(&sF[tri(orr, orr)], sh.dn_sg[i] * G);
-            for (int j = 0; j < ndn; ++j) {
-              const int q = sh.dn_so[j];
-              const int t = tri(orr, q % n);
-              const double c = 0.5 * sh.dn_sg[i] * sh.dn_sg[j] * G;
-              atomicAdd(&sJ[t], c);
-              if (r / n == q / n) atomicAdd(&sK[t], -c);
-            }
-          }
-        }
-        for (int a = tid; a < 2 * n; a += blockDim.x) {
-          // vdg[a] = F_aa + sum_i dn_i (J - [same spin] K)(a, r_i) + 1/2 (J_aa - K_aa)
-          const double gv = adj_gv[a];
-          if (adj_gf[a] != 0.0) atomicAdd(&sf[a], adj_gf[a]);
-          if (gv == 0.0) continue;
-          const int oa = a % n, sa = a / n;
-          const int ta = tri(oa, oa);
-          atomicAdd(&sF[ta], gv);
-          atomicAdd(&sJ[ta], 0.5 * gv);
-          atomicAdd(&sK[ta], -0.5 * gv);
-          for (int i = 0; i < ndn; ++i) {
-            const int r = sh.dn_so[i];
-            const int t = tri(oa, r % n);
-            atomicAdd(&sJ[t], sh.dn_sg[i] * gv);
-            if (sa == r / n) atomicAdd(&sK[t], -sh.dn_sg[i] * gv);
-          }
-        }
-        __syncthreads();
-        for (int i = tid; i < 2 * n; i += blockDim.x) adj_gv[i] = adj_gf[i] = 0.0;
-        __syncthreads();
+      // expand this block's dE/dhdig and dE/dhmp sums over F, J, K, fmpb
+      if (tid < 2) adj_sh[tid] = 0.0;
+      __syncthreads();
+      double gk = adj_gK, gmk = adj_gM;
+#pragma unroll 1
+      for (int o = 16; o > 0; o >>= 1) {
+        gk += __shfl_down_sync(0xffffffffu, gk, o);
+        gmk += __shfl_down_sync(0xffffffffu, gmk, o);
       }
+      if ((tid & 31) == 0) {
+        atomicAdd(&adj_sh[0], gk);
+        atomicAdd(&adj_sh[1], gmk);
+      }
+      adj_gK = adj_gM = 0.0;
+      __syncthreads();
+      const int n = p.norb, nt = n * (n + 1) / 2, ndn = sh.ndn;
+      double* sF = adj_sl;
+      double* sJ = adj_sl + nt;
+      double* sK = adj_sl + 2 * nt;
+      double* sf = adj_sl + 3 * nt;
+      if (tid == 0) {
+        // hdig(K') = sum_i dn_i F_rr + 1/2 sum_ij dn_i dn_j (J - [same spin] K)
+        const double G = adj_sh[0], M = adj_sh[1];
+#pragma unroll 1
+        for (int i = 0; i < ndn; ++i) {
+          const int r = sh.dn_so[i], orr = r % n;
+          atomicAdd(&sf[r], sh.dn_sg[i] * M);
+          if (G == 0.0) continue;
+          atomicAdd(&sF[tri(orr, orr)], sh.dn_sg[i] * G);
+#pragma unroll 1
+          for (int j = 0; j < ndn; ++j) {
+            const int q = sh.dn_so[j];
+            const int t = tri(orr, q % n);
+            const double c = 0.5 * sh.dn_sg[i] * sh.dn_sg[j] * G;
+            atomicAdd(&sJ[t], c);
+            if (r / n == q / n) atomicAdd(&sK[t], -c);
+          }
+        }
+      }
+#pragma unroll 1
+      for (int a = tid; a < 2 * n; a += blockDim.x) {
+        // vdg[a] = F_aa + sum_i dn_i (J - [same spin] K)(a, r_i) + 1/2 (J_aa - K_aa)
+        const double gv = adj_gv[a];
+        if (adj_gf[a] != 0.0) atomicAdd(&sf[a], adj_gf[a]);
+        if (gv == 0.0) continue;
+        const int oa = a % n, sa = a / n;
+        const int ta = tri(oa, oa);
+        atomicAdd(&sF[ta], gv);
+        atomicAdd(&sJ[ta], 0.5 * gv);
+        atomicAdd(&sK[ta], -0.5 * gv);
+#pragma unroll 1
+        for (int i = 0; i < ndn; ++i) {
+          const int r = sh.dn_so[i];
+          const int t = tri(oa, r % n);
+          atomicAdd(&sJ[t], sh.dn_sg[i] * gv);
+          if (sa == r / n) atomicAdd(&sK[t], -sh.dn_sg[i] * gv);
+        }
+      }
+      __syncthreads();
+#pragma unroll 1
+      for (int i = tid; i < 2 * n; i += blockDim.x) adj_gv[i] = adj_gf[i] = 0.0;
+      __syncthreads();
     }
-    drain_queue<W, R>(p, wq, qn, true, acc, hp);
-    if (!ADJ && p.rec_mode) unit_compact<W>(p, unit, slot0, ctmp, sh.unit_base);
     block_flush<R>(p, acc, unit, red);
   }
 
-  if (!B || cur_geo >= 0) flush_totals<R>(p, acc, hp, hist, sc.ncand, sc.ncmp, sc.np1, sc.np2);
-  if (ADJ) {
 #pragma unroll
-    for (int k3 = 0; k3 < 3; ++k3)
+  for (int k3 = 0; k3 < 3; ++k3)
 #pragma unroll
-      for (int m = 0; m < R; ++m) {
-        double v = adjr[k3][m];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if ((tid & 31) == 0 && m < p0.metat && v != 0.0) atomicAdd(&p0.g_roots[k3 * p0.metat + m], v);
-      }
-  }
+    for (int m = 0; m < R; ++m) {
+      double v = adjr[k3][m];
+#pragma unroll 1
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if ((tid & 31) == 0 && m < p0.metat && v != 0.0) atomicAdd(&p0.g_roots[k3 * p0.metat + m], v);
+    }
 }
 
 }  // namespace
 
-template <int W, int R, bool B, bool ADJ>
-cudaError_t launch_pt2(const Params& p, const BatchArgs& ba, int grid, size_t smem, cudaStream_t st) {
-  cudaError_t e =
-      cudaFuncSetAttribute(k_pt2<W, R, B, ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int W, int R>
+cudaError_t launch_pt2_adj(const Params& p, int grid, size_t smem, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(k_pt2_adj<W, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_pt2<W, R, B, ADJ><<<grid, kThreads, smem, st>>>(p, ba);
+  k_pt2_adj<W, R><<<grid, kThreads, smem, st>>>(p);
   return cudaGetLastError();
 }
 
