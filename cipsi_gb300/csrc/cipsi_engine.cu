@@ -334,12 +334,11 @@ struct cipsi_ctx {
   double *sink_xam = nullptr, *sink_evp = nullptr;
   long long sink_cap = 0;
   void* sink_host[4] = {nullptr, nullptr, nullptr, nullptr};  // the caller's addresses
-  // the Hamiltonian over the space (cipsi_hamiltonian_build): phases of the
-  // determinants, the caller's Fock matrix when given, pairs by rows
-  int8_t* dsigma = nullptr;
+  // the Hamiltonian over the space (cipsi_hamiltonian_build): the caller's Fock
+  // matrix when given, the kept workspace, pairs by rows
   double* dFraw = nullptr;
-  int32_t* dh_count = nullptr;
-  long long* dh_rowptr = nullptr;
+  unsigned char* dh_work = nullptr;
+  size_t h_work_cap = 0;
   int32_t* dh_col = nullptr;
   double* dh_val = nullptr;
   long long h_cap = 0;
@@ -450,7 +449,7 @@ void cipsi_ctx_destroy(cipsi_ctx* ctx) {
   dfree(ctx->dsel_bits); dfree(ctx->dsel_owner); dfree(ctx->dsel_xam); dfree(ctx->dsel_evp);
   dfree(ctx->dpool_bits); dfree(ctx->dpool_xam); dfree(ctx->dpool_evp);
   dfree(ctx->dunit_pool); dfree(ctx->dunit_nsel); dfree(ctx->dunit_out); dfree(ctx->dscan_total);
-  dfree(ctx->dsigma); dfree(ctx->dFraw); dfree(ctx->dh_count); dfree(ctx->dh_rowptr);
+  dfree(ctx->dFraw); dfree(ctx->dh_work);
   dfree(ctx->dh_col); dfree(ctx->dh_val);
   for (int i = 0; i < 2; ++i) {
     dfree(ctx->dout_bits[i]); dfree(ctx->dout_owner[i]); dfree(ctx->dout_xam[i]); dfree(ctx->dout_evp[i]);
@@ -2736,20 +2735,26 @@ int cipsi_hamiltonian_build(cipsi_ctx* ctx, const double* fock, int32_t jmax, in
   const int n = ctx->d.ncf, W = ctx->W, norb = ctx->d.norb;
   *npairs = 0;
   ctx->have_h = false;
-  int rc;
-  {
-    std::vector<int8_t> sg(n);
-    for (int k = 0; k < n; ++k) sg[k] = ctx->sigma[k] < 0 ? -1 : 1;
-    if ((rc = upload(ctx, &ctx->dsigma, sg.data(), sg.size()))) return rc;
+  // workspace of the build, kept for the next one: row offsets, counts by
+  // segment and by row, phases
+  const int seg = hscan_segment(n), nseg = (n + seg - 1) / seg;
+  const size_t off_seg = ((size_t)n + 1) * 8, off_cnt = off_seg + (size_t)nseg * n * 4, off_sg = off_cnt + (size_t)n * 4;
+  const size_t work = off_sg + (size_t)n;
+  if (work > ctx->h_work_cap) {
+    dfree(ctx->dh_work);
+    ctx->h_work_cap = 0;
+    CK(cudaMalloc((void**)&ctx->dh_work, work));
+    ctx->h_work_cap = work;
   }
+  std::vector<int8_t> sg(n);
+  for (int k = 0; k < n; ++k) sg[k] = ctx->sigma[k] < 0 ? -1 : 1;
+  CK(cudaMemcpyAsync(ctx->dh_work + off_sg, sg.data(), sg.size(), cudaMemcpyHostToDevice, ctx->stream));
   const double* dF = ctx->dF;
   if (fock) {
-    if ((rc = upload(ctx, &ctx->dFraw, fock, (size_t)norb * (norb + 1) / 2))) return rc;
+    const int rc = upload(ctx, &ctx->dFraw, fock, (size_t)norb * (norb + 1) / 2);
+    if (rc) return rc;
     dF = ctx->dFraw;
   }
-  dfree(ctx->dh_count);
-  ++ctx->buf_gen;
-  CK(cudaMalloc((void**)&ctx->dh_count, (size_t)n * sizeof(int32_t)));
   HBuildArgs a{};
   a.p.norb = norb;
   a.p.noca = ctx->d.noca;
@@ -2760,7 +2765,10 @@ int cipsi_hamiltonian_build(cipsi_ctx* ctx, const double* fock, int32_t jmax, in
   a.p.ntttt = ctx->dntttt;
   a.p.F = dF;
   a.S = ctx->dS;
-  a.sigma = ctx->dsigma;
+  a.sigma = reinterpret_cast<const int8_t*>(ctx->dh_work + off_sg);
+  a.seg = seg;
+  a.nseg = nseg;
+  a.segcnt = reinterpret_cast<int32_t*>(ctx->dh_work + off_seg);
   a.n = n;
   a.jmax = jmax < 0 ? n : std::min(jmax, n);
   for (int q = 0; q < 4; ++q) a.hf[q] = 0ull;
@@ -2768,17 +2776,17 @@ int cipsi_hamiltonian_build(cipsi_ctx* ctx, const double* fock, int32_t jmax, in
     a.hf[o >> 6] |= 1ull << (o & 63);
     a.hf[W + (o >> 6)] |= 1ull << (o & 63);
   }
-  a.count = ctx->dh_count;
+  a.count = reinterpret_cast<int32_t*>(ctx->dh_work + off_cnt);
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
-  cudaError_t e = W == 1 ? launch_hpairs<1>(a, false, ctx->stream) : launch_hpairs<2>(a, false, ctx->stream);
-  if (e != cudaSuccess) return fail(ctx, CIPSI_ERR_CUDA, std::string("k_hpairs (count): ") + cudaGetErrorString(e));
+  cudaError_t e = W == 1 ? launch_hcount<1>(a, ctx->stream) : launch_hcount<2>(a, ctx->stream);
+  if (e != cudaSuccess) return fail(ctx, CIPSI_ERR_CUDA, std::string("k_hscan (count): ") + cudaGetErrorString(e));
   std::vector<int32_t> cnt(n);
-  CK(cudaMemcpyAsync(cnt.data(), ctx->dh_count, (size_t)n * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaMemcpyAsync(cnt.data(), a.count, (size_t)n * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->h_rowptr.assign((size_t)n + 1, 0);
   for (int i = 0; i < n; ++i) ctx->h_rowptr[i + 1] = ctx->h_rowptr[i] + cnt[i];
   const long long total = ctx->h_rowptr[n];
-  if ((rc = upload(ctx, &ctx->dh_rowptr, ctx->h_rowptr.data(), ctx->h_rowptr.size()))) return rc;
+  CK(cudaMemcpyAsync(ctx->dh_work, ctx->h_rowptr.data(), ctx->h_rowptr.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
   if (total > ctx->h_cap || !ctx->dh_col) {
     dfree(ctx->dh_col);
     dfree(ctx->dh_val);
@@ -2787,11 +2795,13 @@ int cipsi_hamiltonian_build(cipsi_ctx* ctx, const double* fock, int32_t jmax, in
     CK(cudaMalloc((void**)&ctx->dh_val, (size_t)std::max(total, 1ll) * sizeof(double)));
     ctx->h_cap = std::max(total, 1ll);
   }
-  a.rowptr = ctx->dh_rowptr;
+  a.rowptr = reinterpret_cast<const long long*>(ctx->dh_work);
   a.col = ctx->dh_col;
   a.val = ctx->dh_val;
-  e = W == 1 ? launch_hpairs<1>(a, true, ctx->stream) : launch_hpairs<2>(a, true, ctx->stream);
-  if (e != cudaSuccess) return fail(ctx, CIPSI_ERR_CUDA, std::string("k_hpairs (fill): ") + cudaGetErrorString(e));
+  int dev_sms = 0;
+  CK(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
+  e = W == 1 ? launch_hfill<1>(a, dev_sms, ctx->stream) : launch_hfill<2>(a, dev_sms, ctx->stream);
+  if (e != cudaSuccess) return fail(ctx, CIPSI_ERR_CUDA, std::string("k_hscan (fill): ") + cudaGetErrorString(e));
   CK(cudaEventRecord(ctx->ev1, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   CK(cudaEventElapsedTime(&ctx->h_ms, ctx->ev0, ctx->ev1));

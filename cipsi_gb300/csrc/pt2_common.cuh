@@ -231,9 +231,10 @@ int cand_ctas();
 template <int W, int R>
 cudaError_t launch_pt2_adj(const Params& p, int grid, size_t smem, cudaStream_t st);
 
-// The Hamiltonian over a determinant list by rows (hbuild.cu): pass 1
+// The Hamiltonian over a determinant list by rows (hbuild.cu): launch_hcount
 // counts, per row i, the columns j < min(i, jmax) within two excitations;
-// pass 2 writes them, in increasing j, from rowptr[i] on.
+// launch_hfill writes them and their elements, in increasing j, from rowptr[i]
+// on.
 struct HBuildArgs {
   Params p;                 // integrals (pairtab, ntttt, eri / eri64, F) and norb
   const uint64_t* S;        // n x 2W words
@@ -241,13 +242,18 @@ struct HBuildArgs {
   int n;                    // determinants (rows)
   int jmax;                 // columns j < min(i, jmax)
   uint64_t hf[4];           // the reference determinant (2W words)
-  int32_t* count;           // pass 1 output: columns per row
-  const long long* rowptr;  // pass 2 input: first pair of each row
-  int32_t* col;             // pass 2 outputs
+  int seg, nseg;            // columns per segment (hscan_segment), segments
+  int32_t* segcnt;          // nseg x n: hits, then their exclusive sums over the segments
+  int32_t* count;           // columns per row
+  const long long* rowptr;  // first pair of each row
+  int32_t* col;
   double* val;
 };
 
+int hscan_segment(int n);
 template <int W>
-cudaError_t launch_hpairs(const HBuildArgs& a, bool fill, cudaStream_t st);
+cudaError_t launch_hcount(const HBuildArgs& a, cudaStream_t st);
+template <int W>
+cudaError_t launch_hfill(const HBuildArgs& a, int sms, cudaStream_t st);
 
 }  // namespace cipsi_dev
