@@ -31,6 +31,10 @@ def test_scan_edges(tmp_path, engine_lib, norb, ncf, jmax):
     lib.cipsi_hamiltonian_build.argtypes = [P, P, ctypes.c_int32, ctypes.POINTER(I64)]
     lib.cipsi_hamiltonian_get.argtypes = [P, ctypes.c_int32, ctypes.c_int32, P, P, P]
     with engine.Context(inp.dims) as ctx:
+        if n == 1:  # S of the reference determinant alone has no hole list: the upload refuses it
+            with pytest.raises(engine.CipsiError, match="null array"):
+                ctx.upload(inp)
+            return
         ctx.upload(inp)
         for _ in range(2):  # the second build reuses the workspace
             npairs = I64()
