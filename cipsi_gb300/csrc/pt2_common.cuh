@@ -161,10 +161,10 @@ __device__ __forceinline__ void kahan_add(double& s, double& c, double x) {
 
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxDn = 48;      // spin orbitals where K' differs from the reference
-constexpr int kMaxG = 4;        // rows of a block worked together
+constexpr int kMaxG = 16;       // rows of a block worked together
 constexpr int kDenseCap = 64;   // per-warp list of (entry, row): the entry touches the whole row
 constexpr int kEvCap = 256;     // per-warp ring of (entry, row, column) events
-constexpr int kHitCap2 = 32 + 32 * kMaxG;  // per-warp list of (entry, row): the entry holds the row's a1
+constexpr int kHitCap2 = 32 + 32 * 4;  // per-warp list of (entry, row): the entry holds the row's a1
 constexpr int kLrWarpG = 1024;  // overflow entries of each L_R list of a warp, in global scratch
 
 // One warp's part of k_cand's shared memory.  The L_R lists are short: what
@@ -172,7 +172,7 @@ constexpr int kLrWarpG = 1024;  // overflow entries of each L_R list of a warp, 
 template <int W, int R>
 struct WarpMem {
   static constexpr int NC = 64 * W;                  // columns: empty orbitals of one spin
-  static constexpr int XN = R <= 2 ? 128 : 64 * W;   // (row, column) places of the rows worked together
+  static constexpr int XN = R <= 2 ? 128 : 64 * W;   // candidates of the rows worked together
   static constexpr int CapA = 64;                    // L_R entries with |K' \ j| <= 1
   static constexpr int CapB = R == 1 ? 96 : 64;      // and with |K' \ j| = 2
   double vd[2][NC];                      // hdig(K'+a) - hdig(K') by (spin, column)
@@ -184,14 +184,16 @@ struct WarpMem {
   uint32_t own[NC][2 * W];               // candidates (row, column) owned by an earlier generator or in S;
                                          //   from the block's row pass on: those still alive
   uint32_t owncol[2][2 * W];             // orbitals (by spin, column) every candidate of which is owned
-  uint32_t dense[kDenseCap];             // entry << 2 | row
-  uint32_t ev[kEvCap];                   // entry << 8 | list << 7 | place
-  uint32_t hits[kHitCap2];               // entry << 2 | row
-  int ra1[kMaxG], rrow[kMaxG], rpA[kMaxG], rpX[kMaxG];
+  uint32_t dense[kDenseCap];             // entry << 4 | row, rows ascending
+  uint32_t ev[kEvCap];                   // entry << 8 | list << 7 | candidate
+  uint32_t hits[kHitCap2];               // entry << 4 | row
+  int ra1[kMaxG], rrow[kMaxG], rpA[kMaxG], rpX[kMaxG], rfirst[kMaxG];
   uint32_t rsg[kMaxG];
-  uint16_t xf[XN];                       // per place: element found, non-zero, lesp
+  uint32_t rpos[64];                     // by spin orbital code, a byte each: its place in rows[], 255: none
+  uint16_t xf[XN];                       // per candidate: element found, non-zero, lesp
   uint16_t cols[XN];                     // surviving candidates: row << 8 | column
   uint8_t rows[NC];                      // the block's rows with a candidate alive
+  uint8_t dfirst[kMaxG + 4];             // by row: its first place in dense[]
   uint8_t dn_so[kMaxDn], dn_sg[kMaxDn];  // where K' differs from the reference: code, 1 = added
 };
 template <int W, int R>

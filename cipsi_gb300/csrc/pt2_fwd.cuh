@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
     int ws = 1;  // warps that share a block
     // the warp's block
     bool two = false, same = false, opened = false;
-    int so1 = 0, so2 = 0, sr = 0, sc = 0, hfR = 0, symR = 0, bslot = 0, ncol = 0, rcol = 0;
+    int so1 = 0, so2 = 0, sr = 0, sc = 0, hfR = 0, symR = 0, bslot = 0, ncol = 0;
     int nA = 0, nB = 0, sub = 0, capA = 0, capB = 0, nlive = 0, lr0 = 0;
     const uint32_t *geA = nullptr, *geB = nullptr;  // entries beyond capA / capB
     const uint2 *gjA = nullptr, *gjB = nullptr;
@@ -560,7 +560,6 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
       clear_word<2 * W>(kp.w, sr * W + (o1 >> 6), 1ull << (o1 & 63));
       if (two) clear_word<2 * W>(kp.w, sc * W + (o2 >> 6), 1ull << (o2 & 63));
       ncol = sh.nvir[sc];
-      rcol = (65536 + ncol - 1) / ncol;  // x / ncol = x * rcol >> 16 for x < 128
       return (1ull << e1) | (two ? 1ull << e2 : 0ull);
     };
 
@@ -640,6 +639,7 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
 #pragma unroll 1
       for (int i = lane; i < nrows * 2 * W; i += 32) (&wm.own[0][0])[i] = 0u;
       if (lane < 4 * W) (&wm.owncol[0][0])[lane] = 0u;
+      wm.rpos[lane] = wm.rpos[32 + lane] = 0xffffffffu;
       if (lane < 2 * W) {
         const uint64_t x = get_word<2 * W>(kp.w, lane);
         uint64_t y = parity_below(x);
@@ -794,11 +794,16 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
           any = any || x != 0ull;
         }
         const unsigned lm = __ballot_sync(kFull, any);
-        if (any) wm.rows[nlive + __popc(lm & below)] = (uint8_t)rw;
+        if (any) {
+          const int at = nlive + __popc(lm & below);
+          wm.rows[at] = (uint8_t)rw;
+          if (two) reinterpret_cast<uint8_t*>(wm.rpos)[a1 + sr * norb] = (uint8_t)at;
+        }
         nlive += __popc(lm);
       }
       ncand += __reduce_add_sync(kFull, nvalid);
       __syncwarp();
+      ncmp += (unsigned long long)nB * (unsigned)nlive;
       if (nlive > 0) block_energies();
       return true;
     };
@@ -808,23 +813,44 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
     auto open_rows = [&]() {
       nal = pos = 0;
       hasx = false;
-      G = two ? min(min(kMaxG, max(1, XN / ncol)), nlive - lr0) : 1;
-      if (lane < G && two) {
-        const int rw = wm.rows[lr0 + lane], a1 = sh.vir[sr][rw], o1 = orb_of(so1), o2 = orb_of(so2);
+      // as many rows as their candidates fit (one always does): what is done
+      // once per group of rows counts less, and the batches of 32 candidates are
+      // fuller, than with up to four rows by their number of columns (37
+      // orbitals, four irreps, S = 334: 0.93 -> 0.80 ms; 60 orbitals, S = 2001,
+      // an eighth of the generators: 6.25 -> 5.95)
+      const int lrb = lr0, avail = two ? min(kMaxG, nlive - lrb) : 1;
+      const int rw = lane < avail ? wm.rows[lrb + lane] : 0;
+      int mine = 0;
+      if (lane < avail) {
+#pragma unroll
+        for (int h = 0; h < 2 * W; ++h) mine += __popc(wm.own[rw][h]);
+      }
+      int incl = mine;
+#pragma unroll
+      for (int o = 1; o < kMaxG; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += y;
+      }
+      G = __popc(__ballot_sync(kFull, lane < avail && incl <= XN));
+      if (lane < G) {
+        wm.rfirst[lane] = incl - mine;
         wm.rrow[lane] = rw;
-        wm.ra1[lane] = a1;
-        wm.rpA[lane] = __ldg(&p.pairtab[o1 * norb + a1]);
-        wm.rpX[lane] = __ldg(&p.pairtab[o2 * norb + a1]);
-        wm.rsg[lane] = par_of(sr, o1) ^ par_of(sc, o2) ^ par_of(sr, a1);
-        wm.rhv[lane] = hK + wm.vd[sr][rw];
-        wm.rmp[lane] = mK + __ldg(&p.fmpb[a1 + sr * norb]);
+        if (two) {
+          const int a1 = sh.vir[sr][rw], o1 = orb_of(so1), o2 = orb_of(so2);
+          wm.ra1[lane] = a1;
+          wm.rpA[lane] = __ldg(&p.pairtab[o1 * norb + a1]);
+          wm.rpX[lane] = __ldg(&p.pairtab[o2 * norb + a1]);
+          wm.rsg[lane] = par_of(sr, o1) ^ par_of(sc, o2) ^ par_of(sr, a1);
+          wm.rhv[lane] = hK + wm.vd[sr][rw];
+          wm.rmp[lane] = mK + __ldg(&p.fmpb[a1 + sr * norb]);
+        }
       }
 #pragma unroll 1
       for (int g = 0; g < G; ++g) {
-        const int rw = wm.rows[lr0 + g];
+        const int r = __shfl_sync(kFull, rw, g);
 #pragma unroll
         for (int h = 0; h < 2 * W; ++h) {
-          const uint32_t am = wm.own[rw][h];
+          const uint32_t am = wm.own[r][h];
           if ((am >> lane) & 1u) wm.cols[nal + __popc(am & below)] = (uint16_t)(g << 8 | (32 * h + lane));
           nal += __popc(am);
         }
@@ -838,6 +864,7 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
       enum { kDense, kSparseA, kSparseB, kDone };
       int stage = nA > 0 ? kDense : (nB > 0 ? kSparseB : kDone);
       int it = 0, nh = 0, nd = 0, ne = 0, ev0 = 0;
+      int pat = lane, pg = 0;  // this lane's next pair of A entry and row, row after row
 #pragma unroll 1
       for (;;) {
         if (stage != kDone && ne < 32 && nd <= kDenseCap - 32) {
@@ -846,34 +873,42 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
           uint32_t at = 0, E = 0;
           int g = 0;
           if (stage <= kSparseA) {
-            const int i = it + lane;
-            has = i < nA * G;
-            at = (uint32_t)i / (uint32_t)G;
-            g = i - (int)at * G;
-            if (has) E = eA_at((int)at);
+#pragma unroll 1
+            while (pat >= nA && pg < G) {
+              pat -= nA;
+              ++pg;
+            }
+            has = pg < G;
+            at = (uint32_t)pat;
+            g = pg;
+            if (has) E = eA_at(pat);
+            pat += 32;
             it += 32;
           } else {
 #pragma unroll 1
             while (nh < 32 && it < nB) {
               const bool in = it + lane < nB;
               const uint32_t e = in ? eB_at(it + lane) : 0u;
-              unsigned hm = 0;
-              if (two) {
-#pragma unroll 1
-                for (int gg = 0; gg < G; ++gg)
-                  hm |= has_byte(e, (uint32_t)(wm.ra1[gg] + sr * norb) * 0x01010101u) ? 1u << gg : 0u;
-              } else {
-                hm = 1u;
+              unsigned hm = in && !two ? 1u : 0u;
+              if (in && two) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                  const uint32_t d = (uint32_t)reinterpret_cast<const uint8_t*>(wm.rpos)[(e >> (8 * q)) & 0xffu] - (uint32_t)lrb;
+                  hm |= d < (uint32_t)G ? 1u << d : 0u;
+                }
               }
-              if (!in) hm = 0u;
-              ncmp += 32u;
               if (__any_sync(kFull, hm != 0u)) {
+                // up to four rows an entry
+                const int n = __popc(hm);
+                const unsigned n0 = __ballot_sync(kFull, n & 1), n1 = __ballot_sync(kFull, n & 2),
+                               n2 = __ballot_sync(kFull, n & 4);
+                int o = nh + __popc(n0 & below) + 2 * __popc(n1 & below) + 4 * __popc(n2 & below);
+                nh += __popc(n0) + 2 * __popc(n1) + 4 * __popc(n2);
 #pragma unroll 1
-                for (int gg = 0; gg < G; ++gg) {
-                  const bool hit = (hm >> gg) & 1u;
-                  const unsigned bm = __ballot_sync(kFull, hit);
-                  if (hit) wm.hits[nh + __popc(bm & below)] = (uint32_t)(it + lane) << 2 | (uint32_t)gg;
-                  nh += __popc(bm);
+                while (hm) {
+                  const int gg = __ffs((int)hm) - 1;
+                  hm &= hm - 1u;
+                  wm.hits[o++] = (uint32_t)(it + lane) << 4 | (uint32_t)gg;
                 }
               }
               it += 32;
@@ -882,8 +917,8 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
             const int take = min(nh, 32);
             has = lane < take;
             const uint32_t x = wm.hits[lane];
-            at = x >> 2;
-            g = (int)(x & 3u);
+            at = x >> 4;
+            g = (int)(x & 15u);
             if (has) E = eB_at((int)at);
             nh -= take;
 #pragma unroll 1
@@ -901,13 +936,13 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
             whole = !two || a1in || (at < (uint32_t)capA ? wm.jhA[at].y : gjA[at - capA].y) < 1u << 16;
           if (stage == kDense) {
             const unsigned bm = __ballot_sync(kFull, whole);
-            if (whole) wm.dense[nd + __popc(bm & below)] = at << 2 | (uint32_t)g;
+            if (whole) wm.dense[nd + __popc(bm & below)] = at << 4 | (uint32_t)g;
             nd += __popc(bm);
           } else {
             const bool sparse = has && (stage == kSparseB || !whole);
             if (__any_sync(kFull, sparse)) {
               // the columns this entry holds, entry after entry
-              const int rw = sparse ? (two ? wm.rrow[g] : 0) : 0;
+              const int rw = sparse ? wm.rrow[g] : 0;
               unsigned em[4], mine = 0;
 #pragma unroll
               for (int q = 0; q < 4; ++q) {
@@ -926,7 +961,10 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
                 const int q = __ffs((int)mine) - 1;
                 mine &= mine - 1u;
                 const int col = sh.colof[(E >> (8 * q)) & 0xff];
-                wm.ev[o++ & (kEvCap - 1)] = at << 8 | (stage == kSparseB ? 128u : 0u) | (uint32_t)(g * ncol + col);
+                int x = wm.rfirst[g] + __popc(wm.own[rw][col >> 5] & ((1u << (col & 31)) - 1u));
+#pragma unroll
+                for (int h = 0; h < 2 * W - 1; ++h) x += h < (col >> 5) ? __popc(wm.own[rw][h]) : 0;
+                wm.ev[o++ & (kEvCap - 1)] = at << 8 | (stage == kSparseB ? 128u : 0u) | (uint32_t)x;
               }
             }
           }
@@ -935,7 +973,7 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
         if ((nd > 0 || ne > 0) && !hasx) {
           hasx = true;
 #pragma unroll 1
-          for (int c = lane; c < G * ncol; c += 32) {
+          for (int c = lane; c < nal; c += 32) {
             wm.xf[c] = 0;
 #pragma unroll
             for (int m = 0; m < R; ++m) wm.xb[m][c] = 0.0;
@@ -944,24 +982,38 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
         }
         const bool last_dense = stage == kDense && it >= nA * G;
         if (nd > kDenseCap - 32 || (nd > 0 && last_dense)) {
-          // an element for every surviving candidate of the entry's row
+          // an element for every surviving candidate of the entry's row: each lane
+          // goes through its own row's entries
+          if (lane <= G) {
+            int lo = 0, hi = nd;
+#pragma unroll 1
+            while (lo < hi) {
+              const int mid = (lo + hi) >> 1;
+              if ((int)(wm.dense[mid] & 15u) < lane) lo = mid + 1;
+              else hi = mid;
+            }
+            wm.dfirst[lane] = (uint8_t)lo;
+          }
+          __syncwarp();
 #pragma unroll 1
           for (int c0 = 0; c0 < nal; c0 += 32) {
-            const bool act = c0 + lane < nal;
-            const int rc = act ? wm.cols[c0 + lane] : 0;
+            const int x = c0 + lane;
+            const bool act = x < nal;
+            const int rc = act ? wm.cols[x] : 0;
             const int rg = rc >> 8, c = rc & 0xff;
+            int d = act ? wm.dfirst[rg] : 0;
+            const int d1 = act ? wm.dfirst[rg + 1] : 0;
+            if (!__any_sync(kFull, d < d1)) continue;
             const int a1c = two ? wm.ra1[rg] + sr * norb : -1, a2c = sh.vir[sc][c] + sc * norb;
-            const int x = rg * ncol + c;
             double v[R];
 #pragma unroll
             for (int m = 0; m < R; ++m) v[m] = wm.xb[m][x];
             uint32_t xf = 0;
             unsigned n1 = 0, nt = 0;
 #pragma unroll 1
-            for (int d = 0; d < nd; ++d) {
-              const uint32_t de = wm.dense[d];
-              if (act && rg == (int)(de & 3u)) {
-                const int i = (int)(de >> 2);
+            for (; __any_sync(kFull, d < d1); ++d) {
+              if (d < d1) {
+                const int i = (int)(wm.dense[d] >> 4);
                 const uint2 jh = i < capA ? wm.jhA[i] : gjA[i - capA];
                 const int j = (int)jh.x;
                 const Elem el = element_of<W>(p, wm.par, kp, a1c, a2c, eA_at(i), jh);
@@ -989,6 +1041,8 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
         if (last_dense) {
           stage = two ? kSparseA : (nB > 0 ? kSparseB : kDone);
           it = 0;
+          pat = lane;
+          pg = 0;
         } else if (stage == kSparseA && it >= nA * G) {
           stage = nB > 0 ? kSparseB : kDone;
           it = 0;
@@ -1001,7 +1055,7 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
           const uint32_t e = wm.ev[(ev0 + (act ? lane : 0)) & (kEvCap - 1)];
           ne -= cnt;
           ev0 += cnt;
-          const int x = (int)(e & 127u), rg = (x * rcol) >> 16, c = x - rg * ncol, i = (int)(e >> 8);
+          const int x = (int)(e & 127u), i = (int)(e >> 8), rc = wm.cols[x], rg = rc >> 8, c = rc & 0xff;
           double v[R];
 #pragma unroll
           for (int m = 0; m < R; ++m) v[m] = 0.0;
@@ -1105,13 +1159,12 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
         }
         // the next candidates of the rows
         live = pos + lane < nal;
-        const int rc = live ? wm.cols[pos + lane] : 0;
+        const int xi = pos + lane, rc = live ? wm.cols[xi] : 0;
         pos += 32;
         if (live) {
           const int rg = rc >> 8, c = rc & 0xff;
           const int a2 = sh.vir[sc][c];
           const int o1 = orb_of(so1), o2 = orb_of(so2);
-          const int xi = rg * ncol + c;
           uint32_t xf = 0;
           if (hasx) xf = wm.xf[xi];
           hx = (xf & kXHas) != 0u;
