@@ -309,7 +309,7 @@ struct cipsi_ctx {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, evk = nullptr;  // evk: end of k_pt2
   long long last_launches = 0;
   // launch tuning (cipsi_set_tuning): R blocks per work unit for generators
-  // of excitation rank >= 2 (rank 0/1 generators get one block per unit),
+  // of excitation rank >= 2 (those of rank 0 get one block per unit, rank 1 up to kLowChunk),
   // and CTAs per SM (0 = as many as the shared-memory L_R size allows)
   int tune_r_chunk = 6;
   int tune_ctas = 0;
@@ -715,18 +715,21 @@ struct RunPlan {
   bool pertu_ref = false, pertu_mono = false;
 };
 
-constexpr int kLowChunk = 6;  // of the reference and its singles: their L_R are the longest
+// of the singles of the reference: a block a warp (60 orbitals, S = 2001: 41.2 ms at 4, 41.7 at 6,
+// 39.7 at 8, 40.5 at 12; 45 orbitals, S = 451: 4.12, 4.16, 3.88, 4.08)
+constexpr int kLowChunk = 8;
 
 // Blocks of removed electrons per work unit of the forward kernels.  k_cand's
 // warps take the blocks of a unit on their own, so a unit wants a few per warp:
 // 16 at the default r_chunk of 6 (2.7 r_chunk above it; r_chunk itself below,
 // where the caller asks for fine units).  At the default, when the run has few
-// blocks, no more than leaves eight units per CTA, down to two blocks.
+// blocks, no more than leaves six units per CTA, down to two blocks (37
+// orbitals, S = 334: 940 us at six, 1027 at eight).
 // (60 orbitals, S = 2001: 45.8 ms at 24, 45.5 at 16, 47.3 at 8, 55 at 60; one
 // shard of 120 orbitals: 57, 55, 54 ms.)
 int unit_blocks(int r_chunk, long long run_blocks, int sms) {
   if (r_chunk < 6) return r_chunk;
-  return (int)std::max(2ll, std::min<long long>(8ll * r_chunk / 3, run_blocks / (16ll * sms)));
+  return (int)std::max(2ll, std::min<long long>(8ll * r_chunk / 3, run_blocks / (12ll * sms)));
 }
 // all blocks of a run, about: generators times pairs of electrons
 long long run_blocks(const cipsi_ctx* ctx, const cipsi_opts* o) {
@@ -782,7 +785,7 @@ void plan_run(const cipsi_ctx* ctx, const cipsi_opts* o, int r_chunk, int low_ch
   }
   const int ngen = (int)gens.size();
   // work units: a generator's R blocks that have an allowed rank-change class
-  // are split into chunks (one block per unit for generators of rank 0 and 1,
+  // are split into chunks (one block per unit for rank 0, up to kLowChunk for rank 1,
   // which meet most of S; r_chunk blocks for the others), so one heavy
   // generator does not serialise on one SM; low-rank generators are queued
   // first.
@@ -850,7 +853,7 @@ void plan_run(const cipsi_ctx* ctx, const cipsi_opts* o, int r_chunk, int low_ch
         if (m & (1u << (hfR + aV - nRr + 2))) return true;
       return false;
     };
-    const int kRChunk = ctx->rank[k] <= 1 ? low_chunk : kRChunkHigh;
+    const int kRChunk = ctx->rank[k] == 0 ? 1 : ctx->rank[k] == 1 ? low_chunk : kRChunkHigh;
     int cnt = 0, start = -1, last = -1;
     long long slots = 0;
     for (int r = 0; r < nR; ++r) {

@@ -33,6 +33,7 @@
 namespace cipsi_dev {
 namespace {
 
+constexpr int kShareNb = 256;  // neighbours of a generator from which on a lone block's L_R is built once
 constexpr int kWindow = 256;  // blocks of a unit laid out in shared memory at a time
 // a column of the rows worked together: element found, one not zero, lesp
 constexpr uint32_t kXHas = 0x8000u, kXNz = 0x4000u, kXLesp = 0x3fffu;
@@ -663,13 +664,16 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
       }
       bool dead = false, over = false;
       int nc = 0, t0 = 0;
+      // (lists given: the owners, then the entries of list A)
+      const int tend = listed ? nown + nA : nnb;
 #pragma unroll 1
-      while (!over && !dead && (t0 < nnb || nc > 0)) {
+      while (!over && !dead && (t0 < tend || nc > 0)) {
 #pragma unroll 1
-        while (nc < 32 && t0 < nnb) {
+        while (nc < 32 && t0 < tend) {
           const int t = t0 + lane;
-          const int m = t < nnb ? __popcll(my_nb_em[t] & ~rmask) : 9;
-          const bool in = m <= 2 && (!listed || t < nown || m == 0);
+          int m = 9;
+          if (t < tend) m = listed && t >= nown ? 3 * (int)(gjA[t - nown].y >> 16) : __popcll(my_nb_em[t] & ~rmask);
+          const bool in = m <= 2;
           const unsigned bm = __ballot_sync(kFull, in);
           if (in) wm.hits[nc + __popc(bm & below)] = (uint32_t)t;
           nc += __popc(bm);
@@ -682,9 +686,12 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
         __syncwarp();
         wm.hits[lane] = later;
         nc -= take;
-        const bool owner = t < nown;
+        const bool owner = t < nown;  // (or no entry)
         uint3 en = make_uint3(0u, 0u, 9u << 16);
-        if (t >= 0) en = make_entry<W>(p, kp, my_nb_j[t]);
+        if (t >= 0) {
+          if (listed && !owner) en = make_uint3(geA[t - nown], gjA[t - nown].x, gjA[t - nown].y);
+          else en = make_entry<W>(p, kp, my_nb_j[t]);
+        }
         const int m = (int)(en.z >> 16);
         // every candidate of the block has this owner
         dead = __any_sync(kFull, t >= 0 && owner && (m == 0 || (!two && m == 1)));
@@ -1269,14 +1276,25 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
           sh.blk_r[bi] = (uint16_t)r;
           sh.blk_slot[bi] = s0 + incl - nc;
         }
+        // A warp takes whole blocks; only where the unit has few (the reference's
+        // units hold one) several share a block, each with its own copy of L_R
+        // and every second, fourth, eighth row.  Opening a block is most of the
+        // work where candidates are few, so idle warps cost less than copies:
+        // sharing below 16, 8, 4 blocks took 1277 us on 37 orbitals (S = 334),
+        // below 8, 4, 2 1027, below 6, 3, 2 940; 60 orbitals (S = 2001) 44.7,
+        // 42.1 and 41.9 ms; the other way on a two-root active space of 120
+        // orbitals, 67.5 and 69.  One block and a long L_R (the reference's own):
+        // all warps share one copy (45 orbitals, S = 451: its blocks took up to
+        // 5.0 ms, 6 to a unit, of a launch whose work is 3.7 ms a CTA; now 0.9).
+        const bool all = tb == 1 && nnb >= kShareNb;
+        if (all && tid < tb) sh.big[tid] = (uint16_t)tid;
         if (tid == 0) {
           sh.job = 0;
-          sh.nbig = 0;
-          sh.nblk = tb;
+          sh.nbig = all ? tb : 0;
+          sh.nblk = all ? 0 : tb;
         }
         slots += ts;
-        // few blocks: several warps share one, each with its own copy of L_R
-        ws = tb >= 2 * kWarps ? 1 : tb >= kWarps ? 2 : tb >= kWarps / 2 ? 4 : kWarps;
+        ws = tb >= 6 ? 1 : tb >= 3 ? 2 : tb >= 2 ? 4 : kWarps;
         __syncthreads();
       } else if (ph == kPhBig) {
         // L_R of the block by the whole CTA, in the CTA's global scratch (the
