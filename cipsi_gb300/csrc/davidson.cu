@@ -15,10 +15,15 @@
 //
 // Kernels: k_spmm (H times a block of vectors: one warp per row, the row's
 // nonzeros over the lanes, a shuffle reduction per vector), k_gram (V^T T:
-// one CTA per output element, fixed-order tree sums, so results are
-// reproducible run to run), k_combine (X = V S, thread per row), k_precond.
-// HBM-bound: each product reads the 12 bytes of every nonzero once, and the
-// vectors (8 bytes per row and vector) stay L2-resident up to ~10^6 rows.
+// one CTA per output element, fixed-order sums, so results are reproducible
+// run to run), k_combine (X = V S), k_residual, k_precond.  Each product reads
+// the 12 bytes of every nonzero once, and the vectors (8 bytes per row and
+// vector) stay L2-resident up to ~10^6 rows.  At a few thousand rows an
+// iteration is some twenty launches of a few microseconds: what it waits for is
+// the host, so the small matrices travel as kernel arguments or stay on the
+// device, and the host waits four times an iteration (6,001 rows, 240,000
+// elements, 14 iterations: 6.2 ms with a wait after every product and copies
+// between the work vectors, k_gram 14 us and k_combine 8.5 us each; now 4.6 ms).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -64,48 +69,89 @@ __global__ void __launch_bounds__(256) k_spmm(int n, const long long* __restrict
   }
 }
 
-// G[a * kb + b] = sum_i A[a * lda + i] * B[b * ldb + i]; one CTA per (a, b)
-__global__ void __launch_bounds__(256) k_gram(int n, const double* __restrict__ A, int lda, int ka,
-                                              const double* __restrict__ B, int ldb, int kb, double* __restrict__ G) {
-  __shared__ double red[256];
-  const int a = blockIdx.x / kb, b = blockIdx.x % kb;
-  double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s = fma(A[(size_t)a * lda + i], B[(size_t)b * ldb + i], s);
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+// G[a * kb + b] = sum_i A[a * lda + i] * B[b * ldb + i]; one CTA per (a, b) --
+// or, with norms, G[a] = the (a, a) elements alone.  Bound by the latency of
+// its loads (a thread reads n / 256 pairs): four independent chains.
+__global__ void __launch_bounds__(256) k_gram(int n, const double* __restrict__ A, int lda,
+                                              const double* __restrict__ B, int ldb, int kb, int norms,
+                                              double* __restrict__ G) {
+  __shared__ double red[8];
+  const int a = norms ? blockIdx.x : blockIdx.x / kb, b = norms ? blockIdx.x : blockIdx.x % kb;
+  const double* x = A + (size_t)a * lda;
+  const double* y = B + (size_t)b * ldb;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  int i = threadIdx.x;
+  for (; i + 768 < n; i += 1024) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s[q] = fma(__ldg(&x[i + 256 * q]), __ldg(&y[i + 256 * q]), s[q]);
   }
-  if (threadIdx.x == 0) G[(size_t)a * kb + b] = red[0];
-  (void)ka;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (i + 256 * q < n) s[q] = fma(__ldg(&x[i + 256 * q]), __ldg(&y[i + 256 * q]), s[q]);
+  double t = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    t = red[0];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) t += red[w];
+    G[blockIdx.x] = t;
+  }
 }
 
-// Y[:, b] = beta * Y[:, b] + sum_a A[:, a] S[a * kb + b]   (S: ka x kb, row-major)
+// a small matrix as a kernel argument: at most (4 nb) x nb, nb = 10
+struct Small {
+  double s[400];
+};
+
+// Y[:, b] = beta * Y[:, b] + sum_a A[:, a] S[a * kb + b]   (S: ka x kb, row-major;
+// with D, S = -D of the device).  A thread takes a row; with few rows each
+// column b has its own threads (grid.y = kb), else a thread goes through the
+// columns, so that A is read once (its rows stay in L1).
 __global__ void __launch_bounds__(256) k_combine(int n, const double* __restrict__ A, int lda, int ka,
-                                                 const double* __restrict__ S, int kb, double beta,
-                                                 double* __restrict__ Y, int ldy) {
-  extern __shared__ double sS[];
-  for (int i = threadIdx.x; i < ka * kb; i += blockDim.x) sS[i] = S[i];
+                                                 const __grid_constant__ Small S, const double* __restrict__ D, int kb,
+                                                 double beta, double* __restrict__ Y, int ldy) {
+  __shared__ double sS[400];
+  for (int i = threadIdx.x; i < ka * kb; i += blockDim.x) sS[i] = D ? -D[i] : S.s[i];
   __syncthreads();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    for (int b = 0; b < kb; ++b) {
+    for (int b = blockIdx.y; b < kb; b += gridDim.y) {
       double y = beta == 0.0 ? 0.0 : beta * Y[(size_t)b * ldy + i];
-      for (int a = 0; a < ka; ++a) y = fma(A[(size_t)a * lda + i], sS[a * kb + b], y);
+#pragma unroll 8
+      for (int a = 0; a < ka; ++a) y = fma(__ldg(&A[(size_t)a * lda + i]), sS[a * kb + b], y);
       Y[(size_t)b * ldy + i] = y;
     }
   }
 }
 
-// T[:, b] = R[:, b] / (theta_b - d_i), the denominator kept away from zero
-__global__ void k_precond(int n, const double* __restrict__ R, int ldr, const double* __restrict__ diag,
-                          const double* __restrict__ theta, int kb, double* __restrict__ T, int ldt) {
+struct Theta {
+  double theta[kMaxBlock];
+  int from[kMaxBlock];
+};
+// T[:, b] = AX[:, b] - theta_b X[:, b]
+__global__ void k_residual(int n, const double* __restrict__ AX, const double* __restrict__ X,
+                           const __grid_constant__ Theta th, int nx, double* __restrict__ T) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    for (int b = 0; b < kb; ++b) {
-      double den = theta[b] - diag[i];
+    for (int b = blockIdx.y; b < nx; b += gridDim.y)
+      T[(size_t)b * n + i] = fma(X[(size_t)b * n + i], -th.theta[b], AX[(size_t)b * n + i]);
+}
+
+// T[:, b] = R[:, from_b] / (theta_b - d_i), the denominator kept away from zero
+__global__ void k_precond(int n, const double* __restrict__ R, const double* __restrict__ diag,
+                          const __grid_constant__ Theta th, int kb, double* __restrict__ T) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    for (int b = blockIdx.y; b < kb; b += gridDim.y) {
+      double den = th.theta[b] - diag[i];
       if (std::fabs(den) < 1e-8) den = den < 0.0 ? -1e-8 : 1e-8;
-      T[(size_t)b * ldt + i] = R[(size_t)b * ldr + i] / den;
+      T[(size_t)b * n + i] = R[(size_t)th.from[b] * n + i] / den;
     }
+}
+
+// V[:, b] = the unit vector at row from_b (V zeroed)
+__global__ void k_units(int n, const __grid_constant__ Theta th, int nb, double* __restrict__ V) {
+  if ((int)threadIdx.x < nb) V[(size_t)threadIdx.x * n + th.from[threadIdx.x]] = 1.0;
 }
 
 struct Dev {
@@ -181,21 +227,30 @@ extern "C" int cipsi_davidson(int32_t n, int64_t nel, const int32_t* itab, const
   long long* drow = nullptr;
   int32_t* dcol = nullptr;
   double *dval = nullptr, *ddiag = nullptr, *V = nullptr, *Wm = nullptr, *X = nullptr, *AX = nullptr, *T = nullptr,
-         *AT = nullptr, *dG = nullptr, *dS = nullptr, *dth = nullptr;
-  auto alloc = [&](void** p, size_t bytes, const char* what) { d.check(cudaMalloc(p, std::max<size_t>(bytes, 8)), what); };
-  alloc((void**)&drow, rowptr.size() * 8, "rowptr");
-  alloc((void**)&dcol, (size_t)nnz * 4, "col");
-  alloc((void**)&dval, (size_t)nnz * 8, "val");
-  alloc((void**)&ddiag, (size_t)n * 8, "diag");
-  alloc((void**)&V, (size_t)n * kmax * 8, "V");
-  alloc((void**)&Wm, (size_t)n * kmax * 8, "W");
-  alloc((void**)&X, (size_t)n * nb * 8, "X");
-  alloc((void**)&AX, (size_t)n * nb * 8, "AX");
-  alloc((void**)&T, (size_t)n * nb * 8, "T");
-  alloc((void**)&AT, (size_t)n * nb * 8, "AT");
-  alloc((void**)&dG, (size_t)kmax * kmax * 8, "G");
-  alloc((void**)&dS, (size_t)kmax * kmax * 8, "S");
-  alloc((void**)&dth, (size_t)kmax * 8, "theta");
+         *AT = nullptr, *dG = nullptr, *hG = nullptr;
+  // one allocation, cut into parts of whole 256 bytes
+  const size_t gsz = (size_t)kmax * kmax * 8;
+  unsigned char* mem = nullptr;
+  {
+    size_t off = 0;
+    struct Part {
+      void** p;
+      size_t bytes, at;
+    } part[] = {{(void**)&drow, rowptr.size() * 8, 0}, {(void**)&dcol, (size_t)nnz * 4, 0},
+                {(void**)&dval, (size_t)nnz * 8, 0},   {(void**)&ddiag, (size_t)n * 8, 0},
+                {(void**)&V, (size_t)n * kmax * 8, 0}, {(void**)&Wm, (size_t)n * kmax * 8, 0},
+                {(void**)&X, (size_t)n * nb * 8, 0},   {(void**)&AX, (size_t)n * nb * 8, 0},
+                {(void**)&T, (size_t)n * nb * 8, 0},   {(void**)&AT, (size_t)n * nb * 8, 0},
+                {(void**)&dG, 2 * gsz, 0}};
+    for (Part& q : part) {
+      q.at = off;
+      off += (q.bytes + 255) / 256 * 256;
+    }
+    d.check(cudaMalloc((void**)&mem, off), "cudaMalloc");
+    d.check(cudaMallocHost((void**)&hG, 2 * gsz), "cudaMallocHost");
+    if (d.ok)
+      for (Part& q : part) *q.p = mem + q.at;
+  }
   if (d.ok) {
     d.check(cudaMemcpyAsync(drow, rowptr.data(), rowptr.size() * 8, cudaMemcpyHostToDevice, st), "copy");
     d.check(cudaMemcpyAsync(dcol, col.data(), (size_t)nnz * 4, cudaMemcpyHostToDevice, st), "copy");
@@ -205,6 +260,8 @@ extern "C" int cipsi_davidson(int32_t n, int64_t nel, const int32_t* itab, const
   int sms = 0;
   d.check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "attr");
   const int ewgrid = std::max(1, std::min((n + 255) / 256, 8 * sms));
+  // columns side by side while the rows alone leave the device part empty
+  auto ew = [&](int kb) { return dim3((unsigned)ewgrid, ewgrid < 4 * sms ? (unsigned)kb : 1u); };
   const int spgrid = std::max(1, std::min((n * 32 + 255) / 256, 32 * sms));
   auto spmm = [&](const double* Xin, double* Yout, int nv) {
     for (int v0 = 0; v0 < nv && d.ok; v0 += kMaxBlock) {
@@ -220,19 +277,31 @@ extern "C" int cipsi_davidson(int32_t n, int64_t nel, const int32_t* itab, const
       d.check(cudaGetLastError(), "k_spmm");
     }
   };
-  auto gram = [&](const double* A, int ka, const double* B, int kb, std::vector<double>& G) {
-    G.assign((size_t)ka * kb, 0.0);
+  // A^T B into part `at` of the device's and the host's small matrices; the host
+  // may look after sync()
+  auto gram = [&](const double* A, int ka, const double* B, int kb, bool norms, bool host, int at) {
     if (!d.ok || ka == 0 || kb == 0) return;
-    k_gram<<<ka * kb, 256, 0, st>>>(n, A, n, ka, B, n, kb, dG);
+    const int m = norms ? ka : ka * kb;
+    double* g = dG + at * (gsz / 8);
+    k_gram<<<m, 256, 0, st>>>(n, A, n, B, n, kb, norms ? 1 : 0, g);
     d.check(cudaGetLastError(), "k_gram");
-    d.check(cudaMemcpyAsync(G.data(), dG, G.size() * 8, cudaMemcpyDeviceToHost, st), "copy G");
-    d.check(cudaStreamSynchronize(st), "sync");
+    if (host) d.check(cudaMemcpyAsync(hG + at * (gsz / 8), g, (size_t)m * 8, cudaMemcpyDeviceToHost, st), "copy G");
   };
-  auto combine = [&](const double* A, int ka, const std::vector<double>& S, int kb, double beta, double* Y) {
+  auto sync = [&]() {
+    if (d.ok) d.check(cudaStreamSynchronize(st), "sync");
+  };
+  Small sm;
+  auto combine = [&](const double* A, int ka, const double* S, int kb, double beta, double* Y, const double* D) {
     if (!d.ok || kb == 0) return;
-    d.check(cudaMemcpyAsync(dS, S.data(), S.size() * 8, cudaMemcpyHostToDevice, st), "copy S");
-    k_combine<<<ewgrid, 256, (size_t)ka * kb * 8, st>>>(n, A, n, ka, dS, kb, beta, Y, n);
+    if (S) std::memcpy(sm.s, S, (size_t)ka * kb * 8);
+    k_combine<<<ew(kb), 256, 0, st>>>(n, A, n, ka, sm, D, kb, beta, Y, n);
     d.check(cudaGetLastError(), "k_combine");
+  };
+  // T less its components along V; the coefficients stay on the device
+  auto project = [&](int k, int nt) {
+    if (k == 0) return;
+    gram(V, k, T, nt, false, false, 0);
+    combine(V, k, nullptr, nt, 1.0, T, dG);
   };
   // T (nt columns): remove the components along V (two passes), then make
   // the columns orthonormal through their Gram matrix, dropping directions
@@ -240,20 +309,15 @@ extern "C" int cipsi_davidson(int32_t n, int64_t nel, const int32_t* itab, const
   auto orthonormalise = [&](int k, int nt) -> int {
     // the scale of the corrections before projection: a direction is
     // dropped when projecting leaves less than 1e-10 of that scale
-    std::vector<double> G0;
-    gram(T, nt, T, nt, G0);
-    double scale2 = 0.0;
-    for (int q = 0; q < nt; ++q) scale2 = std::max(scale2, G0[(size_t)q * nt + q]);
-    for (int pass = 0; pass < 2 && k > 0; ++pass) {
-      std::vector<double> C;
-      gram(V, k, T, nt, C);  // k x nt
-      for (auto& x : C) x = -x;
-      combine(V, k, C, nt, 1.0, T);
-    }
-    std::vector<double> G, w, U;
-    gram(T, nt, T, nt, G);
+    gram(T, nt, T, nt, true, true, 1);
+    for (int pass = 0; pass < 2; ++pass) project(k, nt);
+    gram(T, nt, T, nt, false, true, 0);
+    sync();
     if (!d.ok) return 0;
-    sym_eig(nt, G, w, U);
+    double scale2 = 0.0;
+    for (int q = 0; q < nt; ++q) scale2 = std::max(scale2, hG[gsz / 8 + q]);
+    std::vector<double> w, U;
+    sym_eig(nt, std::vector<double>(hG, hG + nt * nt), w, U);
     std::vector<int> keep;
     for (int q = nt - 1; q >= 0; --q)
       if (w[q] > 1e-20 * scale2 && w[q] > 0.0) keep.push_back(q);
@@ -262,22 +326,20 @@ extern "C" int cipsi_davidson(int32_t n, int64_t nel, const int32_t* itab, const
     std::vector<double> Sx((size_t)nt * nk);
     for (int c = 0; c < nk; ++c)
       for (int r = 0; r < nt; ++r) Sx[(size_t)r * nk + c] = U[(size_t)r * nt + keep[c]] / std::sqrt(w[keep[c]]);
-    combine(T, nt, Sx, nk, 0.0, AT);  // AT as scratch for the new columns
-    d.check(cudaMemcpyAsync(T, AT, (size_t)n * nk * 8, cudaMemcpyDeviceToDevice, st), "copy T");
+    combine(T, nt, Sx.data(), nk, 0.0, AT, nullptr);
+    std::swap(T, AT);
     // once more against V: the Gram step can bring back rounding-level overlap
     if (k > 0) {
-      std::vector<double> C;
-      gram(V, k, T, nk, C);
-      for (auto& x : C) x = -x;
-      combine(V, k, C, nk, 1.0, T);
-      gram(T, nk, T, nk, G);
+      project(k, nk);
+      gram(T, nk, T, nk, false, true, 0);
+      sync();
       if (!d.ok) return 0;
-      sym_eig(nk, G, w, U);
+      sym_eig(nk, std::vector<double>(hG, hG + nk * nk), w, U);
       std::vector<double> S2((size_t)nk * nk);
       for (int c = 0; c < nk; ++c)
         for (int r = 0; r < nk; ++r) S2[(size_t)r * nk + c] = U[(size_t)r * nk + c] / std::sqrt(std::max(w[c], 1e-300));
-      combine(T, nk, S2, nk, 0.0, AT);
-      d.check(cudaMemcpyAsync(T, AT, (size_t)n * nk * 8, cudaMemcpyDeviceToDevice, st), "copy T");
+      combine(T, nk, S2.data(), nk, 0.0, AT, nullptr);
+      std::swap(T, AT);
     }
     return nk;
   };
@@ -286,18 +348,24 @@ extern "C" int cipsi_davidson(int32_t n, int64_t nel, const int32_t* itab, const
     std::vector<int> ord(n);
     for (int i = 0; i < n; ++i) ord[i] = i;
     std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return diag[a] < diag[b]; });
-    std::vector<double> v0((size_t)n * nb, 0.0);
-    for (int b = 0; b < nb; ++b) v0[(size_t)b * n + ord[b]] = 1.0;
-    if (d.ok) d.check(cudaMemcpyAsync(V, v0.data(), v0.size() * 8, cudaMemcpyHostToDevice, st), "copy V0");
+    Theta u{};
+    for (int b = 0; b < nb; ++b) u.from[b] = ord[b];
+    if (d.ok) {
+      d.check(cudaMemsetAsync(V, 0, (size_t)n * nb * 8, st), "clear V0");
+      k_units<<<1, 32, 0, st>>>(n, u, nb, V);
+      d.check(cudaGetLastError(), "k_units");
+    }
     spmm(V, Wm, nb);
   }
   int k = nb, it = 0;
   std::vector<double> theta, Sm, res(nroots, 0.0);
   bool converged = false;
   for (it = 1; it <= std::max(1, maxiter) && d.ok; ++it) {
-    std::vector<double> Hs, w, U;
-    gram(V, k, Wm, k, Hs);
+    std::vector<double> w, U;
+    gram(V, k, Wm, k, false, true, 0);
+    sync();
     if (!d.ok) break;
+    std::vector<double> Hs(hG, hG + (size_t)k * k);
     for (int a = 0; a < k; ++a)  // symmetrise (rounding)
       for (int b = a + 1; b < k; ++b) Hs[(size_t)a * k + b] = Hs[(size_t)b * k + a] = 0.5 * (Hs[(size_t)a * k + b] + Hs[(size_t)b * k + a]);
     sym_eig(k, Hs, w, U);
@@ -306,21 +374,21 @@ extern "C" int cipsi_davidson(int32_t n, int64_t nel, const int32_t* itab, const
     for (int a = 0; a < k; ++a)
       for (int b = 0; b < nx; ++b) Sm[(size_t)a * nx + b] = U[(size_t)a * k + b];
     theta.assign(w.begin(), w.begin() + nx);
-    combine(V, k, Sm, nx, 0.0, X);
-    combine(Wm, k, Sm, nx, 0.0, AX);
+    combine(V, k, Sm.data(), nx, 0.0, X, nullptr);
+    combine(Wm, k, Sm.data(), nx, 0.0, AX, nullptr);
     // residuals R = AX - X theta (into T)
-    d.check(cudaMemcpyAsync(T, AX, (size_t)n * nx * 8, cudaMemcpyDeviceToDevice, st), "copy R");
-    {
-      std::vector<double> D((size_t)nx * nx, 0.0);
-      for (int b = 0; b < nx; ++b) D[(size_t)b * nx + b] = -theta[b];
-      combine(X, nx, D, nx, 1.0, T);
+    Theta th{};
+    for (int b = 0; b < nx; ++b) th.theta[b] = theta[b];
+    if (d.ok) {
+      k_residual<<<ew(nx), 256, 0, st>>>(n, AX, X, th, nx, T);
+      d.check(cudaGetLastError(), "k_residual");
     }
-    std::vector<double> RR;
-    gram(T, nx, T, nx, RR);
+    gram(T, nx, T, nx, true, true, 0);
+    sync();
     if (!d.ok) break;
     double worst = 0.0;
     for (int b = 0; b < nroots; ++b) {
-      res[b] = std::sqrt(std::max(RR[(size_t)b * nx + b], 0.0));
+      res[b] = std::sqrt(std::max(hG[b], 0.0));
       worst = std::max(worst, res[b]);
     }
     if (worst <= tol) {
@@ -339,17 +407,13 @@ extern "C" int cipsi_davidson(int32_t n, int64_t nel, const int32_t* itab, const
     for (int b = 0; b < nx; ++b)
       if (b >= nroots || res[b] > tol) todo.push_back(b);
     const int nu = (int)todo.size();
-    {
-      std::vector<double> sel((size_t)nx * nu, 0.0), th(nu);
-      for (int c = 0; c < nu; ++c) {
-        sel[(size_t)todo[c] * nu + c] = 1.0;
-        th[c] = theta[todo[c]];
-      }
-      combine(T, nx, sel, nu, 0.0, AT);
-      d.check(cudaMemcpyAsync(dth, th.data(), nu * 8, cudaMemcpyHostToDevice, st), "theta");
-      k_precond<<<ewgrid, 256, 0, st>>>(n, AT, n, ddiag, dth, nu, T, n);
-      d.check(cudaGetLastError(), "k_precond");
+    for (int c = 0; c < nu; ++c) {
+      th.from[c] = todo[c];
+      th.theta[c] = theta[todo[c]];
     }
+    k_precond<<<ew(nu), 256, 0, st>>>(n, T, ddiag, th, nu, AT);
+    d.check(cudaGetLastError(), "k_precond");
+    std::swap(T, AT);
     const int nt = std::min(orthonormalise(k, nu), kmax - k);
     if (nt <= 0) break;  // the space is exhausted (n small)
     d.check(cudaMemcpyAsync(V + (size_t)k * n, T, (size_t)n * nt * 8, cudaMemcpyDeviceToDevice, st), "append V");
@@ -361,9 +425,8 @@ extern "C" int cipsi_davidson(int32_t n, int64_t nel, const int32_t* itab, const
     d.check(cudaMemcpyAsync(xo.data(), X, (size_t)n * std::min(nb, k) * 8, cudaMemcpyDeviceToHost, st), "copy X");
     d.check(cudaStreamSynchronize(st), "sync");
   }
-  for (void* p : {(void*)drow, (void*)dcol, (void*)dval, (void*)ddiag, (void*)V, (void*)Wm, (void*)X, (void*)AX,
-                  (void*)T, (void*)AT, (void*)dG, (void*)dS, (void*)dth})
-    if (p) cudaFree(p);
+  if (mem) cudaFree(mem);
+  if (hG) cudaFreeHost(hG);
   if (st) cudaStreamDestroy(st);
   if (!d.ok) {
     seterr(errbuf, errlen, "cipsi_davidson: " + d.err);
