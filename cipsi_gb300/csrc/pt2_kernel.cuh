@@ -1085,8 +1085,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
       }
       // dE/dhdig, dE/dhmp of a row's candidates, by lane: a shared FP64 atomic is
       // a compare-and-swap loop, and a row's lanes would all take it on one
-      // address (30 orbitals, S = 301: 2.95 -> 2.64 ms for
-      // the kernel, with the tail below spread over the threads)
+      // address (30 orbitals, S = 301: 2.95 -> 2.64 ms for the kernel, with the
+      // K' terms below spread over the threads)
       double row_gh = 0.0, row_gm = 0.0;
       // One candidate I = K' + {a1[, a2]}: rank-change class, symmetry and
       // spin-pattern rules, then a scan of L_R entries [0, nscan) plus the
