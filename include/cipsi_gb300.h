@@ -87,16 +87,17 @@ typedef struct {
   double tabvp[CIPSI_NCLASS * CIPSI_MAX_ROOTS];    /* tabvp(class, root)     */
   /* work counters (not in the reference; for throughput and roofline)      */
   int64_t n_candidates;   /* excitations examined                           */
-  int64_t n_compares;     /* candidate-vs-S determinant comparisons          */
+  int64_t n_compares;     /* comparisons of entries of S with candidates or  */
+                          /* rows of candidates                              */
   int64_t n_pairs_1;      /* interacting (I,K) pairs differing by 1 spin orb */
   int64_t n_pairs_2;      /* interacting (I,K) pairs differing by 2          */
   int64_t alg_bytes;      /* algorithmic bytes (integrals, coefficients,     */
                           /* diagonal terms) read by the E2 loop             */
   double kernel_ms;       /* device time of the perturbation kernels         */
-  double pt2_ms;          /* of which the perturbation kernel itself (k_pt2, */
-                          /* summed over its launches)                        */
-  int64_t launches;       /* kernel launches of the run (k_pt2, record scan  */
-                          /* and gather per chunk, final reduction)           */
+  double pt2_ms;          /* of which the two perturbation kernels (k_cand,  */
+                          /* k_pt2, summed over their launches)               */
+  int64_t launches;       /* kernel launches of the run (k_cand, k_pt2,      */
+                          /* record scan and gather per chunk, k_finish)      */
 } cipsi_result;
 
 /* Create a context on CUDA device `device`.
@@ -156,11 +157,10 @@ int cipsi_run_pt2(cipsi_ctx* ctx, const cipsi_opts* opts, cipsi_result* res);
 /* Launch shape of later runs on this context (no counterpart in the
    reference; results do not depend on it beyond summation order):
      r_chunk      removed-electron blocks per work unit for generators of
-                  excitation rank >= 2 (rank 0 and 1 generators always get
-                  one block per unit); default 6
-     ctas_per_sm  0 or 2 = shared-memory list sized so that two CTAs fit
-                  per SM (the rest of a longer list is read from global
-                  memory), 1 = one CTA per SM with a 200 KB list
+                  excitation rank >= 2: up to 8/3 of it, fewer in small runs;
+                  below 6, that number (rank 0 always gets one block per
+                  unit, rank 1 at most 8); default 6
+     ctas_per_sm  0 or 2 = two CTAs per SM where shared memory allows, 1 = one
    cipsi_gb300.tune (Python) picks both by timing a generator sample. */
 int cipsi_set_tuning(cipsi_ctx* ctx, int32_t r_chunk, int32_t ctas_per_sm);
 
