@@ -684,7 +684,8 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
         const int t = lane < take ? (int)wm.hits[lane] : -1;
         const uint32_t later = wm.hits[32 + lane];
         __syncwarp();
-        wm.hits[lane] = later;
+        wm.hits[lane] = later;  // (by every lane, whatever is left: before the next lot's stores)
+        __syncwarp();
         nc -= take;
         const bool owner = t < nown;  // (or no entry)
         uint3 en = make_uint3(0u, 0u, 9u << 16);
@@ -792,7 +793,7 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
           }
           nvalid += (unsigned)__popcll(x);
           uint64_t o = (uint64_t)wm.owncol[sc][2 * w] | (uint64_t)wm.owncol[sc][2 * w + 1] << 32;
-          if (two) o |= (uint64_t)wm.own[rw][2 * w] | (uint64_t)wm.own[rw][2 * w + 1] << 32;
+          if (two && on) o |= (uint64_t)wm.own[rw][2 * w] | (uint64_t)wm.own[rw][2 * w + 1] << 32;
           x = drow ? 0ull : x & ~o;
           if (on) {
             wm.own[rw][2 * w] = (uint32_t)x;
@@ -818,6 +819,7 @@ __global__ void __launch_bounds__(kThreads, kCandCtas<W, R>) k_cand(Params p0, L
     // the next rows of the block: surviving candidates (cols[0..nal)), the
     // other determinants' elements (xb, xf), the constants of <I|H|k>
     auto open_rows = [&]() {
+      __syncwarp();  // the last rows' tables have been read by every lane
       nal = pos = 0;
       hasx = false;
       // as many rows as their candidates fit (one always does): what is done
