@@ -394,6 +394,30 @@ void dfree(T*& p) {
   p = nullptr;
 }
 
+int roots_pad(int mt) { return mt <= 1 ? 1 : mt <= 2 ? 2 : mt <= 4 ? 4 : 8; }
+
+// the forward form of k_pt2_one of class (W, R)
+cudaError_t launch_one(int W, int R, const Params& p, int grid, size_t smem, cudaStream_t st) {
+  if (W == 1)
+    return R == 1 ? launch_pt2_one<1, 1, false>(p, grid, smem, st)
+         : R == 2 ? launch_pt2_one<1, 2, false>(p, grid, smem, st)
+         : R == 4 ? launch_pt2_one<1, 4, false>(p, grid, smem, st)
+                  : launch_pt2_one<1, 8, false>(p, grid, smem, st);
+  return R == 1 ? launch_pt2_one<2, 1, false>(p, grid, smem, st)
+       : R == 2 ? launch_pt2_one<2, 2, false>(p, grid, smem, st)
+       : R == 4 ? launch_pt2_one<2, 4, false>(p, grid, smem, st)
+                : launch_pt2_one<2, 8, false>(p, grid, smem, st);
+}
+
+// The code and the local memory that cipsi_run_pt2_static's kernels take on the
+// device, which the runtime allocates at their first launch: a context has them
+// from its creation on, so that the call itself allocates nothing.
+cudaError_t load_static(int W, int R, cudaStream_t st) {
+  cudaFuncAttributes at;
+  const cudaError_t e = cudaFuncGetAttributes(&at, k_reduce);
+  return e != cudaSuccess ? e : launch_one(W, R, Params{}, 1, 0, st);  // no units: it returns at once
+}
+
 }  // namespace
 
 extern "C" {
@@ -437,6 +461,7 @@ int cipsi_ctx_create(cipsi_ctx** out, const cipsi_dims* dims, int32_t device) {
   CK(cudaEventCreate(&ctx->ev0));
   CK(cudaEventCreate(&ctx->ev1));
   CK(cudaEventCreate(&ctx->evk));
+  CK(load_static(ctx->W, roots_pad(d.metat), ctx->stream));
   return CIPSI_OK;
 }
 
@@ -700,8 +725,6 @@ int cipsi_set_roots(cipsi_ctx* ctx, const double* c, const double* e, const doub
 
 namespace {
 
-int roots_pad(int mt) { return mt <= 1 ? 1 : mt <= 2 ? 2 : mt <= 4 ? 4 : 8; }
-
 int check_run_args(cipsi_ctx* ctx, const cipsi_opts* o) {
   if (!ctx || !o) return CIPSI_ERR_ARG;
   if (!ctx->have_int || !ctx->have_space || !ctx->have_roots)
@@ -925,24 +948,35 @@ std::vector<int> cut_units(const std::vector<long long>& slots, long long cap, s
   return cut;
 }
 
-// The adjoint kernel's shared-memory L_R capacity, dynamic shared memory and
-// CTAs per SM.  ctas: 1 = one CTA per SM with a long list, else two: the part
-// of a longer list is read from the block's global scratch, 8 bytes per
-// entry, which costs less than halving the resident warps (82 + 32 KB of
-// static shared memory fit an SM twice).
+// k_pt2_one's shared-memory L_R capacity, dynamic shared memory and CTAs per
+// SM.  ctas: 1 = one CTA per SM with a long list, else two: the part of a longer
+// list is read from the block's global scratch, 8 bytes per entry, which costs
+// less than halving the resident warps.  `total` and one CTA's static shared
+// memory (up to 32 KB) fit an SM twice; `queues` of it are not the list's.
 struct LaunchShape {
   int lr_cap;
   size_t smem;
   int blocks_per_sm;
 };
-LaunchShape adj_shape(int ncf_max, int ctas) {
+LaunchShape list_shape(int ncf_max, size_t total, size_t queues, int blocks) {
   const size_t per_entry = 8;  // compact L_R entry
-  const size_t smem_budget = (ctas == 1 ? (size_t)188 * 1024 : (size_t)78 * 1024) - 16;
   LaunchShape ls;
-  ls.lr_cap = (int)std::min<size_t>((size_t)ncf_max, smem_budget / per_entry);
-  ls.smem = (((size_t)ls.lr_cap * per_entry + 15) & ~(size_t)15) + 16;
-  ls.blocks_per_sm = ctas == 1 ? 1 : 2;
+  ls.lr_cap = (int)std::min<size_t>((size_t)ncf_max, (total - queues - 16) / per_entry);
+  ls.smem = (((size_t)ls.lr_cap * per_entry + 15) & ~(size_t)15) + queues + 16;
+  ls.blocks_per_sm = blocks;
   return ls;
+}
+// the adjoint form, which has no queues and 4 KB more of static sums
+LaunchShape adj_shape(int ncf_max, int ctas) {
+  return list_shape(ncf_max, (size_t)(ctas == 1 ? 188 : 78) * 1024, 0, ctas == 1 ? 1 : 2);
+}
+// the forward form, with its warps' epilogue queues
+LaunchShape one_shape(int R, int ncf_max) {
+  const size_t q = R == 1   ? sizeof(WarpQueue<1>)
+                   : R == 2 ? sizeof(WarpQueue<2>)
+                   : R == 4 ? sizeof(WarpQueue<4>)
+                            : sizeof(WarpQueue<8>);
+  return list_shape(ncf_max, (size_t)82 * 1024, kWarps * q, 2);
 }
 
 // The record pool (unit segments), for `cap` records.
@@ -1874,17 +1908,17 @@ int run_adjoint(cipsi_ctx* ctx, const cipsi_opts* o, const double* seed, double*
   if (nunits > 0) {
     cudaError_t e;
     if (W == 1) {
-      e = R == 1 ? launch_pt2_adj<1, 1>(p, grid, ls.smem, ctx->stream)
-        : R == 2 ? launch_pt2_adj<1, 2>(p, grid, ls.smem, ctx->stream)
-        : R == 4 ? launch_pt2_adj<1, 4>(p, grid, ls.smem, ctx->stream)
-                 : launch_pt2_adj<1, 8>(p, grid, ls.smem, ctx->stream);
+      e = R == 1 ? launch_pt2_one<1, 1, true>(p, grid, ls.smem, ctx->stream)
+        : R == 2 ? launch_pt2_one<1, 2, true>(p, grid, ls.smem, ctx->stream)
+        : R == 4 ? launch_pt2_one<1, 4, true>(p, grid, ls.smem, ctx->stream)
+                 : launch_pt2_one<1, 8, true>(p, grid, ls.smem, ctx->stream);
     } else {
-      e = R == 1 ? launch_pt2_adj<2, 1>(p, grid, ls.smem, ctx->stream)
-        : R == 2 ? launch_pt2_adj<2, 2>(p, grid, ls.smem, ctx->stream)
-        : R == 4 ? launch_pt2_adj<2, 4>(p, grid, ls.smem, ctx->stream)
-                 : launch_pt2_adj<2, 8>(p, grid, ls.smem, ctx->stream);
+      e = R == 1 ? launch_pt2_one<2, 1, true>(p, grid, ls.smem, ctx->stream)
+        : R == 2 ? launch_pt2_one<2, 2, true>(p, grid, ls.smem, ctx->stream)
+        : R == 4 ? launch_pt2_one<2, 4, true>(p, grid, ls.smem, ctx->stream)
+                 : launch_pt2_one<2, 8, true>(p, grid, ls.smem, ctx->stream);
     }
-    if ((rc = ck(e, "k_pt2_adj launch"))) return rc;
+    if ((rc = ck(e, "adjoint k_pt2_one launch"))) return rc;
     k_reduce<<<(unsigned)nq, kReduceThreads, 0, ctx->stream>>>(ctx->dgen_part, nunits, (int)nq, ctx->dred);
   } else {
     if ((rc = ck(cudaMemsetAsync(ctx->dred, 0, nq * sizeof(double), ctx->stream), "memset"))) return rc;
@@ -2321,14 +2355,16 @@ void cipsi_batch_destroy(cipsi_batch* b) {
 }
 
 // ------------------------------------------------- run without allocation
-// cipsi_run_pt2_static runs k_cand, k_pt2 and k_finish with every per-run buffer taken
-// from file-scope device arrays instead of cudaMalloc'd context buffers: what
-// the kernel accumulates into (kZeroWords), and a scratch array (each region
-// 256-byte aligned): histogram sums | reduced sums | generator list |
-// generator masks | work units | per-block neighbour scratch (nb_j, nb_emask,
-// lr_ent).  The size limit is that of the entry's first form, which also kept
-// counters and five sums per work unit and root in the array: the room for
-// them stays reserved, so that what fits and what does not is unchanged.  The generator and
+// cipsi_run_pt2_static runs k_pt2_one + k_reduce with every per-run buffer taken
+// from one file-scope device array instead of cudaMalloc'd context buffers.
+// The two forward kernels do not fit it: their candidate buffer wants gigabytes
+// (through 128 MB, in parts that left most of the device idle, this entry took
+// 49, 409 and 574 ms at 60, 100 and 124 orbitals, S = 1001, 2001 and 2501; one
+// kernel takes 36, 212 and 249).
+// Layout of the array (each region 256-byte aligned): counters + dpivot +
+// histogram counts | histogram sums | reduced sums | work counter |
+// generator list | generator masks | work units | per-unit partial sums |
+// per-block neighbour scratch (nb_j, nb_emask, lr_ent).  The generator and
 // unit lists are staged in file-scope host arrays of fixed size.
 
 }  // extern "C"
@@ -2336,26 +2372,19 @@ void cipsi_batch_destroy(cipsi_batch* b) {
 namespace {
 
 constexpr size_t kStaticScratchBytes = (size_t)32 << 20;  // 32 MiB
-constexpr size_t kStaticCandBytes = (size_t)128 << 20;  // candidate buffer
 constexpr int kStaticMaxUnits = 1 << 18;
 constexpr int kStaticMaxGens = 1 << 17;
 constexpr int kStaticMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_pt2_scratch[kStaticScratchBytes];
-static __device__ __align__(256) unsigned long long g_pt2_zeroed[kZeroWords];
-static __device__ __align__(256) unsigned char g_pt2_cand[kStaticCandBytes];
 
 // host staging of the generator and unit lists (copied to the device array)
 static int32_t g_static_gens[kStaticMaxGens];
 static uint8_t g_static_gmask[kStaticMaxGens];
 static int32_t g_static_units[3 * kStaticMaxUnits];
-static int32_t g_static_nslots[kStaticMaxUnits];
-static long long g_static_slot[kStaticMaxUnits];
 
-// device addresses of the arrays, looked up once per device
+// device address of g_pt2_scratch, looked up once per device
 static unsigned char* g_static_ptr[kStaticMaxDevices];
-static unsigned long long* g_static_zeroed[kStaticMaxDevices];
-static unsigned char* g_static_cand[kStaticMaxDevices];
 static bool g_static_ready[kStaticMaxDevices];
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -2382,10 +2411,6 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
     void* ptr = nullptr;
     CK(cudaGetSymbolAddress(&ptr, g_pt2_scratch));
     g_static_ptr[ctx->device] = static_cast<unsigned char*>(ptr);
-    CK(cudaGetSymbolAddress(&ptr, g_pt2_zeroed));
-    g_static_zeroed[ctx->device] = static_cast<unsigned long long*>(ptr);
-    CK(cudaGetSymbolAddress(&ptr, g_pt2_cand));
-    g_static_cand[ctx->device] = static_cast<unsigned char*>(ptr);
     g_static_ready[ctx->device] = true;
   }
   unsigned char* base = g_static_ptr[ctx->device];
@@ -2444,12 +2469,11 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   int32_t* ug = g_static_units;
   int32_t* ur0 = g_static_units + kStaticMaxUnits;
   int32_t* ur1 = g_static_units + 2 * kStaticMaxUnits;
-  auto push_unit = [&](int g, int a, int b, long long slots) {
+  auto push_unit = [&](int g, int a, int b) {
     if (nunits == kStaticMaxUnits) return false;
     ug[nunits] = g;
     ur0[nunits] = a;
     ur1[nunits] = b;
-    g_static_nslots[nunits] = (int32_t)slots;
     ++nunits;
     return true;
   };
@@ -2457,7 +2481,7 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
     return fail(ctx, CIPSI_ERR_OVERFLOW,
                 "cipsi_run_pt2_static: more than " + std::to_string(kStaticMaxUnits) + " work units");
   };
-  int hfe[2 * 128], spe[2 * 128];
+  int hfe[2 * 128];
   for (int rk = -1; rk <= maxrank; ++rk) {
     for (int g = 0; g < ngen; ++g) {
       const int k = g_static_gens[g];
@@ -2465,23 +2489,18 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
       if (k < 0) {
         const int ntot = (pertu_ref ? 1 : 0) + (pertu_mono ? 2 * noca * (n - noca) : 0);
         for (int t = 0; t < ntot; t += kPertuChunk)
-          if (!push_unit(g, t, std::min(ntot, t + kPertuChunk), std::min(ntot - t, kPertuChunk))) return too_many_units();
+          if (!push_unit(g, t, std::min(ntot, t + kPertuChunk))) return too_many_units();
         continue;
       }
-      int ne = 0, nes[2] = {0, 0};
+      int ne = 0;
       for (int sp = 0; sp < 2; ++sp)
         for (int orb = 0; orb < n; ++orb)
-          if ((ctx->Sbits[(size_t)k * 2 * W + sp * W + (orb >> 6)] >> (orb & 63)) & 1ull) {
-            spe[ne] = sp;
+          if ((ctx->Sbits[(size_t)k * 2 * W + sp * W + (orb >> 6)] >> (orb & 63)) & 1ull)
             hfe[ne++] = orb < noca;
-            ++nes[sp];
-          }
-      const int nv[2] = {n - nes[0], n - nes[1]};
       const uint8_t m = g_static_gmask[g];
       int cnt = 0, start = -1;
-      long long slots = 0;
       for (int rb = 0; rb < nR; ++rb) {
-        int hfR, nRr, x1 = rb, x2 = -1;
+        int hfR, nRr;
         if (rb < nel) {
           hfR = hfe[rb];
           nRr = 1;
@@ -2491,9 +2510,7 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
             t -= nel - 1 - e1;
             ++e1;
           }
-          x1 = e1;
-          x2 = e1 + 1 + t;
-          hfR = hfe[x1] + hfe[x2];
+          hfR = hfe[e1] + hfe[e1 + 1 + t];
           nRr = 2;
         }
         bool ok = false;
@@ -2501,15 +2518,13 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
           if (m & (1u << (hfR + aV - nRr + 2))) ok = true;
         if (!ok) continue;
         if (start < 0) start = rb;
-        slots += block_candidates(nRr, x2 >= 0 && spe[x1] == spe[x2], nv[spe[x1]], nv[0], nv[1]);
         if (++cnt == kRChunk) {
-          if (!push_unit(g, start, rb + 1, slots)) return too_many_units();
+          if (!push_unit(g, start, rb + 1)) return too_many_units();
           cnt = 0;
           start = -1;
-          slots = 0;
         }
       }
-      if (start >= 0 && !push_unit(g, start, nR, slots)) return too_many_units();
+      if (start >= 0 && !push_unit(g, start, nR)) return too_many_units();
     }
   }
 
@@ -2518,9 +2533,12 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   int dev_sms = 0;
   CK(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device));
   const int R = mt <= 1 ? 1 : mt <= 2 ? 2 : mt <= 4 ? 4 : 8;
-  const int blocks_per_sm = fwd_blocks_per_sm(W, R, 0);
+  const LaunchShape ls = one_shape(R, ncf);
+  const int lr_cap = ls.lr_cap;
+  const size_t smem = ls.smem;
+  const int blocks_per_sm = ls.blocks_per_sm;
   const size_t nq = (size_t)5 * mt;
-  const size_t ncount = kCountWords;
+  const size_t ncount = C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots;
   const size_t off_counters = 0;
   const size_t off_tab = align256(off_counters + ncount * sizeof(unsigned long long));
   const size_t off_red = align256(off_tab + 2 * kNClass * kMaxRoots * sizeof(double));
@@ -2543,31 +2561,15 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   unsigned char* nb0 = base + off_nb;
 
   // zero what the kernels accumulate into; upload the lists
-  unsigned long long* zeroed = g_static_zeroed[ctx->device];
-  CK(cudaMemsetAsync(zeroed, 0, kZeroWords * sizeof(unsigned long long), ctx->stream));
+  CK(cudaMemsetAsync(base, 0, off_gens, ctx->stream));
+  CK(cudaMemsetAsync(base + off_part, 0, (size_t)std::max(nunits, 1) * nq * sizeof(double), ctx->stream));
   if (ngen) {
     CK(cudaMemcpyAsync(base + off_gens, g_static_gens, (size_t)ngen * sizeof(int32_t),
                        cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(base + off_gmask, g_static_gmask, (size_t)ngen, cudaMemcpyHostToDevice, ctx->stream));
   }
   int32_t* dunits = reinterpret_cast<int32_t*>(base + off_units);
-  // units in parts that fit the candidate buffer (a unit has at most 6 * 16,256
-  // slots, a few per cent of it); their slots take 12 of the >= 40 bytes per
-  // unit reserved at off_part
-  const long long cand_cap = (long long)(kStaticCandBytes / cand_slot_bytes(R)) / 64 * 64;
-  {
-    long long acc = 0;
-    for (int u = 0; u < nunits; ++u) {
-      if (acc + g_static_nslots[u] > cand_cap) acc = 0;
-      g_static_slot[u] = acc;
-      acc += g_static_nslots[u];
-    }
-  }
-  long long* dslot = reinterpret_cast<long long*>(base + off_part);
-  int32_t* dnslots = reinterpret_cast<int32_t*>(dslot + nunits);
   if (nunits) {
-    CK(cudaMemcpyAsync(dslot, g_static_slot, (size_t)nunits * 8, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(dnslots, g_static_nslots, (size_t)nunits * 4, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(dunits, ug, (size_t)nunits * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(dunits + nunits, ur0, (size_t)nunits * sizeof(int32_t), cudaMemcpyHostToDevice,
                        ctx->stream));
@@ -2602,7 +2604,6 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   p.F = ctx->dF;
   p.J = ctx->dJ;
   p.K = ctx->dK;
-  p.jx = ctx->djx;
   p.fmpb = ctx->dfmpb;
   p.orbsym = ctx->dorbsym;
   for (int i = 0; i < ctx->d.nsym; ++i)
@@ -2625,53 +2626,35 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   for (int i = 0; i < kNClass; ++i) {
     p.aval[i] = o->aval[i];
     std::memcpy(&p.aval_bits[i], &o->aval[i], 8);
-    p.aval_hi[i] = i + 1 < o->nclass ? (int)(p.aval_bits[i] >> 32) : 0x7fffffff;
   }
   p.pertu_ref = pertu_ref ? 1 : 0;
   p.pertu_mono = pertu_mono ? 1 : 0;
-  // nb_j and lr_e (4 bytes), nb_emask and lr_jh (8 bytes): grid x ncf entries
-  // each (k_pt2 indexes block b at b * ncf), in three regions of
-  // grid * nb_stride >= grid * ncf * 8 bytes; what is left holds the warps'
-  // overflow lists (12 bytes an entry; without them a long list is worked by
-  // the whole CTA)
-  const size_t region = (size_t)grid * nb_stride;
+  // nb_j, nb_emask, lr_ent: grid x ncf entries each (k_pt2 indexes block b at
+  // b * ncf), in three regions of grid * nb_stride >= grid * ncf * 8 bytes
   p.nb_j = reinterpret_cast<int32_t*>(nb0);
-  p.lr_e = reinterpret_cast<uint32_t*>(nb0 + region / 2);
-  p.nb_emask = reinterpret_cast<uint64_t*>(nb0 + region);
-  p.lr_jh = reinterpret_cast<uint2*>(nb0 + 2 * region);
-  const size_t lists = (size_t)grid * kWarps * 2;
-  const size_t left = kStaticScratchBytes - off_nb - 3 * region;
-  p.lrw_cap = (int)std::min<size_t>(left / (lists * 12), (size_t)lrw_entries(ncf));
-  p.lrw_jh = reinterpret_cast<uint2*>(nb0 + 3 * region);
-  p.lrw_e = reinterpret_cast<uint32_t*>(p.lrw_jh + lists * p.lrw_cap);
+  p.nb_emask = reinterpret_cast<uint64_t*>(nb0 + (size_t)grid * nb_stride);
+  p.lr_ent = reinterpret_cast<uint64_t*>(nb0 + (size_t)2 * grid * nb_stride);
+  p.lr_cap = lr_cap;
   p.nb_stride = ncf;
-  set_zeroed(p, zeroed);
+  p.gen_part = reinterpret_cast<double*>(base + off_part);
+  unsigned long long* dcounters = reinterpret_cast<unsigned long long*>(base + off_counters);
+  p.counters = dcounters;
+  p.dpivot_bits = dcounters + C_NCOUNTERS;
+  p.hist_nom = dcounters + C_NCOUNTERS + 1;
+  p.hist_nam = dcounters + C_NCOUNTERS + 1 + kNClass;
   p.hist_tab = reinterpret_cast<double*>(base + off_tab);
   // no record storage: selected perturbers are counted only
   p.rec_mode = 0;
+  p.work = reinterpret_cast<int*>(base + off_work);
   double* dred = reinterpret_cast<double*>(base + off_red);
-  p.red = dred;
 
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
-  int parts = 0;
-  for (int u0 = 0; u0 < nunits; ++parts) {
-    int u1 = u0 + 1;
-    while (u1 < nunits && g_static_slot[u1] != 0) ++u1;
-    if (u0) CK(cudaMemsetAsync(p.work, 0, 2 * sizeof(int), ctx->stream));
-    LaunchArgs la{};
-    la.unit_slot = dslot + u0;
-    la.unit_nslots = dnslots + u0;
-    la.cand = cand_views(g_static_cand[ctx->device], cand_cap, R);
-    la.nunits = u1 - u0;
-    la.work = p.work;
-    const cudaError_t e = launch_forward<false>(part_params(p, u0), la, W, R, std::min(grid, u1 - u0), dev_sms,
-                                                g_static_slot[u1 - 1] + g_static_nslots[u1 - 1], ctx->stream);
-    if (e != cudaSuccess)
-      return fail(ctx, CIPSI_ERR_CUDA, std::string("k_cand / k_pt2 launch: ") + cudaGetErrorString(e));
-    u0 = u1;
+  if (nunits > 0) {
+    const cudaError_t e = launch_one(W, R, p, grid, smem, ctx->stream);
+    if (e != cudaSuccess) return fail(ctx, CIPSI_ERR_CUDA, std::string("k_pt2_one launch: ") + cudaGetErrorString(e));
+    k_reduce<<<(unsigned)nq, kReduceThreads, 0, ctx->stream>>>(p.gen_part, nunits, (int)nq, dred);
+    CK(cudaGetLastError());
   }
-  k_finish<<<1, kFinishThreads, 0, ctx->stream>>>(p, nullptr);
-  CK(cudaGetLastError());
   CK(cudaEventRecord(ctx->ev1, ctx->stream));
 
   // results (same fields as cipsi_fetch_result; no records are kept), read
@@ -2681,7 +2664,7 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   unsigned long long cnt[C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots];
   double tab[2 * kNClass * kMaxRoots];
   CK(cudaMemcpyAsync(red, dred, nq * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(cnt, zeroed, ncount * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaMemcpyAsync(cnt, dcounters, ncount * sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaMemcpyAsync(tab, p.hist_tab, 2 * kNClass * kMaxRoots * sizeof(double), cudaMemcpyDeviceToHost,
                      ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -2721,7 +2704,7 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
   r->kernel_ms = ms;
   r->pt2_ms = ms;
-  r->launches = 2ll * parts + 1;
+  r->launches = nunits > 0 ? 2 : 0;
   r->n_selected = (int64_t)cnt[C_NSEL];
   return CIPSI_OK;
 }

@@ -159,6 +159,19 @@ __device__ __forceinline__ void kahan_add(double& s, double& c, double x) {
   s = t;
 }
 
+// k_pt2_one, forward: per-warp queue of perturbers that survived the interaction
+// scan.  The FP64 epilogue then runs on full warps: the FP64 pipe of GB300 is
+// narrow, and a warp instruction costs the same with 32 lanes or with the few
+// that would be live at the candidate level.
+constexpr int kQCap = 64;
+template <int R>
+struct WarpQueue {
+  double bc[R][kQCap];
+  double hmp[kQCap], hvp[kQCap], fmul[kQCap];
+  int nmul[kQCap];
+  unsigned char flags[kQCap];  // bit 0 ybis, bit 1 is_pert1
+};
+
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxDn = 48;      // spin orbitals where K' differs from the reference
 constexpr int kMaxG = 16;       // rows of a block worked together
@@ -228,10 +241,10 @@ cudaError_t launch_pt2(const Params& p, const LaunchArgs& la, int sms, cudaStrea
 // CTAs of k_cand<W, R, *> per SM
 template <int W, int R>
 int cand_ctas();
-// k_pt2_adj<W, R> launched with `smem` bytes of dynamic shared memory
-// (pt2_adj.cu, pt2_adj_w2.cu)
-template <int W, int R>
-cudaError_t launch_pt2_adj(const Params& p, int grid, size_t smem, cudaStream_t st);
+// k_pt2_one<W, R, ADJ> launched with `smem` bytes of dynamic shared memory
+// (pt2_adj.cu, pt2_adj_w2.cu: adjoint; pt2_one.cu: forward)
+template <int W, int R, bool ADJ>
+cudaError_t launch_pt2_one(const Params& p, int grid, size_t smem, cudaStream_t st);
 
 // The Hamiltonian over a determinant list by rows (hbuild.cu): launch_hcount
 // counts, per row i, the columns j < min(i, jmax) within two excitations;

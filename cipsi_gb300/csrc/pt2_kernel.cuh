@@ -664,6 +664,226 @@ __device__ void block_flush(const Params& p, Acc<R>& acc, int gslot, double* red
   }
 }
 
+// One thread's histogram (cip/isto.f): class sums and counts, indexed by class
+// at run time, so it lives in local memory (L1-resident); one FP64 add per
+// contribution, no atomics; merged into the block's at kernel end.
+template <int R>
+struct HistPriv {
+  double tab[kNClass][2][R];
+  unsigned int nom[kNClass];  // per-thread counts stay far below 2^32
+  unsigned int nam[kNClass][R];
+  __device__ void zero() {
+    for (int c = 0; c < kNClass; ++c) {
+      nom[c] = 0u;
+      for (int m = 0; m < R; ++m) {
+        tab[c][0][m] = tab[c][1][m] = 0.0;
+        nam[c][m] = 0u;
+      }
+    }
+  }
+};
+
+struct SmemHist {
+  unsigned long long nom[kNClass];
+  unsigned long long nam[kNClass * kMaxRoots];
+  double tab[2 * kNClass * kMaxRoots];
+};
+
+// What follows a candidate's interaction scan in the one-kernel form:
+// denominators, E2, selection (counted: this form keeps no records), histogram.
+// Called by all 32 lanes of a warp; `live` marks the lanes holding a perturber.
+template <int R>
+__device__ void finish_candidate(const Params& p, bool live, double hmpi, double hvpi, const double* bc, double fmul,
+                                 int nmul, bool ybis, bool is_pert1, Acc<R>& acc, HistPriv<R>& hp) {
+  double xam = 0.0;
+  bool ydeg = false;
+  // weighted E2 terms per root: term * (1 + fmul), which is also what the
+  // histogram (isto.f, fm = fmul + 1) uses
+  double vil[R], semp[R], sevp[R];
+  // the reference adds each term and then term*fmul (spin-flip weight,
+  // pert1.f:280-287); one compensated add of term*(1+fmul) is used here.
+  // fmul = 0 whenever ybis is false, so wgt = fmul + 1 for every perturber.
+  const double wgt = ybis ? 1.0 + fmul : 1.0;
+#pragma unroll
+  for (int m = 0; m < R; ++m) {
+    vil[m] = 0.0;
+    semp[m] = sevp[m] = 0.0;
+    if (!live || m >= p.metat) continue;
+    const double bcalc = bc[m];
+    const double dmp = p.emp[m] - hmpi;
+    double eivp = 0.0, tvp = 0.0, cimp, xim, deno, eim;
+    if (p.yen) {
+      // the three denominators share one FP64 division (GB300's FP64 rate is
+      // 1/64 of FP32): br = b/(dmp*dvp*db), b/dmp = dvp*db*br, etc.
+      const double dvp = p.e[m] - hvpi;
+      const double db = p.eb[m] - hvpi;
+      const double pvb = dvp * db;
+      const double prod = dmp * pvb;
+      double civp, cib;
+      // 1e-280 < |prod| < 1e280 tested on the exponent field (integer pipe):
+      // binary exponent in [-930, 929]
+      const unsigned pex = (unsigned)(__double_as_longlong(prod) >> 52) & 0x7FFu;
+      if (pex - 93u < 1860u) {
+        const double br = bcalc / prod;
+        cimp = br * pvb;
+        civp = br * (dmp * db);
+        cib = br * (dmp * dvp);
+      } else {  // a denominator at (or near) zero or huge: divide one by one
+        cimp = bcalc / dmp;
+        civp = bcalc / dvp;
+        cib = bcalc / db;
+      }
+      eivp = bcalc * civp;
+      tvp = eivp * wgt;
+      kahan_add(acc.e2vp[m], acc.cvp[m], tvp);
+      acc.psivp[m] = fma(civp * civp, wgt, acc.psivp[m]);
+      kahan_add(acc.e2b[m], acc.cb[m], (bcalc * cib) * wgt);
+      xim = p.ysele ? fabs(eivp) : fabs(civp);
+      deno = dvp;
+      eim = eivp;
+    } else {
+      cimp = bcalc / dmp;
+    }
+    const double eimp = bcalc * cimp;
+    const double tmp = eimp * wgt;
+    kahan_add(acc.e2mp[m], acc.cmp[m], tmp);
+    acc.psimp[m] = fma(cimp * cimp, wgt, acc.psimp[m]);
+    if (!p.yen) {
+      xim = p.ysele ? fabs(eimp) : fabs(cimp);
+      deno = dmp;
+      eim = eimp;
+    }
+    // comparisons of magnitudes on their IEEE bit patterns (exact for
+    // non-negative doubles; NaN compares as in the reference: never below)
+    const long long bdeno = __double_as_longlong(deno) & 0x7fffffffffffffffll;
+    const long long beim = __double_as_longlong(eim) & 0x7fffffffffffffffll;
+    if (!(bdeno > kBits005 && bdeno <= kBitsInf) && !(beim < kBits1em6) && p.ywdeg) ydeg = true;
+    if (lt_nonneg(xim, p.teste[m])) acc.dpivot = max_nonneg(acc.dpivot, xim);
+    if (p.ymoyen) {
+      xim = xim * p.taum[m];
+      vil[m] = xim;
+      xam = max_nonneg(xam, xim);
+    }
+    semp[m] = tmp;
+    sevp[m] = tvp;
+  }
+  if (live) {
+    acc.ietat += (unsigned long long)(long long)(nmul + 1);
+    acc.nproc += 1;
+  }
+  // histogram (cip/isto.f; pert1 calls it always, diexcit only if ymoyen)
+  if (live && (is_pert1 || p.ymoyen) && xam >= p.teseff) {
+    const int cls = hist_class(p, xam);
+    hp.nom[cls] += (unsigned)(1 + nmul);
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+      if (m >= p.metat || vil[m] < p.teseff) continue;
+      hp.tab[cls][0][m] += semp[m];  // eimp * (fmul + 1)
+      hp.tab[cls][1][m] += sevp[m];  // eivp * (fmul + 1)
+      hp.nam[hist_class(p, vil[m])][m] += (unsigned)(1 + nmul);
+    }
+  }
+  if (ydeg) xam = 1.0;
+  const bool sel = live && xam > p.tau && p.ymoyen;
+  const unsigned sm = __ballot_sync(0xffffffffu, sel);
+  if (sm && (threadIdx.x & 31) == 0) atomicAdd(&p.counters[C_NSEL], (unsigned long long)__popc(sm));
+}
+
+template <int R>
+__device__ __noinline__ void drain_queue(const Params& p, WarpQueue<R>& q, int& qn, bool all, Acc<R>& acc,
+                                         HistPriv<R>& hp) {
+  const int lane = threadIdx.x & 31;
+  while (qn >= 32 || (all && qn > 0)) {
+    const int base = qn >= 32 ? qn - 32 : 0;
+    const int cnt = qn >= 32 ? 32 : qn;
+    const bool live = lane < cnt;
+    const int e = base + (live ? lane : 0);
+    double bc[R];
+#pragma unroll
+    for (int m = 0; m < R; ++m) bc[m] = q.bc[m][e];
+    const unsigned char f = q.flags[e];
+    finish_candidate<R>(p, live, q.hmp[e], q.hvp[e], bc, q.fmul[e], q.nmul[e], (f & 1) != 0, (f & 2) != 0, acc, hp);
+    __syncwarp();
+    qn = base;
+  }
+}
+
+// Enqueue the live lanes' perturbers (called by a whole warp); runs the
+// epilogue on every full batch of 32.
+template <int R>
+__device__ void enqueue_candidate(const Params& p, WarpQueue<R>& q, int& qn, bool live, double hmpi, double hvpi,
+                                  const double* bc, double fmul, int nmul, bool ybis, bool is_pert1, Acc<R>& acc,
+                                  HistPriv<R>& hp) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lm = __ballot_sync(0xffffffffu, live);
+  if (live) {
+    const int e = qn + __popc(lm & ((1u << lane) - 1u));
+#pragma unroll
+    for (int m = 0; m < R; ++m) q.bc[m][e] = bc[m];
+    q.hmp[e] = hmpi;
+    q.hvp[e] = hvpi;
+    q.fmul[e] = fmul;
+    q.nmul[e] = nmul;
+    q.flags[e] = (unsigned char)((ybis ? 1 : 0) | (is_pert1 ? 2 : 0));
+  }
+  qn += __popc(lm);
+  __syncwarp();
+  // the drain is out of line; calling it only with a full batch spares the
+  // register saves of a call on every other candidate round
+  if (qn >= 32) drain_queue<R>(p, q, qn, false, acc, hp);
+}
+
+// Counters of the candidate scan (in registers: Acc lives in local memory)
+struct ScanCounts {
+  unsigned long long ncand, ncmp, np1, np2;
+};
+
+// Block totals of the integer counters and the histogram into the global ones.
+template <int R>
+__device__ void flush_totals(const Params& p, const Acc<R>& acc, const HistPriv<R>& hp, SmemHist& hist,
+                             const ScanCounts& sc) {
+  const int tid = threadIdx.x;
+  for (int i = tid; i < kNClass; i += blockDim.x) hist.nom[i] = 0;
+  for (int i = tid; i < kNClass * kMaxRoots; i += blockDim.x) hist.nam[i] = 0;
+  for (int i = tid; i < 2 * kNClass * kMaxRoots; i += blockDim.x) hist.tab[i] = 0.0;
+  __syncthreads();
+  auto count = [&](unsigned long long x, int q) {
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if ((tid & 31) == 0 && x) atomicAdd(&p.counters[q], x);
+  };
+  count(acc.ietat, C_IETAT);
+  count(acc.nproc, C_NPROC);
+  count(sc.ncand, C_NCAND);
+  count(sc.ncmp, C_NCMP);
+  count(sc.np1, C_NP1);
+  count(sc.np2, C_NP2);
+  unsigned long long db = __double_as_longlong(acc.dpivot);
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long y = __shfl_down_sync(0xffffffffu, db, o);
+    db = y > db ? y : db;
+  }
+  if ((tid & 31) == 0) atomicMax(p.dpivot_bits, db);
+  // this thread's histogram into the block's
+  for (int c = 0; c < p.nclass; ++c) {
+    if (hp.nom[c]) atomicAdd(&hist.nom[c], (unsigned long long)hp.nom[c]);
+    for (int m = 0; m < R && m < p.metat; ++m) {
+      if (hp.tab[c][0][m] != 0.0) atomicAdd(&hist.tab[c * kMaxRoots + m], hp.tab[c][0][m]);
+      if (hp.tab[c][1][m] != 0.0) atomicAdd(&hist.tab[kNClass * kMaxRoots + c * kMaxRoots + m], hp.tab[c][1][m]);
+      if (hp.nam[c][m]) atomicAdd(&hist.nam[c * kMaxRoots + m], (unsigned long long)hp.nam[c][m]);
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < p.nclass; i += blockDim.x)
+    if (hist.nom[i]) atomicAdd(&p.hist_nom[i], hist.nom[i]);
+  for (int i = tid; i < p.nclass * kMaxRoots; i += blockDim.x) {
+    const int c = i / kMaxRoots, m = i % kMaxRoots;
+    if (m >= p.metat) continue;
+    if (hist.nam[i]) atomicAdd(&p.hist_nam[c * p.metat + m], hist.nam[i]);
+    if (hist.tab[i] != 0.0) atomicAdd(&p.hist_tab[c * p.metat + m], hist.tab[i]);
+    const double tv = hist.tab[kNClass * kMaxRoots + i];
+    if (tv != 0.0) atomicAdd(&p.hist_tab[p.nclass * p.metat + c * p.metat + m], tv);
+  }
+}
 
 // ------------------------------------------------------------------ kernel
 struct BlockShared {
@@ -684,11 +904,14 @@ struct BlockShared {
   int rank_k;
 };
 
-// The adjoint kernel: E2 sums and the gradients of the integrals and root
-// energies.
-template <int W, int R>
-__global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
+// One kernel for a whole run.  ADJ: E2 sums and the gradients of the integrals
+// and root energies.  Else: the forward run without records, in the memory of
+// its neighbour lists.
+template <int W, int R, bool ADJ>
+__global__ void __launch_bounds__(kThreads, 2) k_pt2_one(Params p0) {
   extern __shared__ __align__(16) unsigned char dyn[];
+  if (p0.nunits <= 0) return;
+  if (p0.nunits <= 0) return;
   // the current geometry's parameters, in shared memory (device functions
   // then read them through a shared-memory reference instead of a local
   // copy of the kernel argument)
@@ -706,6 +929,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
   // L_R entries (compact form, lr_entry) up to lr_cap in shared memory; the
   // rest of a longer list stays in the block's global scratch
   uint64_t* lr_ent = reinterpret_cast<uint64_t*>(dyn);
+  // forward: per-warp epilogue queues, 16-byte aligned after the L_R entries
+  const size_t qoff = (((size_t)p0.lr_cap * 8) + 15) & ~(size_t)15;
+  WarpQueue<R>& wq = reinterpret_cast<WarpQueue<R>*>(dyn + qoff)[threadIdx.x >> 5];
+  int qn = 0;
+  HistPriv<R> hp;
+  ScanCounts sc{};
+  if (!ADJ) hp.zero();
   // per-geometry state
   int32_t* my_nb_j = nullptr;
   uint64_t* my_nb_em = nullptr;
@@ -732,15 +962,17 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
   // adjoint: per-thread root-energy gradients and per-block accumulators of
   // dE/dhdig and dE/dhmp over one block of removed electrons (K' terms:
   // adj_sh[0..1]; per added spin orbital: adj_gv, adj_gf)
-  __shared__ double adj_gv[2 * kMaxOrb], adj_gf[2 * kMaxOrb], adj_sh[2];
+  __shared__ double adj_gv[ADJ ? 2 * kMaxOrb : 1], adj_gf[ADJ ? 2 * kMaxOrb : 1], adj_sh[2];
   double adjr[3][R];
   double adj_gK = 0.0, adj_gM = 0.0;
   double* adj_sl = nullptr;
+  if (ADJ) {
 #pragma unroll
-  for (int m = 0; m < R; ++m) adjr[0][m] = adjr[1][m] = adjr[2][m] = 0.0;
+    for (int m = 0; m < R; ++m) adjr[0][m] = adjr[1][m] = adjr[2][m] = 0.0;
 #pragma unroll 1
-  for (int i = tid; i < 2 * kMaxOrb; i += blockDim.x) adj_gv[i] = adj_gf[i] = 0.0;
-  adj_sl = p0.g_slice + (size_t)blockIdx.x * p0.slice_stride;
+    for (int i = tid; i < 2 * kMaxOrb; i += blockDim.x) adj_gv[i] = adj_gf[i] = 0.0;
+    adj_sl = p0.g_slice + (size_t)blockIdx.x * p0.slice_stride;
+  }
 
   for (;;) {
     __syncthreads();
@@ -777,6 +1009,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
         for (int m = 0; m < R; ++m) bc[m] = 0.0;
         double hmpi = 0.0, hvpi = 0.0;
         if (live) {
+          if (!ADJ) ++sc.ncand;
           int rankI = 0;
 #pragma unroll
           for (int q = 0; q < 2 * W; ++q) rankI += __popcll(hf[q] & ~u[q]);
@@ -788,6 +1021,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
             int x = 0;
 #pragma unroll
             for (int q = 0; q < 2 * W; ++q) x += __popcll(u[q] ^ __ldg(&v[q]));
+            if (!ADJ) ++sc.ncmp;
             if (x > 4) continue;
             if (x == 0) {
               drop = true;
@@ -801,6 +1035,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
             for (int q = 0; q < 2 * W; ++q) rankJ += __popcll(hf[q] & ~vv[q]);
             int kind;
             const double h = hmat<W>(p, u, vv, rankI, rankJ, hf, kind);
+            if (!ADJ) ++(kind == 1 ? sc.np1 : sc.np2);
             ++nint;
 #pragma unroll
             for (int m = 0; m < R; ++m)
@@ -809,11 +1044,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
           if (drop || nint == 0) live = false;
           if (live) diag_terms<W>(p, u, hf, hmpi, hvpi, p.yen != 0);
         }
-        if (live) {
+        if (!ADJ) enqueue_candidate<R>(p, wq, qn, live, hmpi, hvpi, bc, 0.0, 0, false, true, acc, hp);
+        if (ADJ && live) {
           double gb[R], gh, gm;
           adj_factors<R>(p, bc, hmpi, hvpi, 1.0, gb, gh, gm, adjr, acc);
-          acc.ietat += 1;
-          acc.nproc += 1;
           int rankI = 0;
 #pragma unroll
           for (int q = 0; q < 2 * W; ++q) rankI += __popcll(hf[q] & ~u[q]);
@@ -840,6 +1074,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
           diag_terms_adj<W>(p, u, hf, p.yen ? gh : 0.0, gm, adj_sl);
         }
       }
+      if (!ADJ) drain_queue<R>(p, wq, qn, true, acc, hp);
       block_flush<R>(p, acc, unit, red);
       continue;
     }
@@ -1138,11 +1373,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
         // adjoint: the first two one-difference partners j (and their count),
         // for the one-electron second pass
         int s1n = 0, s1j0 = 0, s1j1 = 0;
+        unsigned n1 = 0;  // forward: one-difference pairs of this candidate
         const int rankI = rank_k + D;
         const bool two = a2 >= 0;
         const uint32_t c1x4 = live ? (uint32_t)(a1 + sa1 * p.norb) * 0x01010101u : 0u;
         const uint32_t c2x4 = live && two ? (uint32_t)(a2 + sa2 * p.norb) * 0x01010101u : 0u;
         if (live) {
+          if (!ADJ) ++sc.ncand;
           or_word<2 * W>(u, sa1 * W + (a1 >> 6), 1ull << (a1 & 63));
           if (a2 >= 0) or_word<2 * W>(u, sa2 * W + (a2 >> 6), 1ull << (a2 & 63));
         }
@@ -1175,7 +1412,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
               for (int q = 0; q < 2 * W; ++q) rankJ += __popcll(hf[q] & ~vv[q]);
               int kind;
               const double h = hmat<W>(p, u, vv, rankI, rankJ, hf, kind);
-                if (kind == 1) {
+              if (!ADJ) n1 += kind == 1 ? 1u : 0u;
+              if (ADJ && kind == 1) {
                 s1j1 = s1n == 1 ? j : s1j1;
                 s1j0 = s1n == 0 ? j : s1j0;
                 ++s1n;
@@ -1225,6 +1463,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
         }
         flush();
         if (live) {
+          if (!ADJ) {  // the pairs of what no earlier generator owns, as k_cand counts them
+            sc.ncmp += (unsigned long long)(nscan + nrb);
+            if (!drop) {
+              sc.np1 += n1;
+              sc.np2 += (unsigned)nint - n1;
+            }
+          }
           if (drop || nint == 0) live = false;
           if (live && D == 2 && nnz == 0) live = false;  // diexcit drops zero couplings
         }
@@ -1259,13 +1504,15 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
             hvpi += sh.vdg[a2 + sa2 * p.norb] + gq;
           }
         }
+        if (!ADJ) {
+          enqueue_candidate<R>(p, wq, qn, live, hmpi, hvpi, bc, fmul, nmul, ybis, is_pert1, acc, hp);
+          return;
+        }
         double gb[R], gh = 0.0, gm = 0.0;
 #pragma unroll
         for (int m = 0; m < R; ++m) gb[m] = 0.0;
         if (live) {
           adj_factors<R>(p, bc, hmpi, hvpi, ybis ? 1.0 + fmul : 1.0, gb, gh, gm, adjr, acc);
-          acc.ietat += (unsigned long long)(long long)(nmul + 1);
-          acc.nproc += 1;
           if (!p.yen) gh = 0.0;
         }
         // second pass over the same entries: dE/dH_Ij = sum_m gb[m] c_jm,
@@ -1416,7 +1663,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
             candidate(live, a1, a2, sr, sc, overflow ? nlr : n01, rowbuf, overflow ? 0 : nrb);
           }
           __syncwarp();
-          if (__any_sync(0xffffffffu, row_gh != 0.0 || row_gm != 0.0)) {
+          if (ADJ && __any_sync(0xffffffffu, row_gh != 0.0 || row_gm != 0.0)) {
 #pragma unroll 1
             for (int o = 16; o > 0; o >>= 1) {
               row_gh += __shfl_down_sync(0xffffffffu, row_gh, o);
@@ -1431,6 +1678,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
         }
       }
       __syncthreads();
+      if (!ADJ) continue;
       // expand this block's dE/dhdig and dE/dhmp sums over F, J, K, fmpb
       if (tid < 2) adj_sh[tid] = 0.0;
       __syncthreads();
@@ -1494,9 +1742,15 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
       for (int i = tid; i < 2 * n; i += blockDim.x) adj_gv[i] = adj_gf[i] = 0.0;
       __syncthreads();
     }
+    if (!ADJ) drain_queue<R>(p, wq, qn, true, acc, hp);
     block_flush<R>(p, acc, unit, red);
   }
 
+  if (!ADJ) {
+    __shared__ SmemHist hist;
+    flush_totals<R>(p, acc, hp, hist, sc);
+    return;
+  }
 #pragma unroll
   for (int k3 = 0; k3 < 3; ++k3)
 #pragma unroll
@@ -1510,11 +1764,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_pt2_adj(Params p0) {
 
 }  // namespace
 
-template <int W, int R>
-cudaError_t launch_pt2_adj(const Params& p, int grid, size_t smem, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(k_pt2_adj<W, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k_pt2_adj<W, R><<<grid, kThreads, smem, st>>>(p);
+template <int W, int R, bool ADJ>
+cudaError_t launch_pt2_one(const Params& p, int grid, size_t smem, cudaStream_t st) {
+  if (smem) {
+    cudaError_t e = cudaFuncSetAttribute(k_pt2_one<W, R, ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  k_pt2_one<W, R, ADJ><<<grid, kThreads, smem, st>>>(p);
   return cudaGetLastError();
 }
 
