@@ -44,30 +44,34 @@ __global__ void __launch_bounds__(kReduceThreads) k_reduce(const double* part, i
   }
 }
 
-// One exact sum (words of 32 bits in 64-bit counters, the top one signed, in
-// units of 2^-unit) as a double, rounded once from its leading 96 bits.
+// One exact sum (N words of 32 bits in 64-bit counters, the top one signed, in
+// units of 2^-unit) as a double, from its leading 96 bits (at least 65 of them
+// significant: an error of half an ulp and 2^-11 of one at most).
+template <int N>
 __device__ double fx_value(const unsigned long long* g, int unit) {
-  uint32_t w[5];
-  unsigned long long c = 0;
-  for (int i = 0; i < 3; ++i) {
+  uint32_t w[N + 1];
+  unsigned long long c = 0, any = 0;
+  for (int i = 0; i < N; ++i) any |= g[i];
+  if (any == 0) return 0.0;
+  for (int i = 0; i < N - 1; ++i) {
     // the carry is below 2^32 and the counter well below 2^64 - 2^32
     const unsigned long long x = g[i] + c;
     w[i] = (uint32_t)x;
     c = x >> 32;
   }
-  const long long top = (long long)(g[3] + c);
-  w[3] = (uint32_t)top;
-  w[4] = (uint32_t)((unsigned long long)top >> 32);
+  const long long top = (long long)(g[N - 1] + c);
+  w[N - 1] = (uint32_t)top;
+  w[N] = (uint32_t)((unsigned long long)top >> 32);
   const bool neg = top < 0;
   if (neg) {
     unsigned long long b = 1;
-    for (int i = 0; i < 5; ++i) {
+    for (int i = 0; i <= N; ++i) {
       b += (uint32_t)~w[i];
       w[i] = (uint32_t)b;
       b >>= 32;
     }
   }
-  int h = 4;
+  int h = N;
   while (h > 0 && w[h] == 0u) --h;
   const unsigned long long hi = ((unsigned long long)w[h] << 32) | (h >= 1 ? w[h - 1] : 0u);
   double v = (double)hi * 4294967296.0 + (double)(h >= 2 ? w[h - 2] : 0u);
@@ -78,32 +82,44 @@ __device__ double fx_value(const unsigned long long* g, int unit) {
 // The forward kernel's exact sums of geometry blockIdx.x as doubles: class
 // sums to hist_tab, E2 sums and norms (every class together, and the terms
 // outside the histogram) to red.  One small block per geometry: no partial
-// sums per work unit are kept or added up.
+// sums per work unit are kept or added up.  The tables (22 KB, one after the
+// other) come to shared memory first, all loads in flight at once: a thread
+// that walks its classes' words in global memory waits for each.
 constexpr int kFinishThreads = 256;
+constexpr int kFxTables = (kFxWords + kFxWordsHi + kFxWordsLo + 1) * kFxSums;
 __global__ void __launch_bounds__(kFinishThreads) k_finish(Params p0, const Params* geo) {
+  __shared__ unsigned long long tables[kFxTables];
   const Params& p = geo ? geo[blockIdx.x] : p0;
   const int mt = p.metat, nc = p.nclass;
-  auto value = [&](const unsigned long long* lo, const unsigned long long* hi, double big) {
-    return fx_value(lo, 84) + (fx_value(hi, 44) + big);
+  const unsigned long long* from = p.sums;
+#pragma unroll 11
+  for (int i = threadIdx.x; i < kFxTables; i += kFinishThreads) tables[i] = from[i];
+  __syncthreads();
+  const unsigned long long *main = tables, *high = main + kFxWords * kFxSums, *low = high + kFxWordsHi * kFxSums;
+  const double* big = reinterpret_cast<const double*>(low + kFxWordsLo * kFxSums);
+  auto value = [&](const unsigned long long* s, const unsigned long long* hi, const unsigned long long* lo, double x) {
+    return (fx_value<kFxWords>(s, kFxUnit) + fx_value<kFxWordsLo>(lo, kFxUnitLo)) +
+           (fx_value<kFxWordsHi>(hi, kFxUnitHi) + x);
   };
-  for (int i = threadIdx.x; i < 2 * nc * mt; i += kFinishThreads) {
-    const int q = i / (nc * mt), c = i / mt % nc, m = i % mt;
-    const int x = fx_tab(q, c, m);
-    p.hist_tab[i] = value(p.sums + 4 * x, p.sums_hi + 4 * x, p.sums_big[x]);
-  }
-  for (int i = threadIdx.x; i < 5 * mt; i += kFinishThreads) {
+  // (the E2 sums' threads have the most to do: theirs are the first warps)
+  for (int i = threadIdx.x; i < 5 * mt + 2 * nc * mt; i += kFinishThreads) {
+    if (i >= 5 * mt) {
+      const int h = i - 5 * mt, q = h / (nc * mt), c = h / mt % nc, m = h % mt;
+      const int x = fx_tab(q, c, m);
+      p.hist_tab[h] = value(main + kFxWords * x, high + kFxWordsHi * x, low + kFxWordsLo * x, big[x]);
+      continue;
+    }
     const int q = i / mt, m = i % mt;
-    unsigned long long lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
-    double big = 0.0;
+    unsigned long long s[kFxWords] = {}, hi[kFxWordsHi] = {}, lo[kFxWordsLo] = {};
+    double b = 0.0;
     for (int c = 0; c <= (q < 2 ? kNClass : 0); ++c) {
       const int x = q < 2 ? fx_tab(q, c, m) : fx_acc(q - 2, m);
-      for (int w = 0; w < 4; ++w) {
-        lo[w] += p.sums[4 * x + w];
-        hi[w] += p.sums_hi[4 * x + w];
-      }
-      big += p.sums_big[x];
+      for (int w = 0; w < kFxWords; ++w) s[w] += main[kFxWords * x + w];
+      for (int w = 0; w < kFxWordsHi; ++w) hi[w] += high[kFxWordsHi * x + w];
+      for (int w = 0; w < kFxWordsLo; ++w) lo[w] += low[kFxWordsLo * x + w];
+      b += big[x];
     }
-    p.red[i] = value(lo, hi, big);
+    p.red[i] = value(s, hi, lo, b);
   }
 }
 
@@ -200,10 +216,10 @@ __global__ void __launch_bounds__(256) k_gather(GatherArgs a) {
 }
 
 // What a run accumulates into, in one allocation cleared by one call:
-// counters, dpivot, histogram counts | exact sums | work counter, records in
-// the pool (8 bytes each).
+// counters, dpivot, histogram counts | exact sums (k_finish reads their tables
+// as one array) | work counter, records in the pool (8 bytes each).
 constexpr size_t kCountWords = C_NCOUNTERS + 1 + kNClass + kNClass * kMaxRoots;
-constexpr size_t kZeroWords = kCountWords + (size_t)9 * kFxSums + 2;
+constexpr size_t kZeroWords = kCountWords + (size_t)kFxTables + 2;
 // a run's result on the device: reduced sums, class sums, counters
 constexpr size_t kTabWord = 5 * kMaxRoots, kTabWords = 2 * kNClass * kMaxRoots;
 constexpr size_t kResWords = kTabWord + kTabWords + kCountWords;
@@ -213,8 +229,9 @@ void set_zeroed(Params& p, unsigned long long* z) {
   p.hist_nom = z + C_NCOUNTERS + 1;
   p.hist_nam = z + C_NCOUNTERS + 1 + kNClass;
   p.sums = z + kCountWords;
-  p.sums_hi = p.sums + (size_t)4 * kFxSums;
-  p.sums_big = reinterpret_cast<double*>(p.sums_hi + (size_t)4 * kFxSums);
+  p.sums_hi = p.sums + (size_t)kFxWords * kFxSums;
+  p.sums_lo = p.sums_hi + (size_t)kFxWordsHi * kFxSums;
+  p.sums_big = reinterpret_cast<double*>(p.sums_lo + (size_t)kFxWordsLo * kFxSums);
   p.work = reinterpret_cast<int*>(z + kZeroWords - 2);
   p.pool_count = z + kZeroWords - 1;
 }

@@ -86,10 +86,11 @@ struct Params {
   double* hist_tab;                  // 2 x nclass x metat (tabmp, tabvp)
   double* red;                       // 5 x metat reduced sums (k_reduce / k_finish output)
   // exact sums of the forward kernel, indexed by fx_tab / fx_acc: words of 32
-  // bits in 64-bit counters (units 2^-84), the same for terms of 2^22 and
-  // more (units 2^-44), and what lies beyond 2^62 or is not finite
+  // bits in 64-bit counters, for terms of 2^-64 to 2^22, for larger and for
+  // smaller ones (kFx*), and what lies beyond those or is not finite
   unsigned long long* sums;
   unsigned long long* sums_hi;
+  unsigned long long* sums_lo;
   double* sums_big;
   // unit-60 records.  When k_pt2 is done with a work unit, it compacts the
   // selected candidates, in slot order, into one segment of the record pool
@@ -219,6 +220,11 @@ constexpr size_t fwd_smem() {
 __host__ __device__ constexpr int fx_tab(int q, int c, int m) { return (q * (kNClass + 1) + c) * kMaxRoots + m; }
 __host__ __device__ constexpr int fx_acc(int q, int m) { return (2 * (kNClass + 1) + q) * kMaxRoots + m; }
 constexpr int kFxSums = (2 * (kNClass + 1) + 3) * kMaxRoots;
+// words of the three tables and their units (2^-unit): every bit of a term is
+// held, whatever its size -- terms of 2^-64 to 2^22 end at 2^-116 or above,
+// those up to 2^62 at 2^-30 or above, those down to 2^-127 at 2^-179 or above
+constexpr int kFxWords = 5, kFxUnit = 116, kFxWordsHi = 4, kFxUnitHi = 44, kFxWordsLo = 4, kFxUnitLo = 180;
+constexpr int kFxMin = -64, kFxMax = 22, kFxMinLo = -127;  // exponents: the main table's terms; the least of sums_lo
 
 // Candidates of one block of removed electrons R: nv added orbitals for
 // |R| = 1, nv(nv-1)/2 same-spin pairs, nva * nvb opposite-spin pairs (nv:

@@ -20,72 +20,117 @@ namespace {
 constexpr int kWtCap = 8;  // spin-flip weights tabulated for lesp < kWtCap
 
 // ------------------------------------------------------------ exact sums
-// A sum in units of 2^-84 as a 128-bit two's complement integer.  A term is
-// rounded to that unit (error <= 2.6e-26) and added exactly; terms of 2^22 and
-// more go to the global table at once (fx_big).
+// A lane's sum in units of 2^-kFxUnit as a two's complement integer.  Terms of
+// 2^kFxMin to 2^kFxMax have no bit below that unit and are added exactly; larger
+// and smaller ones go to tables of their own (fx_out), so that a sum of small
+// terms keeps as many places as one of large terms.
 struct Fx {
-  uint32_t w[4];
+  uint32_t w[kFxWords];
 };
 
-// words of |t| 2^84 rounded to nearest, and the add's carry-in and sign mask
+__device__ __forceinline__ Fx fx_of(uint4 w, uint32_t top) { return Fx{{w.x, w.y, w.z, w.w, top}}; }
+
+// adds t if 2^kFxMin <= |t| < 2^kFxMax, else nothing
 __device__ __forceinline__ void fx_add(Fx& s, double t) {
   const int hi = __double2hiint(t);
   const uint32_t lo = (uint32_t)__double2loint(t);
   const int ex = (hi >> 20) & 0x7ff;
   const uint32_t m1 = ((uint32_t)hi & 0xfffffu) | 0x100000u;
-  // |t| = m 2^(ex-1075); bit position of m's lowest bit in a number whose
-  // unit is 2^-148 (two words below the sum's)
-  const int sh = ex - (1075 - 148);
-  const int w = sh >> 5;  // below 0: |t| < 2^-96, under half a unit
+  // |t| = m 2^(ex-1075); bit position of m's lowest bit in the sum
+  const int sh = ex - (1075 - kFxUnit);
+  const int w = sh >> 5;  // 0, 1, 2
   const uint32_t a0 = __funnelshift_l(0u, lo, sh);
   const uint32_t a1 = __funnelshift_l(lo, m1, sh);
   const uint32_t a2 = __funnelshift_l(m1, 0u, sh);
-  const bool w0 = w == 0, w1 = w == 1, w2 = w == 2, w3 = w == 3;  // |t| < 2^22: w <= 3
-  uint32_t v0 = w2 ? a0 : (w1 ? a1 : (w0 ? a2 : 0u));
-  uint32_t v1 = w3 ? a0 : (w2 ? a1 : (w1 ? a2 : 0u));
-  uint32_t v2 = w3 ? a1 : (w2 ? a2 : 0u);
-  uint32_t v3 = w3 ? a2 : 0u;
-  const uint32_t below = w1 ? a0 : (w0 ? a1 : 0u);
-  const uint32_t sg = (uint32_t)(hi >> 31);
-  const uint32_t cin = (below >> 31) ^ (sg & 1u);  // s + v + r, or s - v - r = s + ~v + (1 - r)
+  const bool w0 = w == 0, w1 = w == 1, w2 = (unsigned)(sh - 64) < (unsigned)(kFxMax - kFxMin - 64);
+  uint32_t v0 = w0 ? a0 : 0u;
+  uint32_t v1 = w1 ? a0 : (w0 ? a1 : 0u);
+  uint32_t v2 = w2 ? a0 : (w1 ? a1 : (w0 ? a2 : 0u));
+  uint32_t v3 = w2 ? a1 : (w1 ? a2 : 0u);
+  uint32_t v4 = w2 ? a2 : 0u;
+  const uint32_t sg = (uint32_t)(hi >> 31);  // s + v, or s - v = s + ~v + 1
   v0 ^= sg;
   v1 ^= sg;
   v2 ^= sg;
   v3 ^= sg;
+  v4 ^= sg;
   asm("{\n\t.reg .u32 t;\n\t"
-      "add.cc.u32 t, %8, 0xffffffff;\n\t"
-      "addc.cc.u32 %0, %0, %4;\n\t"
-      "addc.cc.u32 %1, %1, %5;\n\t"
-      "addc.cc.u32 %2, %2, %6;\n\t"
-      "addc.u32 %3, %3, %7;\n\t}"
-      : "+r"(s.w[0]), "+r"(s.w[1]), "+r"(s.w[2]), "+r"(s.w[3])
-      : "r"(v0), "r"(v1), "r"(v2), "r"(v3), "r"(cin));
+      "add.cc.u32 t, %10, 0xffffffff;\n\t"
+      "addc.cc.u32 %0, %0, %5;\n\t"
+      "addc.cc.u32 %1, %1, %6;\n\t"
+      "addc.cc.u32 %2, %2, %7;\n\t"
+      "addc.cc.u32 %3, %3, %8;\n\t"
+      "addc.u32 %4, %4, %9;\n\t}"
+      : "+r"(s.w[0]), "+r"(s.w[1]), "+r"(s.w[2]), "+r"(s.w[3]), "+r"(s.w[4])
+      : "r"(v0), "r"(v1), "r"(v2), "r"(v3), "r"(v4), "r"(sg & 1u));
 }
 
-// |t| < 2^22
-__device__ __forceinline__ bool fx_fits(double t) { return ((__double2hiint(t) >> 20) & 0x7ff) < 1023 + 22; }
+__device__ __forceinline__ int fx_exponent(double t) { return ((__double2hiint(t) >> 20) & 0x7ff) - 1023; }
+// high word of |t|; that of every term of the lanes' sums lies in [kFxHiMin, kFxHiMax)
+__device__ __forceinline__ int fx_high(double t) { return __double2hiint(t) & 0x7fffffff; }
+constexpr int kFxHiMin = (1023 + kFxMin) << 20, kFxHiMax = (1023 + kFxMax) << 20;
 
-// a large term into the global table of sum q: a second fixed-point number in
-// units of 2^-44 below 2^62 (exact for these terms), plain FP64 beyond, for
-// infinities and for NaN
-__device__ __noinline__ void fx_big(const Params& p, int q, double t) {
-  double* big = p.sums_big + q;
-  const double a = fabs(t);
-  if (!(a < 4611686018427387904.0)) {
-    atomicAdd(big, t);
-    return;
-  }
-  // 106 bits: two 53-bit halves would do; words of 32 bits as in the lanes' sums
-  const unsigned __int128 v = (unsigned __int128)(unsigned long long)a << 44 |
-                              (unsigned __int128)(unsigned long long)((a - trunc(a)) * 17592186044416.0);
-  unsigned __int128 x = t < 0 ? (unsigned __int128)0 - v : v;
-  unsigned long long* g = p.sums_hi + (size_t)q * 4;
+// |t| = (hi + lo 2^-64) units into the words g; its sign
+__device__ void fx_words(unsigned long long* g, unsigned long long hi, unsigned long long lo, bool neg) {
+  unsigned __int128 x = (unsigned __int128)hi << 64 | lo;
+  if (neg) x = (unsigned __int128)0 - x;
 #pragma unroll 1
   for (int i = 0; i < 3; ++i) {
     atomicAdd(&g[i], (unsigned long long)(uint32_t)x);
     x >>= 32;
   }
   atomicAdd(&g[3], (unsigned long long)(long long)(int32_t)(uint32_t)x);
+}
+static_assert(kFxWordsHi == 4 && kFxWordsLo == 4, "fx_words writes four");
+
+// a term of 2^kFxMax or more to sum q's own table (exact below 2^62); plain
+// FP64 beyond, for infinities and for NaN
+__device__ __noinline__ void fx_big(const Params& p, int q, double t) {
+  const double a = fabs(t);
+  if (!(a < 0x1p62)) {
+    atomicAdd(p.sums_big + q, t);
+    return;
+  }
+  // 2^-kFxUnitHi units: the whole part above the lowest 44 bits of the words
+  const unsigned long long n = (unsigned long long)a;
+  const unsigned long long f = (unsigned long long)((a - trunc(a)) * 0x1p44);
+  fx_words(p.sums_hi + (size_t)q * kFxWordsHi, n >> (64 - kFxUnitHi), n << kFxUnitHi | f, t < 0.0);
+}
+// a sum of up to 32 terms below 2^kFxMin, likewise; plain FP64 below 2^kFxMinLo
+__device__ __noinline__ void fx_small(const Params& p, int q, double t) {
+  if (t == 0.0) return;
+  if (fx_exponent(t) < kFxMinLo) {
+    atomicAdd(p.sums_big + q, t);
+    return;
+  }
+  const double a = fabs(t) * 0x1p116;  // whole part: units of 2^64 of the words' 2^-180
+  const unsigned long long n = (unsigned long long)a;
+  fx_words(p.sums_lo + (size_t)q * kFxWordsLo, n, (unsigned long long)((a - (double)n) * 0x1p64), t < 0.0);
+}
+static_assert(kFxUnitHi == 44 && kFxUnitLo == 180 && kFxMin == -64, "fx_big and fx_small are written for these");
+
+// The term t of each lane that has one (`mine`) to a table of sum q, if the
+// lanes' sums do not take it.  Called by the whole warp.  Small terms are added
+// up by sum first, in an order that only the queue decides: couplings that
+// vanish but for rounding are many, and thousands of warps would wait for one
+// address.
+__device__ __noinline__ void fx_out(const Params& p, bool mine, int q, double t) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int h = fx_high(t);
+  const bool small = mine && h < kFxHiMin;
+  if (mine && h >= kFxHiMax) fx_big(p, q, t);
+  unsigned rest = __ballot_sync(kFull, small);
+#pragma unroll 1
+  while (rest) {
+    const int src = __ffs((int)rest) - 1;
+    const int qs = __shfl_sync(kFull, q, src);
+    const bool same = small && q == qs;
+    rest &= ~__ballot_sync(kFull, same);
+    double s = same ? t : 0.0;
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+    if ((threadIdx.x & 31) == src) fx_small(p, qs, s);
+  }
 }
 
 // 1/d to within about an ulp: hardware approximation r0 (relative error below
@@ -105,7 +150,7 @@ __device__ __forceinline__ bool recip_ok(double d) {
 // One perturber's terms of a root: b^2 w / d for the MP, EN and barycentric
 // denominators, the norms (b/d)^2 w, and the coefficient the selection looks at
 struct Terms {
-  double mp, vp, b, pm, pv, c;
+  double mp, vp, b, pm, pv, c, deno;
 };
 __device__ __noinline__ Terms terms_by_division(double b, double wgt, double dmp, double dvp, double db, bool en) {
   Terms t;
@@ -122,22 +167,84 @@ __device__ __noinline__ Terms terms_by_division(double b, double wgt, double dmp
   }
   return t;
 }
+// the terms of root m for a coupling b
+__device__ __forceinline__ Terms terms_of(const Params& p, int m, double b, double wgt, double hmpi, double hvpi) {
+  Terms t;
+  const double dmp = p.emp[m] - hmpi;
+  if (p.yen) {
+    const double dvp = p.e[m] - hvpi, db = p.eb[m] - hvpi;
+    if (recip_ok(dmp) && recip_ok(dvp) && recip_ok(db)) {
+      const double b2w = (b * b) * wgt;
+      const double rm = recip(dmp), rv = recip(dvp);
+      t.mp = b2w * rm;
+      t.vp = b2w * rv;
+      t.b = b2w * recip(db);
+      t.pm = t.mp * rm;
+      t.pv = t.vp * rv;
+      t.c = b * rv;
+    } else {  // a denominator at (or near) zero or huge
+      t = terms_by_division(b, wgt, dmp, dvp, db, true);
+    }
+    t.deno = dvp;
+    return t;
+  }
+  if (recip_ok(dmp)) {
+    const double rm = recip(dmp);
+    t.c = b * rm;
+    t.mp = (b * t.c) * wgt;
+    t.pm = t.mp * rm;
+    t.vp = t.b = t.pv = 0.0;
+  } else {
+    t = terms_by_division(b, wgt, dmp, 0.0, 0.0, false);
+  }
+  t.deno = dmp;
+  return t;
+}
+// all of them fit the lanes' sums
+__device__ __forceinline__ bool terms_in(const Params& p, const Terms& t, double b) {
+  int lo = min(fx_high(t.mp), fx_high(t.pm)), hi = max(fx_high(t.mp), fx_high(t.pm));
+  if (p.yen) {
+    lo = min(min(lo, fx_high(t.vp)), min(fx_high(t.b), fx_high(t.pv)));
+    hi = max(max(hi, fx_high(t.vp)), max(fx_high(t.b), fx_high(t.pv)));
+  }
+  return (lo >= kFxHiMin && hi < kFxHiMax) || (__double_as_longlong(b) << 1) == 0;
+}
+// those of root m, class ct, that do not, to the global tables (of the lanes that
+// have some: `mine`); called by the whole warp
+__device__ __noinline__ void odd_terms(const Params& p, bool mine, int m, int ct, double b, double wgt, double hmpi,
+                                       double hvpi) {
+  Terms t{};
+  if (mine) t = terms_of(p, m, b, wgt, hmpi, hvpi);
+  fx_out(p, mine, fx_tab(0, ct, m), t.mp);
+  fx_out(p, mine, fx_acc(1, m), t.pm);
+  if (!p.yen) return;
+  fx_out(p, mine, fx_tab(1, ct, m), t.vp);
+  fx_out(p, mine, fx_acc(0, m), t.b);
+  fx_out(p, mine, fx_acc(2, m), t.pv);
+}
 __device__ __noinline__ double spin_weight_any(int nespf, int lesp) { return spin_weight(nespf, lesp); }
+
+// tests of run parameters on their bits too: an FP64 compare takes as long as an
+// addition
+constexpr long long kBitsOne = 0x3ff0000000000000ll;
+__device__ __forceinline__ bool below_zero(double x) {
+  return __double_as_longlong(x) < 0 && (__double_as_longlong(x) << 1) != 0;
+}
 
 // one lane sum over the warp, added to global sum q (words of 32 bits in
 // 64-bit counters: carries are resolved when the sums are converted)
 __device__ __noinline__ void flush_fx(const Params& p, Fx s, int q) {
   constexpr unsigned kFull = 0xffffffffu;
-  if (!__any_sync(kFull, (s.w[0] | s.w[1] | s.w[2] | s.w[3]) != 0u)) return;
+  if (!__any_sync(kFull, (s.w[0] | s.w[1] | s.w[2] | s.w[3] | s.w[4]) != 0u)) return;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < kFxWords; ++i) {
     // 32 words summed as two 16-bit halves in 32-bit lanes
     const uint32_t x = s.w[i];
     const long long lo = (long long)__reduce_add_sync(kFull, x & 0xffffu);
-    const long long hi = i < 3 ? (long long)__reduce_add_sync(kFull, x >> 16)
-                               : (long long)__reduce_add_sync(kFull, (int)x >> 16);
+    const long long hi = i < kFxWords - 1 ? (long long)__reduce_add_sync(kFull, x >> 16)
+                                          : (long long)__reduce_add_sync(kFull, (int)x >> 16);
     const long long v = lo + hi * 65536;
-    if ((threadIdx.x & 31) == 0 && v != 0) atomicAdd(&p.sums[(size_t)q * 4 + i], (unsigned long long)v);
+    if ((threadIdx.x & 31) == 0 && v != 0) atomicAdd(&p.sums[(size_t)q * kFxWords + i], (unsigned long long)v);
   }
 }
 
@@ -193,18 +300,24 @@ __global__ void __launch_bounds__(kThreads, kEpiCtas<R>) k_pt2(Params p0, Launch
 
   // lane sums: by class the MP and EN terms (class kNClass: terms outside the
   // histogram), then e2b, psimp, psivp
-  Fx tab[kNClass + 1][2][R];
+  // (the tables in local memory: four words of a sum are one access, the top
+  // words of both another)
+  uint4 tab[kNClass + 1][R][2];
+  uint2 top[kNClass + 1][R];
   Fx acc[3][R];
   unsigned long long ietat = 0;
   unsigned int nproc = 0, nsel = 0;
   double dpivot = 0.0;
   auto zero_sums = [&]() {
 #pragma unroll 1
-    for (int i = 0; i < (kNClass + 1) * 2 * R; ++i) (&tab[0][0][0])[i] = Fx{{0u, 0u, 0u, 0u}};
+    for (int i = 0; i < (kNClass + 1) * R; ++i) {
+      tab[i / R][i % R][0] = tab[i / R][i % R][1] = make_uint4(0u, 0u, 0u, 0u);
+      top[i / R][i % R] = make_uint2(0u, 0u);
+    }
 #pragma unroll
     for (int q = 0; q < 3; ++q)
 #pragma unroll
-      for (int m = 0; m < R; ++m) acc[q][m] = Fx{{0u, 0u, 0u, 0u}};
+      for (int m = 0; m < R; ++m) acc[q][m] = Fx{};
 #pragma unroll 1
     for (int i = lane; i < (kNClass + 1) * (1 + R); i += 32) sh.hn[wid][i] = 0u;
     ietat = 0ull;
@@ -217,9 +330,11 @@ __global__ void __launch_bounds__(kThreads, kEpiCtas<R>) k_pt2(Params p0, Launch
   // the warp's sums and counters into the geometry's; then zero
   auto flush_geometry = [&]() {
 #pragma unroll 1
-    for (int i = 0; i < (kNClass + 1) * 2 * R; ++i) {
-      const int c = i / (2 * R), q = i / R % 2, m = i % R;
-      flush_fx(p, tab[c][q][m], fx_tab(q, c, m));
+    for (int i = 0; i < (kNClass + 1) * R; ++i) {
+      const int c = i / R, m = i % R;
+      const uint2 t = top[c][m];
+      flush_fx(p, fx_of(tab[c][m][0], t.x), fx_tab(0, c, m));
+      flush_fx(p, fx_of(tab[c][m][1], t.y), fx_tab(1, c, m));
     }
 #pragma unroll
     for (int q = 0; q < 3; ++q)
@@ -319,104 +434,80 @@ __global__ void __launch_bounds__(kThreads, kEpiCtas<R>) k_pt2(Params p0, Launch
       }
       double tmp[R], tvp[R], vil[R], xam = 0.0;
       bool ydeg = false;
+      unsigned odd = 0u;  // roots with a term that the lane's sums do not take
 #pragma unroll
       for (int m = 0; m < R; ++m) {
         tmp[m] = tvp[m] = vil[m] = 0.0;
         if (!live || m >= p.metat) continue;
         const double b = la.cand.b[m * la.cand.cap + s];
-        const double dmp = p.emp[m] - hmpi;
-        double deno;
-        Terms t;
-        if (p.yen) {
-          const double dvp = p.e[m] - hvpi, db = p.eb[m] - hvpi;
-          deno = dvp;
-          if (recip_ok(dmp) && recip_ok(dvp) && recip_ok(db)) {
-            const double b2w = (b * b) * wgt;
-            const double rm = recip(dmp), rv = recip(dvp);
-            t.mp = b2w * rm;
-            t.vp = b2w * rv;
-            t.b = b2w * recip(db);
-            t.pm = t.mp * rm;
-            t.pv = t.vp * rv;
-            t.c = b * rv;
-          } else {  // a denominator at (or near) zero or huge
-            t = terms_by_division(b, wgt, dmp, dvp, db, true);
-          }
-        } else {
-          deno = dmp;
-          if (recip_ok(dmp)) {
-            const double rm = recip(dmp);
-            t.c = b * rm;
-            t.mp = (b * t.c) * wgt;
-            t.pm = t.mp * rm;
-            t.vp = t.b = t.pv = 0.0;
-          } else {
-            t = terms_by_division(b, wgt, dmp, 0.0, 0.0, false);
-          }
-        }
+        const Terms t = terms_of(p, m, b, wgt, hmpi, hvpi);
         tmp[m] = t.mp;
         tvp[m] = t.vp;
-        double tb = t.b, pm = t.pm, pv = t.pv;
-        const double cx = t.c;
-        // large, infinite and NaN terms straight to the global table
-        if (!(fx_fits(tb) && fx_fits(pm) && fx_fits(pv))) {
-          if (!fx_fits(tb)) { fx_big(p, fx_acc(0, m), tb); tb = 0.0; }
-          if (!fx_fits(pm)) { fx_big(p, fx_acc(1, m), pm); pm = 0.0; }
-          if (!fx_fits(pv)) { fx_big(p, fx_acc(2, m), pv); pv = 0.0; }
-        }
         if (p.yen) {
-          fx_add(acc[0][m], tb);
-          fx_add(acc[2][m], pv);
+          fx_add(acc[0][m], t.b);
+          fx_add(acc[2][m], t.pv);
         }
-        fx_add(acc[1][m], pm);
+        fx_add(acc[1][m], t.pm);
+        if (!terms_in(p, t, b)) odd |= 1u << m;
         // comparisons of magnitudes on their IEEE bit patterns (exact for
         // non-negative doubles; NaN compares as in the reference: never below)
-        const long long bdeno = __double_as_longlong(deno) & 0x7fffffffffffffffll;
+        const long long bdeno = __double_as_longlong(t.deno) & 0x7fffffffffffffffll;
         if (p.ywdeg && !(bdeno > kBits005 && bdeno <= kBitsInf)) {
-          const long long beim = __double_as_longlong(b * cx) & 0x7fffffffffffffffll;
+          const long long beim = __double_as_longlong(b * t.c) & 0x7fffffffffffffffll;
           if (!(beim < kBits1em6)) ydeg = true;
         }
-        double xim = fabs(cx);
-        if (p.ysele) xim = fabs(b * cx);
+        double xim = fabs(t.c);
+        if (p.ysele) xim = fabs(b * t.c);
         if (lt_nonneg(xim, p.teste[m])) dpivot = max_nonneg(dpivot, xim);
         if (p.ymoyen) {
-          if (p.taum[m] != 1.0) xim *= p.taum[m];
+          if (__double_as_longlong(p.taum[m]) != kBitsOne) xim *= p.taum[m];
           vil[m] = xim;
           xam = max_nonneg(xam, xim);
         }
       }
+      // histogram (cip/isto.f; pert1 calls it always, diexcit only if ymoyen)
+      const bool all = __double_as_longlong(p.teseff) <= 0;
+      const bool hist = live && (!(flag & kMD2) || p.ymoyen) &&
+                        (all || __double_as_longlong(xam) >= __double_as_longlong(p.teseff));
+      const int cls = hist ? hist_class_hi(p, xam) : kNClass;
+      auto class_of = [&](int m) { return hist && (all || !lt_nonneg(vil[m], p.teseff)) ? cls : kNClass; };
       if (live) {
         ietat += (unsigned long long)(long long)(nmul + 1);
         nproc += 1u;
-        // histogram (cip/isto.f; pert1 calls it always, diexcit only if ymoyen)
-        const bool all = p.teseff <= 0.0;
-        const bool hist = (!(flag & kMD2) || p.ymoyen) &&
-                          (all || __double_as_longlong(xam) >= __double_as_longlong(p.teseff));
-        int cls = kNClass;
-        if (hist) {
-          cls = hist_class_hi(p, xam);
-          atomicAdd(&sh.hn[wid][cls], (uint32_t)(1 + nmul));
-        }
+        if (hist) atomicAdd(&sh.hn[wid][cls], (uint32_t)(1 + nmul));
 #pragma unroll
         for (int m = 0; m < R; ++m) {
           if (m >= p.metat) continue;
-          const bool in = hist && (all || !lt_nonneg(vil[m], p.teseff));
-          const int ct = in ? cls : kNClass;
-          if (in) atomicAdd(&sh.hn[wid][(kNClass + 1) * (1 + m) + (R == 1 ? cls : hist_class_hi(p, vil[m]))], (uint32_t)(1 + nmul));
-          double t0 = tmp[m], t1 = tvp[m];
-          if (!(fx_fits(t0) && fx_fits(t1))) {
-            if (!fx_fits(t0)) { fx_big(p, fx_tab(0, ct, m), t0); t0 = 0.0; }
-            if (!fx_fits(t1)) { fx_big(p, fx_tab(1, ct, m), t1); t1 = 0.0; }
+          const int ct = class_of(m);
+          if (ct < kNClass)
+            atomicAdd(&sh.hn[wid][(kNClass + 1) * (1 + m) + (R == 1 ? cls : hist_class_hi(p, vil[m]))], (uint32_t)(1 + nmul));
+          uint2 top2 = top[ct][m];
+          Fx f = fx_of(tab[ct][m][0], top2.x);
+          fx_add(f, tmp[m]);
+          tab[ct][m][0] = make_uint4(f.w[0], f.w[1], f.w[2], f.w[3]);
+          top2.x = f.w[4];
+          if (p.yen) {
+            f = fx_of(tab[ct][m][1], top2.y);
+            fx_add(f, tvp[m]);
+            tab[ct][m][1] = make_uint4(f.w[0], f.w[1], f.w[2], f.w[3]);
+            top2.y = f.w[4];
           }
-          fx_add(tab[ct][0][m], t0);
-          if (p.yen) fx_add(tab[ct][1][m], t1);
+          top[ct][m] = top2;
+        }
+      }
+      if (__any_sync(kFull, odd != 0u)) {
+#pragma unroll
+        for (int m = 0; m < R; ++m) {
+          if (m >= p.metat) continue;
+          const bool mine = (odd >> m) & 1u;
+          odd_terms(p, mine, m, class_of(m), mine ? la.cand.b[m * la.cand.cap + s] : 0.0, wgt, hmpi, hvpi);
         }
       }
       if (ydeg) xam = 1.0;
       // unit-60 record (pie.f): counted; its values stay at the candidate's slot
       // until the unit is done
       const bool sel = live && p.ymoyen &&
-                       (p.tau < 0.0 || __double_as_longlong(xam) > (__double_as_longlong(p.tau) & 0x7fffffffffffffffll));
+                       (below_zero(p.tau) || __double_as_longlong(xam) > (__double_as_longlong(p.tau) & 0x7fffffffffffffffll));
       if (sel) {
         ++nsel;
         if (p.rec_mode) {
