@@ -152,19 +152,15 @@ __device__ __forceinline__ bool recip_ok(double d) {
 struct Terms {
   double mp, vp, b, pm, pv, c, deno;
 };
-__device__ __noinline__ Terms terms_by_division(double b, double wgt, double dmp, double dvp, double db, bool en) {
+__device__ __noinline__ Terms terms_by_division(double b, double wgt, double dmp, double dvp, double db) {
   Terms t;
   const double cm = b / dmp;
   t.mp = (b * cm) * wgt;
   t.pm = cm * cm * wgt;
-  t.c = cm;
-  t.vp = t.b = t.pv = 0.0;
-  if (en) {
-    t.c = b / dvp;
-    t.vp = (b * t.c) * wgt;
-    t.pv = t.c * t.c * wgt;
-    t.b = (b * (b / db)) * wgt;
-  }
+  t.c = b / dvp;
+  t.vp = (b * t.c) * wgt;
+  t.pv = t.c * t.c * wgt;
+  t.b = (b * (b / db)) * wgt;
   return t;
 }
 // the terms of root m for a coupling b
@@ -183,20 +179,18 @@ __device__ __forceinline__ Terms terms_of(const Params& p, int m, double b, doub
       t.pv = t.vp * rv;
       t.c = b * rv;
     } else {  // a denominator at (or near) zero or huge
-      t = terms_by_division(b, wgt, dmp, dvp, db, true);
+      t = terms_by_division(b, wgt, dmp, dvp, db);
     }
     t.deno = dvp;
     return t;
   }
-  if (recip_ok(dmp)) {
-    const double rm = recip(dmp);
-    t.c = b * rm;
-    t.mp = (b * t.c) * wgt;
-    t.pm = t.mp * rm;
-    t.vp = t.b = t.pv = 0.0;
-  } else {
-    t = terms_by_division(b, wgt, dmp, 0.0, 0.0, false);
-  }
+  // one quotient, the coefficient that the selection looks at: by division, as
+  // every other quotient of the reference (b times the reciprocal is off by up to
+  // 1.4 ulp)
+  t.c = b / dmp;
+  t.mp = (b * t.c) * wgt;
+  t.pm = t.c * t.c * wgt;
+  t.vp = t.b = t.pv = 0.0;
   t.deno = dmp;
   return t;
 }
