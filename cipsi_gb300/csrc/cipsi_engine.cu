@@ -9,6 +9,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -283,8 +284,12 @@ struct cipsi_ctx {
   size_t plan_cap = 0;
   std::vector<unsigned char> hplan;
   int nunits = 0;
-  unsigned char* dcand = nullptr;  // candidate buffer of cand_cap slots
-  long long cand_cap = 0;
+  // candidate buffer of runs whose slots take up to kCandOwnBytes; those of
+  // larger runs go through the device's (CandArena): cand_shared, of the last
+  // run; cand_user: this context counts among its users
+  unsigned char* dcand = nullptr;
+  size_t cand_bytes = 0, cand_limit = 0;  // cand_limit: cipsi_set_candidate_bytes
+  bool cand_shared = false, cand_user = false;
   int32_t* dnb_j = nullptr;
   uint64_t* dnb_em = nullptr;
   uint64_t* dlr_ent = nullptr;
@@ -411,6 +416,49 @@ void dfree(T*& p) {
   p = nullptr;
 }
 
+// The candidate buffer of large runs, one per device for all contexts of the
+// process: such a run fills the device by itself, so that taking turns costs
+// nothing, and a program that keeps hundreds of contexts keeps one buffer.
+// `busy` is recorded after a part's kernels; whoever enqueues the next part, on
+// whatever stream, waits for it there, holding the lock.  The last user frees
+// the buffer.
+struct CandArena {
+  std::mutex mu;
+  unsigned char* base = nullptr;
+  size_t bytes = 0;
+  cudaEvent_t busy = nullptr;
+  int users = 0;
+};
+constexpr int kMaxDevices = 64;
+CandArena g_arena[kMaxDevices];
+
+void leave_arena(cipsi_ctx* ctx) {
+  if (!ctx->cand_user) return;
+  CandArena& a = g_arena[ctx->device];
+  std::lock_guard<std::mutex> hold(a.mu);
+  ctx->cand_user = false;
+  if (--a.users > 0) return;
+  if (a.base) cudaFree(a.base);  // (waits for the device)
+  if (a.busy) cudaEventDestroy(a.busy);
+  a.base = nullptr;
+  a.bytes = 0;
+  a.busy = nullptr;
+}
+
+// `want` bytes of device memory, or half as often as it takes down to `need`
+cudaError_t alloc_down(unsigned char** p, size_t need, size_t want, size_t* got) {
+  for (size_t b = std::max(want, need);; b = std::max(b / 2, need)) {
+    const cudaError_t e = cudaMalloc((void**)p, b);
+    if (e == cudaSuccess) {
+      *got = b;
+      return e;
+    }
+    *p = nullptr;
+    cudaGetLastError();
+    if (e != cudaErrorMemoryAllocation || b == need) return e;
+  }
+}
+
 int roots_pad(int mt) { return mt <= 1 ? 1 : mt <= 2 ? 2 : mt <= 4 ? 4 : 8; }
 
 // the forward form of k_pt2_one of class (W, R)
@@ -489,6 +537,7 @@ void cipsi_ctx_destroy(cipsi_ctx* ctx) {
   dfree(ctx->dS); dfree(ctx->dygen); dfree(ctx->dyef); dfree(ctx->dnesp); dfree(ctx->dc);
   dfree(ctx->deri); dfree(ctx->dpairtab); dfree(ctx->dntttt); dfree(ctx->dF); dfree(ctx->dJ);
   dfree(ctx->dK); dfree(ctx->djx); dfree(ctx->dfmpb); dfree(ctx->dorbsym); dfree(ctx->dplan); dfree(ctx->dcand);
+  leave_arena(ctx);
   dfree(ctx->deri64);
   dfree(ctx->deri_w);
   dfree(ctx->dnb_j); dfree(ctx->dnb_em); dfree(ctx->dlr_ent); dfree(ctx->dgen_part);
@@ -930,11 +979,12 @@ int fwd_blocks_per_sm(int W, int R, int ctas) {
   return ctas == 0 ? fit : std::min(fit, ctas);
 }
 
-// Bytes of a candidate's slot, and the most that one buffer takes: runs with
-// more slots go through it in parts (a few GB: enough units for every SM even
-// at 120 orbitals, where a unit has 200,000 slots).
+// Bytes of a candidate's slot, the most that the device's candidate buffer
+// takes (runs with more slots go through it in parts), and the most that a
+// context keeps for itself.
 constexpr size_t cand_slot_bytes(int R) { return 8 * (size_t)R + 8 + 8 + 4 + 4; }
 constexpr size_t kCandMaxBytes = (size_t)8 << 30;
+constexpr size_t kCandOwnBytes = (size_t)256 << 20;
 CandBuf cand_views(unsigned char* base, long long cap, int R) {
   CandBuf c;
   c.cap = cap;
@@ -944,6 +994,76 @@ CandBuf cand_views(unsigned char* base, long long cap, int R) {
   c.code = reinterpret_cast<uint32_t*>(c.vp + cap);
   c.meta = c.code + cap;
   return c;
+}
+
+// A share of the device's free memory for a candidate buffer of up to `want`
+// bytes: a quarter, the rest stays for records and for others
+size_t cand_share(size_t want) {
+  size_t fr = 0, tot = 0;
+  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+    cudaGetLastError();
+    return want;
+  }
+  return std::min(want, fr / 4);
+}
+
+// Room for a run's candidates: *cap slots, all of them or enough for the
+// largest unit at least.
+int reserve_cand(cipsi_ctx* ctx, long long max_slots, long long all_slots, long long* cap) {
+  const size_t sb = cand_slot_bytes(roots_pad(ctx->d.metat));
+  auto bytes = [&](long long slots) { return (size_t)((std::max(slots, 1ll) + 63) / 64 * 64) * sb; };
+  const size_t need = bytes(max_slots), all = bytes(all_slots);
+  const size_t own = ctx->cand_limit ? ctx->cand_limit : kCandOwnBytes;
+  ctx->cand_shared = !ctx->cand_limit && all > own;
+  // larger when it has to be, or when the memory for it is free
+  auto grows = [&](size_t bytes, size_t want) {
+    return bytes < need || (bytes < want && cand_share(want) > bytes);
+  };
+  cudaError_t e = cudaSuccess;
+  size_t have;
+  if (!ctx->cand_shared) {
+    const size_t want = std::max(need, std::min(all, own));
+    if (grows(ctx->cand_bytes, want)) {
+      dfree(ctx->dcand);
+      ctx->cand_bytes = 0;
+      e = alloc_down(&ctx->dcand, need, cand_share(want), &ctx->cand_bytes);
+    }
+    have = ctx->cand_bytes;
+  } else {
+    CandArena& a = g_arena[ctx->device];
+    std::lock_guard<std::mutex> hold(a.mu);
+    if (!ctx->cand_user) {
+      if (!a.busy) CK(cudaEventCreateWithFlags(&a.busy, cudaEventDisableTiming));
+      ctx->cand_user = true;
+      ++a.users;
+    }
+    const size_t want = std::min(all, kCandMaxBytes);
+    if (grows(a.bytes, want)) {
+      const size_t least = std::max(need, a.bytes);  // runs under way count on what it was
+      CK(cudaEventSynchronize(a.busy));
+      dfree(a.base);
+      a.bytes = 0;
+      e = alloc_down(&a.base, least, cand_share(want), &a.bytes);
+    }
+    have = a.bytes;
+  }
+  if (e != cudaSuccess)
+    return fail(ctx, CIPSI_ERR_CUDA,
+                "candidate buffer of " + std::to_string(need) + " bytes: " + cudaGetErrorString(e));
+  *cap = (long long)(have / sb) / 64 * 64;
+  return CIPSI_OK;
+}
+
+// Blocks per work unit where `cap` slots at a time go through the buffer: units
+// of `ub`, or as many fewer as it takes to have three for every CTA (a part ends
+// with its last unit: an active space of 120 orbitals, two roots, through 1 GB
+// takes 111 ms, and 173 with units of 16 blocks, of which a part has half as many
+// as CTAs; through 8 GB 67 ms).
+int fitted_blocks(int ub, const RunPlan& pl, long long cap, int ctas) {
+  const long long nu = (long long)pl.ug.size();
+  if (cap >= pl.all_slots || nu == 0) return ub;
+  const long long units = cap / std::max(1ll, pl.all_slots / nu);
+  return units >= 3ll * ctas ? ub : (int)std::max(1ll, ub * units / (3ll * ctas));
 }
 
 // Units in parts whose slots add up to at most cap (a unit's own slots fit):
@@ -1102,18 +1222,6 @@ int prepare_run(cipsi_ctx* ctx, const RunPlan& pl, const std::vector<long long>*
     ++ctx->buf_gen;
     CK(cudaMalloc(&ctx->dscan_total, sizeof(unsigned long long)));
   }
-  return CIPSI_OK;
-}
-
-// The candidate buffer, for at least `slots` slots.
-int ensure_cand(cipsi_ctx* ctx, long long slots) {
-  if (slots <= ctx->cand_cap && ctx->dcand) return CIPSI_OK;
-  ++ctx->buf_gen;
-  dfree(ctx->dcand);
-  ctx->cand_cap = 0;
-  const long long cap = std::max<long long>((slots + 63) / 64 * 64, 64);
-  CK(cudaMalloc(&ctx->dcand, (size_t)cap * cand_slot_bytes(roots_pad(ctx->d.metat))));
-  ctx->cand_cap = cap;
   return CIPSI_OK;
 }
 
@@ -1287,7 +1395,6 @@ LaunchArgs plan_args(const cipsi_ctx* ctx, const Params& p, int u0, int u1) {
   LaunchArgs la{};
   la.unit_slot = reinterpret_cast<const long long*>(ctx->dplan) + u0;
   la.unit_nslots = reinterpret_cast<const int32_t*>(ctx->dplan + (size_t)ctx->nunits * 8) + 3 * (size_t)ctx->nunits + u0;
-  la.cand = cand_views(ctx->dcand, ctx->cand_cap, roots_pad(ctx->d.metat));
   la.nunits = u1 - u0;
   la.work = p.work;
   return la;
@@ -1303,6 +1410,34 @@ Params part_params(const Params& p, int u0) {
   return q;
 }
 
+// both forward kernels over units [u0, u1) of the context's plan, `slots` in all
+int launch_part(cipsi_ctx* ctx, const Params& p, int u0, int u1, int grid, int sms, long long slots) {
+  const int R = roots_pad(ctx->d.metat);
+  const size_t sb = cand_slot_bytes(R);
+  LaunchArgs la = plan_args(ctx, p, u0, u1);
+  auto launch = [&](unsigned char* base, size_t bytes) {
+    la.cand = cand_views(base, (long long)(bytes / sb) / 64 * 64, R);
+    return slots <= la.cand.cap ? launch_forward<false>(part_params(p, u0), la, ctx->W, R, grid, sms, slots, ctx->stream)
+                                : cudaErrorMemoryAllocation;
+  };
+  cudaError_t e;
+  if (!ctx->cand_shared) {
+    e = launch(ctx->dcand, ctx->cand_bytes);
+  } else {
+    CandArena& a = g_arena[ctx->device];
+    std::lock_guard<std::mutex> hold(a.mu);
+    e = cudaStreamWaitEvent(ctx->stream, a.busy, 0);
+    if (e == cudaSuccess) {
+      e = launch(a.base, a.bytes);
+      const cudaError_t r = cudaEventRecord(a.busy, ctx->stream);  // whatever was enqueued
+      if (e == cudaSuccess) e = r;
+    }
+  }
+  if (e != cudaSuccess)
+    return fail(ctx, CIPSI_ERR_CUDA, std::string("k_cand / k_pt2 launch: ") + cudaGetErrorString(e));
+  return CIPSI_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1313,6 +1448,16 @@ int cipsi_set_tuning(cipsi_ctx* ctx, int32_t r_chunk, int32_t ctas_per_sm) {
   if (ctas_per_sm < 0 || ctas_per_sm > 2) return fail(ctx, CIPSI_ERR_ARG, "ctas_per_sm must be 0, 1 or 2");
   ctx->tune_r_chunk = r_chunk;
   ctx->tune_ctas = ctas_per_sm;
+  return CIPSI_OK;
+}
+
+int cipsi_set_candidate_bytes(cipsi_ctx* ctx, int64_t bytes) {
+  if (!ctx) return CIPSI_ERR_ARG;
+  if (bytes < 0) return fail(ctx, CIPSI_ERR_ARG, "candidate bytes must not be negative");
+  if (ctx->pending) return fail(ctx, CIPSI_ERR_STATE, "an asynchronous run is pending: fetch its result first");
+  ctx->cand_limit = (size_t)bytes;
+  dfree(ctx->dcand);
+  ctx->cand_bytes = 0;
   return CIPSI_OK;
 }
 
@@ -1364,17 +1509,19 @@ int cipsi_run_pt2_async(cipsi_ctx* ctx, const cipsi_opts* o) {
   RunPlan pl;
   const int ub = unit_blocks(ctx->tune_r_chunk, run_blocks(ctx, o), dev_sms);
   plan_run(ctx, o, ub, std::min(ub, kLowChunk), pl);
+  const int ctas = dev_sms * fwd_blocks_per_sm(W, roots_pad(mt), ctx->tune_ctas);
+  long long cap = 0;
+  rc = reserve_cand(ctx, pl.max_slots, pl.all_slots, &cap);
+  if (rc) return rc;
+  const int fit = fitted_blocks(ub, pl, cap, ctas);
+  if (fit < ub) plan_run(ctx, o, fit, std::min(fit, kLowChunk), pl = RunPlan{});
   const int nunits = (int)pl.ug.size();
-  const int R = roots_pad(mt);
-  const int grid = std::max(1, std::min(nunits, dev_sms * fwd_blocks_per_sm(W, R, ctx->tune_ctas)));
+  const int grid = std::max(1, std::min(nunits, ctas));
   rc = ensure_neighbour_scratch(ctx, grid);
   if (rc) return rc;
-  const long long cap = std::max(pl.max_slots, (long long)(kCandMaxBytes / cand_slot_bytes(R)));
   std::vector<long long> slot0;
   const std::vector<int> cut = cut_units(pl.uslots, cap, slot0);
   rc = prepare_run(ctx, pl, &slot0, ctx->stream);
-  if (rc) return rc;
-  rc = ensure_cand(ctx, std::min(cap, pl.all_slots));
   if (rc) return rc;
   CK(cudaMemsetAsync(ctx->dcounters, 0, kZeroWords * sizeof(unsigned long long), ctx->stream));
 
@@ -1384,21 +1531,17 @@ int cipsi_run_pt2_async(cipsi_ctx* ctx, const cipsi_opts* o) {
 
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   if (nunits > 0) {
-    cudaError_t e = cudaSuccess;
     for (size_t c = 0; c + 1 < cut.size(); ++c) {
       const int u0 = cut[c], u1 = cut[c + 1];
       if (c) CK(cudaMemsetAsync(p.work, 0, 2 * sizeof(int), ctx->stream));
-      const LaunchArgs la = plan_args(ctx, p, u0, u1);
-      e = launch_forward<false>(part_params(p, u0), la, W, R, std::min(grid, u1 - u0), dev_sms,
-                                slot0[u1 - 1] + pl.uslots[u1 - 1], ctx->stream);
-      if (e != cudaSuccess)
-        return fail(ctx, CIPSI_ERR_CUDA, std::string("k_cand / k_pt2 launch: ") + cudaGetErrorString(e));
+      rc = launch_part(ctx, p, u0, u1, std::min(grid, u1 - u0), dev_sms, slot0[u1 - 1] + pl.uslots[u1 - 1]);
+      if (rc) return rc;
     }
     CK(cudaEventRecord(ctx->evk, ctx->stream));
     ctx->last_launches = 2 * (long long)(cut.size() - 1) + 3;  // and the unit scan, the gather, k_finish
     GatherArgs ga{};
     record_target(ctx, ga);
-    e = enqueue_gather(ctx, p, 0, nunits, 0, ga, ctx->stream, dev_sms);
+    const cudaError_t e = enqueue_gather(ctx, p, 0, nunits, 0, ga, ctx->stream, dev_sms);
     if (e != cudaSuccess) return fail(ctx, CIPSI_ERR_CUDA, std::string("record gather: ") + cudaGetErrorString(e));
   } else {
     CK(cudaEventRecord(ctx->evk, ctx->stream));
@@ -1626,10 +1769,7 @@ int cipsi_run_pt2_stream(cipsi_ctx* ctx, const cipsi_opts* o, int64_t chunk_reco
   RunPlan pl;
   const int ub = unit_blocks(ctx->tune_r_chunk, run_blocks(ctx, o), dev_sms);
   plan_run(ctx, o, ub, std::min(ub, kLowChunk), pl);
-  const int nunits = (int)pl.ug.size();
-  const int R = roots_pad(mt);
-  const int grid = std::max(1, std::min(nunits, dev_sms * fwd_blocks_per_sm(W, R, ctx->tune_ctas)));
-  if ((rc = ensure_neighbour_scratch(ctx, grid))) return rc;
+  const int ctas = dev_sms * fwd_blocks_per_sm(W, roots_pad(mt), ctx->tune_ctas);
   // chunk capacity: what was asked, else what about half the free device
   // memory holds (pool + two record buffers), at most 2^29 records; at
   // least the largest unit's slots
@@ -1651,11 +1791,17 @@ int cipsi_run_pt2_stream(cipsi_ctx* ctx, const cipsi_opts* o, int64_t chunk_reco
   }
   cap = std::max(cap, std::max<long long>(pl.max_slots, 1024));
   // a chunk's candidates have to fit their buffer too
-  cap = std::min(cap, std::max(std::max<long long>(pl.max_slots, 1024), (long long)(kCandMaxBytes / cand_slot_bytes(R))));
+  long long cand_cap = 0;
+  if ((rc = reserve_cand(ctx, pl.max_slots, std::min(cap, pl.all_slots), &cand_cap))) return rc;
+  cap = std::min(cap, cand_cap);
+  const int fit = fitted_blocks(ub, pl, cap, ctas);
+  if (fit < ub) plan_run(ctx, o, fit, std::min(fit, kLowChunk), pl = RunPlan{});
+  const int nunits = (int)pl.ug.size();
+  const int grid = std::max(1, std::min(nunits, ctas));
+  if ((rc = ensure_neighbour_scratch(ctx, grid))) return rc;
   std::vector<long long> slot0;
   const std::vector<int> cut = cut_units(pl.uslots, cap, slot0);
   if ((rc = prepare_run(ctx, pl, &slot0, ctx->stream))) return rc;
-  if ((rc = ensure_cand(ctx, std::min(cap, pl.all_slots)))) return rc;
   if (ctx->pool_cap < cap && (rc = grow_pool(ctx, cap))) return rc;
   const long long hb_cap = std::min<long long>(cap, 1ll << 24);
   if ((rc = ensure_stream_buffers(ctx, cap, fn != nullptr, hb_cap))) return rc;
@@ -1738,12 +1884,9 @@ int cipsi_run_pt2_stream(cipsi_ctx* ctx, const cipsi_opts* o, int64_t chunk_reco
     if (c >= 2 && fn) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_copied[b], 0));
     // work counter and pool count (next to each other)
     CK(cudaMemsetAsync(p.work, 0, 2 * sizeof(unsigned long long), ctx->stream));
-    const LaunchArgs la = plan_args(ctx, p, u0, u1);
     CK(cudaEventRecord(kev[2 * c], ctx->stream));
-    cudaError_t e = launch_forward<false>(part_params(p, u0), la, W, R, std::min(grid, u1 - u0), dev_sms,
-                                          slot0[u1 - 1] + pl.uslots[u1 - 1], ctx->stream);
-    if (e != cudaSuccess)
-      return fail(ctx, CIPSI_ERR_CUDA, std::string("k_cand / k_pt2 launch: ") + cudaGetErrorString(e));
+    if ((rc = launch_part(ctx, p, u0, u1, std::min(grid, u1 - u0), dev_sms, slot0[u1 - 1] + pl.uslots[u1 - 1])))
+      return rc;
     CK(cudaEventRecord(kev[2 * c + 1], ctx->stream));
     GatherArgs ga{};
     ga.out_bits = ctx->dout_bits[b];
@@ -1751,7 +1894,7 @@ int cipsi_run_pt2_stream(cipsi_ctx* ctx, const cipsi_opts* o, int64_t chunk_reco
     ga.out_xam = ctx->dout_xam[b];
     ga.out_evp = ctx->dout_evp[b];
     ga.out_cap = ctx->out_cap;
-    e = enqueue_gather(ctx, p, u0, u1, 0, ga, ctx->stream, dev_sms);
+    const cudaError_t e = enqueue_gather(ctx, p, u0, u1, 0, ga, ctx->stream, dev_sms);
     if (e != cudaSuccess) return fail(ctx, CIPSI_ERR_CUDA, std::string("record gather: ") + cudaGetErrorString(e));
     CK(cudaMemcpyAsync(&hcnt[2 * c], ctx->dscan_total, 8, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(&hcnt[2 * c + 1], p.pool_count, 8, cudaMemcpyDeviceToHost, ctx->stream));
@@ -2086,7 +2229,7 @@ struct cipsi_batch {
     // the units' slots and the candidate buffer, shared by the class's geometries
     unsigned char* dunit_slot = nullptr;
     unsigned char* dcand = nullptr;
-    long long cand_cap = 0;
+    size_t cand_bytes = 0;
     std::vector<int> cut;
     std::vector<long long> part_slots;
     cudaStream_t st = nullptr;
@@ -2222,12 +2365,17 @@ int cipsi_batch_create(cipsi_batch** out, cipsi_ctx* const* ctxs, int32_t n, con
       max_slots = std::max(max_slots, x);
       all_slots += x;
     }
-    const long long cap = std::max(max_slots, (long long)(kCandMaxBytes / cand_slot_bytes(c.R)));
+    // the graph holds its address, so the buffer is the batch's own
+    const size_t sb = cand_slot_bytes(c.R);
+    auto bytes = [&](long long x) { return (size_t)((std::max(x, 1ll) + 63) / 64 * 64) * sb; };
+    size_t want = std::min(bytes(all_slots), kCandMaxBytes);
+    for (int i : c.geos)
+      if (ctxs[i]->cand_limit) want = std::min(want, ctxs[i]->cand_limit);
+    BCK(alloc_down(&c.dcand, bytes(max_slots), cand_share(want), &c.cand_bytes));
+    const long long cap = (long long)(c.cand_bytes / sb) / 64 * 64;
     std::vector<long long> slot0;
     c.cut = cut_units(slots, cap, slot0);
     for (size_t q = 0; q + 1 < c.cut.size(); ++q) c.part_slots.push_back(slot0[c.cut[q + 1] - 1] + slots[c.cut[q + 1] - 1]);
-    c.cand_cap = std::max<long long>(64, (std::min(cap, all_slots) + 63) / 64 * 64);
-    BCK(cudaMalloc(&c.dcand, (size_t)c.cand_cap * cand_slot_bytes(c.R)));
     {
       const std::vector<int32_t> ns(slots.begin(), slots.end());
       BCK(cudaMalloc(&c.dunit_slot, std::max<size_t>(12 * slots.size(), 64)));
@@ -2281,7 +2429,7 @@ int cipsi_batch_create(cipsi_batch** out, cipsi_ctx* const* ctxs, int32_t n, con
       LaunchArgs la{};
       la.unit_slot = reinterpret_cast<const long long*>(c.dunit_slot) + u0;
       la.unit_nslots = reinterpret_cast<const int32_t*>(c.dunit_slot + 8 * (size_t)c.nunits) + u0;
-      la.cand = cand_views(c.dcand, c.cand_cap, c.R);
+      la.cand = cand_views(c.dcand, (long long)(c.cand_bytes / cand_slot_bytes(c.R)) / 64 * 64, c.R);
       la.nunits = u1 - u0;
       la.work = c.dwork;
       la.geo = b->dgeo;

@@ -99,6 +99,7 @@ def _lib():
         "cipsi_run_pt2": ([P, ctypes.POINTER(Opts), ctypes.POINTER(Result)], ctypes.c_int),
         "cipsi_run_pt2_async": ([P, ctypes.POINTER(Opts)], ctypes.c_int),
         "cipsi_set_tuning": ([P, ctypes.c_int32, ctypes.c_int32], ctypes.c_int),
+        "cipsi_set_candidate_bytes": ([P, ctypes.c_int64], ctypes.c_int),
         "cipsi_set_selection_sink": ([P, P, P, P, P, ctypes.c_int64], ctypes.c_int),
         "cipsi_fetch_result": ([P, ctypes.POINTER(Result)], ctypes.c_int),
         "cipsi_selection_get": ([P, ctypes.c_int64, ctypes.c_int64, P, P, P, P, P, P], ctypes.c_int),
@@ -234,6 +235,11 @@ class Context:
 
     def set_tuning(self, r_chunk: int = 6, ctas_per_sm: int = 0):
         self._check(self.lib.cipsi_set_tuning(self._c, r_chunk, ctas_per_sm), "set_tuning")
+
+    def set_candidate_bytes(self, limit: int = 0):
+        """Bound the device memory between the two forward kernels
+        (cipsi_set_candidate_bytes); 0: the default."""
+        self._check(self.lib.cipsi_set_candidate_bytes(self._c, limit), "set_candidate_bytes")
 
     def set_integrals_f64store(self, itsym, its, F, J, K, ij0, ntttt, eri):
         """Integrals with (pq|rs) kept in FP64 on the device."""

@@ -164,6 +164,20 @@ int cipsi_run_pt2(cipsi_ctx* ctx, const cipsi_opts* opts, cipsi_result* res);
    cipsi_gb300.tune (Python) picks both by timing a generator sample. */
 int cipsi_set_tuning(cipsi_ctx* ctx, int32_t r_chunk, int32_t ctas_per_sm);
 
+/* Device memory between the two forward kernels (no counterpart in the
+   reference; results do not depend on it).  A run leaves 24 bytes and 8 per
+   root (1, 2, 4 or 8) for each of its candidates in a buffer, and goes through
+   it in parts where they do not all fit.  Runs that need up to 256 MiB keep a
+   buffer of their context's own.  Larger ones share one of up to 8 GiB per
+   device among the process's contexts, taking turns on the device; the last
+   context that used it frees it.  Both take at most a quarter of the free
+   memory, and less when that fails, down to what one work unit needs.
+     bytes  0 (default): as above.  Else: a buffer of the context's own of at
+            most this size (but room for one work unit), for runs and, as the
+            smallest of its members' limits, for a batch.
+   CIPSI_ERR_STATE while an asynchronous run is pending. */
+int cipsi_set_candidate_bytes(cipsi_ctx* ctx, int64_t bytes);
+
 /* Unit-60 records straight into caller memory (no counterpart in the
    reference): pinned host arrays (cudaHostAlloc / cudaHostRegister) of
    `capacity` records, laid out as cipsi_selection_raw returns them (bits
