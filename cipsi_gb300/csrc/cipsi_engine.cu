@@ -1177,15 +1177,17 @@ void set_plan(Params& p, const unsigned char* d, int nunits, int ngen) {
 }
 
 // Device buffers of one run on ctx (counters, histogram, records; the plan,
-// uploaded on stream st, unless the caller keeps it: slot0 null), sized for it.
-int prepare_run(cipsi_ctx* ctx, const RunPlan& pl, const std::vector<long long>* slot0, cudaStream_t st) {
+// uploaded on stream st, unless the caller keeps it: slot0 null), sized for it;
+// the unit tables for `units` at least.  (buf_gen counts what a batch's graph
+// refers to: not the plan.)
+int prepare_run(cipsi_ctx* ctx, const RunPlan& pl, const std::vector<long long>* slot0, cudaStream_t st,
+                int units = 0) {
   const int nunits = (int)pl.ug.size();
   if (slot0) {
     ctx->hplan.clear();
     pack_plan(pl, *slot0, ctx->hplan);
     const size_t bytes = ctx->hplan.size();
     if (bytes > ctx->plan_cap || !ctx->dplan) {
-      ++ctx->buf_gen;
       dfree(ctx->dplan);
       ctx->plan_cap = 0;
       CK(cudaMalloc(&ctx->dplan, std::max<size_t>(bytes, 64)));
@@ -1210,13 +1212,14 @@ int prepare_run(cipsi_ctx* ctx, const RunPlan& pl, const std::vector<long long>*
     const int rc = grow_sel(ctx, 1 << 20);
     if (rc) return rc;
   }
-  if (nunits > ctx->unit_tab_cap) {
+  units = std::max(units, nunits);
+  if (units > ctx->unit_tab_cap) {
     ++ctx->buf_gen;
     dfree(ctx->dunit_pool); dfree(ctx->dunit_nsel); dfree(ctx->dunit_out);
-    CK(cudaMalloc(&ctx->dunit_pool, (size_t)nunits * sizeof(long long)));
-    CK(cudaMalloc(&ctx->dunit_nsel, (size_t)nunits * sizeof(int32_t)));
-    CK(cudaMalloc(&ctx->dunit_out, (size_t)nunits * sizeof(long long)));
-    ctx->unit_tab_cap = nunits;
+    CK(cudaMalloc(&ctx->dunit_pool, (size_t)units * sizeof(long long)));
+    CK(cudaMalloc(&ctx->dunit_nsel, (size_t)units * sizeof(int32_t)));
+    CK(cudaMalloc(&ctx->dunit_out, (size_t)units * sizeof(long long)));
+    ctx->unit_tab_cap = units;
   }
   if (!ctx->dscan_total) {
     ++ctx->buf_gen;
@@ -1338,6 +1341,11 @@ int lrw_entries(int ncf) { return std::min(kLrWarpG, ncf); }
 int ensure_neighbour_scratch(cipsi_ctx* ctx, int grid) {
   if ((size_t)grid <= ctx->scratch_blocks && ctx->dnb_j) return CIPSI_OK;
   const int ncf = ctx->d.ncf;
+  // two CTAs per SM, the most that any run launches: a later run with more units
+  // finds room (and a batch of this context stays valid)
+  int sms = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+  grid = std::max(grid, 2 * sms);
   ++ctx->buf_gen;
   dfree(ctx->dnb_j); dfree(ctx->dnb_em); dfree(ctx->dlr_ent);
   dfree(ctx->dlr_e); dfree(ctx->dlrw_e); dfree(ctx->dlrw_jh);
@@ -2329,7 +2337,12 @@ int cipsi_batch_create(cipsi_batch** out, cipsi_ctx* const* ctxs, int32_t n, con
     // the plan is the batch's own: the context's is replaced by every plain run
     plan_at[i] = pack_plan(pl, std::vector<long long>(pl.ug.size(), 0), hplan);
     plan_gens[i] = (int)pl.gens.size();
-    if (prepare_run(ctx, pl, nullptr, b->stream)) return bfail(b, CIPSI_ERR_CUDA, "context " + std::to_string(i) + ": " + ctx->err);
+    // a batch's units are larger than those of its contexts' own runs, which
+    // should not outgrow the unit tables
+    RunPlan own;
+    const int oub = unit_blocks(ctx->tune_r_chunk, run_blocks(ctx, &opts[i]), dev_sms);
+    if (oub < ub) plan_run(ctx, &opts[i], oub, std::min(oub, kLowChunk), own);
+    if (prepare_run(ctx, pl, nullptr, b->stream, (int)own.ug.size())) return bfail(b, CIPSI_ERR_CUDA, "context " + std::to_string(i) + ": " + ctx->err);
     fill_params(ctx, &opts[i], pl, P[i]);
     uslots[i] = pl.uslots;
     work[i] = (long long)pl.ug.size() * ctx->d.ncf;
