@@ -298,16 +298,16 @@ __global__ void __launch_bounds__(kThreads, kEpiCtas<R>) k_pt2(Params p0, Launch
   // words of both another)
   uint4 tab[kNClass + 1][R][2];
   uint2 top[kNClass + 1][R];
+  // classes that the lane has terms of; the rows of the others are not touched
+  // (all of them, of all resident threads, are 50 MB to clear and to read again,
+  // 270 with eight roots: 33 and 140 us of a run that has few perturbers)
+  unsigned held = 0u;
   Fx acc[3][R];
   unsigned long long ietat = 0;
   unsigned int nproc = 0, nsel = 0;
   double dpivot = 0.0;
   auto zero_sums = [&]() {
-#pragma unroll 1
-    for (int i = 0; i < (kNClass + 1) * R; ++i) {
-      tab[i / R][i % R][0] = tab[i / R][i % R][1] = make_uint4(0u, 0u, 0u, 0u);
-      top[i / R][i % R] = make_uint2(0u, 0u);
-    }
+    held = 0u;
 #pragma unroll
     for (int q = 0; q < 3; ++q)
 #pragma unroll
@@ -323,17 +323,21 @@ __global__ void __launch_bounds__(kThreads, kEpiCtas<R>) k_pt2(Params p0, Launch
 
   // the warp's sums and counters into the geometry's; then zero
   auto flush_geometry = [&]() {
+    const unsigned classes = __reduce_or_sync(kFull, held);
 #pragma unroll 1
     for (int i = 0; i < (kNClass + 1) * R; ++i) {
       const int c = i / R, m = i % R;
-      const uint2 t = top[c][m];
-      flush_fx(p, fx_of(tab[c][m][0], t.x), fx_tab(0, c, m));
-      flush_fx(p, fx_of(tab[c][m][1], t.y), fx_tab(1, c, m));
+      if (!((classes >> c) & 1u) || m >= p.metat) continue;
+      const bool mine = (held >> c) & 1u;
+      const uint2 t = mine ? top[c][m] : make_uint2(0u, 0u);
+      flush_fx(p, mine ? fx_of(tab[c][m][0], t.x) : Fx{}, fx_tab(0, c, m));
+      flush_fx(p, mine ? fx_of(tab[c][m][1], t.y) : Fx{}, fx_tab(1, c, m));
     }
 #pragma unroll
     for (int q = 0; q < 3; ++q)
 #pragma unroll
-      for (int m = 0; m < R; ++m) flush_fx(p, acc[q][m], fx_acc(q, m));
+      for (int m = 0; m < R; ++m)
+        if (m < p.metat) flush_fx(p, acc[q][m], fx_acc(q, m));
     unsigned long long it = ietat, db = __double_as_longlong(dpivot);
 #pragma unroll 1
     for (int o = 16; o > 0; o >>= 1) {
@@ -475,6 +479,14 @@ __global__ void __launch_bounds__(kThreads, kEpiCtas<R>) k_pt2(Params p0, Launch
           const int ct = class_of(m);
           if (ct < kNClass)
             atomicAdd(&sh.hn[wid][(kNClass + 1) * (1 + m) + (R == 1 ? cls : hist_class_hi(p, vil[m]))], (uint32_t)(1 + nmul));
+          if (!((held >> ct) & 1u)) {
+            held |= 1u << ct;
+#pragma unroll 1
+            for (int i = 0; i < R; ++i) {
+              tab[ct][i][0] = tab[ct][i][1] = make_uint4(0u, 0u, 0u, 0u);
+              top[ct][i] = make_uint2(0u, 0u);
+            }
+          }
           uint2 top2 = top[ct][m];
           Fx f = fx_of(tab[ct][m][0], top2.x);
           fx_add(f, tmp[m]);
