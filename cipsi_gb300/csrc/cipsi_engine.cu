@@ -298,6 +298,8 @@ struct cipsi_ctx {
   size_t scratch_blocks = 0;
   double* dgen_part = nullptr;
   size_t gen_part_cap = 0;
+  double* dgrad = nullptr;  // adjoint: small gradient buffers, grad_cap doubles
+  size_t grad_cap = 0;
   unsigned long long* dcounters = nullptr;  // kZeroWords: counters, exact sums, work and pool counters
   // (dred, dhist_tab and the counters are one allocation, in this order, so
   // that a result is one copy into hres, which is pinned)
@@ -540,7 +542,7 @@ void cipsi_ctx_destroy(cipsi_ctx* ctx) {
   leave_arena(ctx);
   dfree(ctx->deri64);
   dfree(ctx->deri_w);
-  dfree(ctx->dnb_j); dfree(ctx->dnb_em); dfree(ctx->dlr_ent); dfree(ctx->dgen_part);
+  dfree(ctx->dnb_j); dfree(ctx->dnb_em); dfree(ctx->dlr_ent); dfree(ctx->dgen_part); dfree(ctx->dgrad);
   dfree(ctx->dlr_e); dfree(ctx->dlrw_e); dfree(ctx->dlrw_jh);
   dfree(ctx->dred);
   if (ctx->hres) cudaFreeHost(ctx->hres);
@@ -1999,6 +2001,9 @@ int cipsi_record_digest(void* user, int64_t first, int64_t count, int32_t words,
 
 namespace {
 
+// gradient buffers up to this size stay with the context
+constexpr size_t kGradKeptBytes = (size_t)16 << 20;
+
 // The adjoint launch behind cipsi_run_pt2_adjoint (geri given) and
 // cipsi_run_pt2_adjoint_1e (geri null: no (pq|rs) gradient, the second pass
 // over singles only).  e2, when given, receives the E2 sums of the same pass.
@@ -2025,36 +2030,42 @@ int run_adjoint(cipsi_ctx* ctx, const cipsi_opts* o, const double* seed, double*
   const size_t nq = (size_t)5 * mt;
   if ((size_t)std::max(nunits, 1) * nq > ctx->gen_part_cap) {  // per-unit partial sums
     dfree(ctx->dgen_part);
+    ctx->gen_part_cap = 0;
+    CK(cudaMalloc(&ctx->dgen_part, (size_t)std::max(nunits, 1) * nq * sizeof(double)));
     ctx->gen_part_cap = (size_t)std::max(nunits, 1) * nq;
-    CK(cudaMalloc(&ctx->dgen_part, ctx->gen_part_cap * sizeof(double)));
   }
   CK(cudaMemsetAsync(ctx->dcounters, 0, kZeroWords * sizeof(unsigned long long), ctx->stream));
   CK(cudaMemsetAsync(ctx->dgen_part, 0, (size_t)std::max(nunits, 1) * nq * sizeof(double), ctx->stream));
-  // gradient buffers (this call only)
+  // gradient buffers, one after the other; those cleared come first.  A small
+  // set is kept for the next call: allocated and freed each time, it can take
+  // memory of the device's own for itself each time (16 orbitals, S = 60: 690 us
+  // a call, 560 with other small buffers beside it)
   const int stride = 3 * nt + 2 * n;
-  double *d_eri = nullptr, *d_F = nullptr, *d_J = nullptr, *d_K = nullptr, *d_f = nullptr, *d_sl = nullptr,
-         *d_roots = nullptr;
+  const bool one_e = geri == nullptr;
+  auto part = [](size_t doubles) { return (doubles + 31) / 32 * 32; };
+  const size_t n_eri = one_e ? 0 : part(ctx->ninte), n_t = part(nt), n_sl = part((size_t)grid * stride), n_r = part(3 * mt);
+  const size_t zeroed = n_eri + n_t + n_sl + n_r, all = zeroed + 2 * n_t + part(2 * n);
+  const bool kept = all * sizeof(double) <= kGradKeptBytes;
+  double* mem = nullptr;
   auto release = [&]() {
-    dfree(d_eri); dfree(d_F); dfree(d_J); dfree(d_K); dfree(d_f); dfree(d_sl); dfree(d_roots);
+    if (!kept) dfree(mem);
   };
   auto ck = [&](cudaError_t e, const char* what) {
     if (e == cudaSuccess) return 0;
     release();
     return fail(ctx, CIPSI_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
   };
-  const bool one_e = geri == nullptr;
-  if (!one_e && (rc = ck(cudaMalloc(&d_eri, (size_t)ctx->ninte * sizeof(double)), "cudaMalloc"))) return rc;
-  if ((rc = ck(cudaMalloc(&d_F, (size_t)nt * sizeof(double)), "cudaMalloc"))) return rc;
-  if ((rc = ck(cudaMalloc(&d_J, (size_t)nt * sizeof(double)), "cudaMalloc"))) return rc;
-  if ((rc = ck(cudaMalloc(&d_K, (size_t)nt * sizeof(double)), "cudaMalloc"))) return rc;
-  if ((rc = ck(cudaMalloc(&d_f, (size_t)2 * n * sizeof(double)), "cudaMalloc"))) return rc;
-  if ((rc = ck(cudaMalloc(&d_sl, (size_t)grid * stride * sizeof(double)), "cudaMalloc"))) return rc;
-  if ((rc = ck(cudaMalloc(&d_roots, (size_t)3 * mt * sizeof(double)), "cudaMalloc"))) return rc;
-  if (!one_e && (rc = ck(cudaMemsetAsync(d_eri, 0, (size_t)ctx->ninte * sizeof(double), ctx->stream), "memset")))
-    return rc;
-  if ((rc = ck(cudaMemsetAsync(d_F, 0, (size_t)nt * sizeof(double), ctx->stream), "memset"))) return rc;
-  if ((rc = ck(cudaMemsetAsync(d_sl, 0, (size_t)grid * stride * sizeof(double), ctx->stream), "memset"))) return rc;
-  if ((rc = ck(cudaMemsetAsync(d_roots, 0, (size_t)3 * mt * sizeof(double), ctx->stream), "memset"))) return rc;
+  if (kept && ctx->grad_cap < all) {
+    dfree(ctx->dgrad);
+    ctx->grad_cap = 0;
+    CK(cudaMalloc(&ctx->dgrad, all * sizeof(double)));
+    ctx->grad_cap = all;
+  }
+  if (!kept && (rc = ck(cudaMalloc(&mem, all * sizeof(double)), "cudaMalloc"))) return rc;
+  double* const d_eri = kept ? ctx->dgrad : mem;
+  double *const d_F = d_eri + n_eri, *const d_sl = d_F + n_t, *const d_roots = d_sl + n_sl;
+  double *const d_J = d_roots + n_r, *const d_K = d_J + n_t, *const d_f = d_K + n_t;
+  if ((rc = ck(cudaMemsetAsync(d_eri, 0, zeroed * sizeof(double), ctx->stream), "memset"))) return rc;
 
   Params p{};
   fill_params(ctx, o, pl, p);
