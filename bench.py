@@ -619,7 +619,7 @@ def run_adjoint_form(args, rank: int, world: int, local_rank: int):
 
 
 # ------------------------------------------------------------ GPU arm
-KERNEL_SOURCES = ["pt2_kernel.cuh", "pt2_common.cuh", "pt2_w1.cu", "pt2_w2.cu"]
+KERNEL_SOURCES = ["pt2_kernel.cuh", "pt2_common.cuh", "pt2_fwd.cuh", "pt2_epi.cuh", "pt2_w1.cu", "pt2_w2.cu", "pt2_epi.cu"]
 
 
 def kernel_sha() -> str:
@@ -631,7 +631,7 @@ def kernel_sha() -> str:
 
 
 def kernel_profile(workload: str):
-    """The ncu figures of k_pt2 on this workload (profiles/k_pt2_<workload>.json)
+    """The ncu figures of k_cand and k_pt2 on this workload (profiles/k_pt2_<workload>.json)
     when they were captured on the current kernel sources, else None."""
     path = os.path.join(ROOT, "profiles", f"k_pt2_{workload}.json")
     if not os.path.exists(path):
@@ -743,7 +743,7 @@ def run_gpu(args, rank: int, world: int, local_rank: int):
            + ncf * (1 + 1 + 4) + ncf * mt * 8 + 2 * n * 8)
     nsel = res["n_selected"]
     rec_bytes = 2 * W * 8 + 4 + 8 + mt * 8
-    d2h = 5 * mt * 8 + 8 * (10 + 1 + 10 + 10 * 8) + 2 * 10 * 8 * 8 + nsel * rec_bytes
+    d2h = 5 * mt * 8 + 8 * (8 + 1 + 10 + 10 * 8) + 2 * 10 * 8 * 8 + nsel * rec_bytes
     peak, peak_kind = measured_peaks()
     kms = statistics.mean(pt2_ms)
     nl = max(1, (r["launches"] - 1) // 4)  # k_cand + k_pt2 pairs per step (one per chunk)
@@ -765,15 +765,16 @@ def run_gpu(args, rank: int, world: int, local_rank: int):
             "gpu_launches": launches,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
-                         "kernel": "k_pt2", "peak_source": peak_kind, "launches_per_step": nl,
+                         "kernel": "k_cand + k_pt2", "peak_source": peak_kind, "launches_per_step": nl,
                          "algorithmic_bytes_per_launch": r["alg_bytes"] / nl,
                          "kernel_ms_per_launch": kms / nl,
                          "note": "achieved = algorithmic bytes of the E2 loop (integral, coefficient and "
-                                 "diagonal-term reads) / k_pt2 time (CUDA events around each chunk's launch on "
-                                 "its stream), against the measured HBM copy bandwidth; traffic: DRAM bytes per "
-                                 "k_pt2 launch, the mean over every launch of one step of this workload in a "
+                                 "diagonal-term reads) / time of both kernels (CUDA events around each chunk's "
+                                 "launches), against the measured HBM copy bandwidth; traffic: DRAM bytes per "
+                                 "chunk, the mean over every launch of one step of this workload in a "
                                  "single-pass ncu capture of this kernel build (null when the kernel changed "
-                                 "since); the kernel is bound by integer issue and latency, not HBM"},
+                                 "since); k_cand is bound by issue and latency, k_pt2 by the FP64 pipe, neither "
+                                 "by HBM"},
             "clocks": clk,
             "work": {"perturbers": r["n_processed"], "candidates": r["n_candidates"],
                      "compares": r["n_compares"], "pairs_1": r["n_pairs_1"], "pairs_2": r["n_pairs_2"],

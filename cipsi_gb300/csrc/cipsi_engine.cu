@@ -1,7 +1,8 @@
 // cipsi_engine.cu -- host side of the GB300 engine for the CIPSI second-order
 // perturbation / selection step: contexts, run planning, launches, results,
 // the batched multi-geometry launch and the allocation-free entry point.
-// The kernel itself is in pt2_kernel.cuh (algorithm described there).
+// The kernels are in pt2_fwd.cuh, pt2_epi.cuh (forward runs) and pt2_kernel.cuh
+// (adjoint and allocation-free run; the algorithm is described there).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -338,9 +339,8 @@ struct cipsi_ctx {
   unsigned long long last_plan_sig = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, evk = nullptr;  // evk: end of k_pt2
   long long last_launches = 0;
-  // launch tuning (cipsi_set_tuning): R blocks per work unit for generators
-  // of excitation rank >= 2 (those of rank 0 get one block per unit, rank 1 up to kLowChunk),
-  // and CTAs per SM (0 = as many as the shared-memory L_R size allows)
+  // launch tuning (cipsi_set_tuning): r_chunk, from which unit_blocks takes the
+  // blocks per work unit, and CTAs per SM (0 = as many as shared memory allows)
   int tune_r_chunk = 6;
   int tune_ctas = 0;
   // set by a batched run: the event that marks its end (fetch waits on it),
@@ -821,7 +821,7 @@ constexpr int kLowChunk = 8;
 // Blocks of removed electrons per work unit of the forward kernels.  k_cand's
 // warps take the blocks of a unit on their own, so a unit wants a few per warp:
 // 16 at the default r_chunk of 6 (2.7 r_chunk above it; r_chunk itself below,
-// where the caller asks for fine units).  At the default, when the run has few
+// where the caller asks for fine units).  From 6 on, when the run has few
 // blocks, no more than leaves six units per CTA, down to two blocks (37
 // orbitals, S = 334: 940 us at six, 1027 at eight).
 // (60 orbitals, S = 2001: 45.8 ms at 24, 45.5 at 16, 47.3 at 8, 55 at 60; one
@@ -1669,7 +1669,7 @@ int cipsi_run_pt2(cipsi_ctx* ctx, const cipsi_opts* opts, cipsi_result* res) {
 // cipsi_run_pt2_stream: the run in chunks of consecutive work units whose
 // candidate slots fit the record pool (a unit never selects more records
 // than it has slots), so any selection size runs in bounded device memory.
-// Per chunk, on the context stream: k_pt2 over the chunk's units, the unit
+// Per chunk, on the context stream: k_cand and k_pt2 over its units, the unit
 // scan and the gather into one of two device record buffers; the copy
 // stream then brings the chunk to a ring of two pinned host buffers piece
 // by piece, and the caller's consumer gets each piece, in record order,
@@ -1877,7 +1877,7 @@ int cipsi_run_pt2_stream(cipsi_ctx* ctx, const cipsi_opts* o, int64_t chunk_reco
     return CIPSI_OK;
   };
 
-  // k_pt2 of each chunk timed by a pair of events
+  // both kernels of each chunk timed by a pair of events
   std::vector<cudaEvent_t> kev(2 * (size_t)nchunks, nullptr);
   struct EvFree {
     std::vector<cudaEvent_t>& v;
@@ -2818,7 +2818,7 @@ int cipsi_run_pt2_static(cipsi_ctx* ctx, const cipsi_opts* o, cipsi_result* r) {
   }
   p.pertu_ref = pertu_ref ? 1 : 0;
   p.pertu_mono = pertu_mono ? 1 : 0;
-  // nb_j, nb_emask, lr_ent: grid x ncf entries each (k_pt2 indexes block b at
+  // nb_j, nb_emask, lr_ent: grid x ncf entries each (k_pt2_one indexes block b at
   // b * ncf), in three regions of grid * nb_stride >= grid * ncf * 8 bytes
   p.nb_j = reinterpret_cast<int32_t*>(nb0);
   p.nb_emask = reinterpret_cast<uint64_t*>(nb0 + (size_t)grid * nb_stride);

@@ -17,8 +17,8 @@ constexpr int kThreads = 256;
 constexpr int kMaxSym = 8;
 constexpr int kMaxElec = 64;
 constexpr int kMaxOrb = 128;
-constexpr int kRowCap = 128;  // adjoint: per-warp list of |K' \ j| = 2 entries holding a1
-constexpr int kHitCap = 8;    // adjoint: per-thread list of scan hits awaiting their matrix elements
+constexpr int kRowCap = 128;  // k_pt2_one: per-warp list of |K' \ j| = 2 entries holding a1
+constexpr int kHitCap = 8;    // k_pt2_one: per-thread list of scan hits awaiting their matrix elements
 
 // counters[] slots
 enum {
@@ -29,8 +29,6 @@ enum {
   C_NCMP,
   C_NP1,
   C_NP2,
-  C_ALGB,
-  C_LRFALLBACK,
   C_STAGE_OVF,  // candidates whose slot lay outside their unit's (must stay 0)
   C_NCOUNTERS
 };
@@ -69,16 +67,16 @@ struct Params {
   // scratch
   int32_t* nb_j;             // per block: ncf entries
   uint64_t* nb_emask;
-  uint64_t* lr_ent;          // per block: ncf compact L_R entries beyond lr_cap (adjoint kernel)
-  uint32_t* lr_e;            // per block: L_R of a block too long for one warp (forward kernel):
+  uint64_t* lr_ent;          // per block: ncf compact L_R entries beyond lr_cap (k_pt2_one)
+  uint32_t* lr_e;            // per block: L_R of a block too long for one warp (k_cand):
   uint2* lr_jh;              //   ncf entries each
   uint32_t* lrw_e;           // per block: 2 x kWarps x lrw_cap entries, the overflow of the warps' lists
   uint2* lrw_jh;
   int lrw_cap;
-  int lr_cap;                // shared-memory capacity of L_R (adjoint kernel)
+  int lr_cap;                // shared-memory capacity of L_R (k_pt2_one)
   int nb_stride;             // entries per block in nb_j / nb_emask / lr_ent
   // outputs
-  double* gen_part;          // nunits x (5 * metat): per-unit sums (adjoint kernel)
+  double* gen_part;          // nunits x (5 * metat): per-unit sums (k_pt2_one)
   unsigned long long* counters;
   unsigned long long* dpivot_bits;
   unsigned long long* hist_nom;      // nclass
@@ -109,7 +107,7 @@ struct Params {
   // (pq|rs) as doubles: the caller's FP64 integrals (derivative checks) or
   // the real*4 ones widened on the device; null = read the real*4 `eri`
   const double* eri64;
-  // adjoint launch (k_pt2<..., ADJ = true>): seeds dE/d e2mp[m], e2vp[m],
+  // adjoint launch (k_pt2_one<..., ADJ = true>): seeds dE/d e2mp[m], e2vp[m],
   // e2b[m] and the gradient outputs
   double seed_mp[kMaxRoots], seed_vp[kMaxRoots], seed_b[kMaxRoots];
   double* g_eri;    // ninte: dE/d(pq|rs) in the packed order

@@ -1,15 +1,17 @@
 #pragma once
-// pt2_kernel.cuh -- the perturbation / selection kernel k_pt2 of the GB300
-// engine (the work of cip/pertu.f + cip/diexcit.f); included by pt2_w1.cu and
-// pt2_w2.cu, which instantiate it for 1 and 2 words per spin string.
+// pt2_kernel.cuh -- bitstring helpers and matrix elements of every kernel, and
+// k_pt2_one, which does a whole run in one kernel (the work of cip/pertu.f +
+// cip/diexcit.f): the adjoint (pt2_adj.cu, pt2_adj_w2.cu), and the forward run
+// without records of the entry that allocates nothing (pt2_one.cu).  Ordinary
+// forward runs are k_cand and k_pt2 (pt2_fwd.cuh, pt2_epi.cuh).
 //
 // Algorithm (same perturber set, owners and weights as the reference, which
 // walks excitation lists one candidate at a time, cip/igene.f, pert1.f):
 //
 //   * S determinants are alpha/beta occupation bitstrings, W 64-bit words per
 //     spin (W = 1 for norb <= 64, 2 for norb <= 128).
-//   * One CTA owns one generator k at a time (persistent grid, atomic work
-//     queue).  It first gathers nb(k) = { j in S : degree(j,k) <= 4 } with the
+//   * One CTA owns some blocks of one generator k at a time (persistent grid,
+//     atomic work queue).  It first gathers nb(k) = { j in S : degree(j,k) <= 4 } with the
 //     mask of k's electrons that j lacks.
 //   * Candidates I = k - R + A are processed in blocks of fixed removed
 //     electrons R (|R| = 1 or 2).  For a block, L_R = { j in nb(k) :
@@ -28,8 +30,8 @@
 //     coefficients are converted once on the host from the reference's
 //     excitation-list phase, so <I|H|Psi>^2 is identical.
 //   * (pq|rs) are read as real*4 (as cip stores them, cip/reijkl.f:27) and
-//     widened to double; everything else is double.  E2 sums are Kahan
-//     compensated per thread and reduced in a fixed order (deterministic).
+//     widened to double; everything else is double.  k_pt2_one's E2 sums are
+//     Kahan compensated per thread and reduced in a fixed order (deterministic).
 
 #include <algorithm>
 #include <cmath>

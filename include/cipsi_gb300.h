@@ -70,7 +70,12 @@ typedef struct {
                          single perturbers (pertu.f:62-108)                   */
 } cipsi_opts;
 
-/* Results: the accumulators of COMMON /ic/ and /hist/ after pertu+diexcit. */
+/* Results: the accumulators of COMMON /ic/ and /hist/ after pertu+diexcit.
+   The sums (e2*, psi*, tab*) of cipsi_run_pt2, its asynchronous, streamed and
+   batched forms do not depend on the order of their terms: every bit of a term
+   between 2^-64 and 2^62 is added exactly; smaller ones, up to 32 at a time,
+   are added in FP64 first and their sum exactly down to 2^-127.  Only what is
+   smaller still, larger or not finite is added in FP64, in any order.         */
 typedef struct {
   double e2mp[CIPSI_MAX_ROOTS];  /* MP barycentric E2 (e2mp)                 */
   double e2vp[CIPSI_MAX_ROOTS];  /* EN eigenvalue E2 (e2vp)                  */
