@@ -7,11 +7,13 @@
 // A CTA owns one work unit at a time; its warps take contiguous parts of the
 // unit's slots, pick the candidates among them and run the epilogue on 32 at a
 // time.  What bounds it is the FP64 pipe, 16 cycles of an SM per warp
-// instruction on GB300, so the epilogue is written for few of those (24 + 14
-// per further root; 55 and 46 before): reciprocals from the hardware's
-// approximation and one third-order step, and sums in fixed point -- integer
-// adds, exact, so independent of the order in which warps and CTAs finish, and
-// the E2 sums are the class sums' totals.
+// instruction on GB300, so the epilogue is written for few of those (20 per
+// root; 26 counted per 32 perturbers with one root, partly filled warps and all,
+// and 55 in one kernel before): reciprocals from the hardware's approximation and
+// one third-order step, and sums in fixed point -- integer adds, exact, so
+// independent of the order in which warps and CTAs finish, and the E2 sums are
+// the class sums' totals.  60 orbitals, S = 2001, an eighth of the generators:
+// 3.08 ms, the FP64 pipe 82 % busy.
 #include "pt2_kernel.cuh"
 
 namespace cipsi_dev {
