@@ -1016,7 +1016,7 @@ int reserve_cand(cipsi_ctx* ctx, long long max_slots, long long all_slots, long 
   auto bytes = [&](long long slots) { return (size_t)((std::max(slots, 1ll) + 63) / 64 * 64) * sb; };
   const size_t need = bytes(max_slots), all = bytes(all_slots);
   const size_t own = ctx->cand_limit ? ctx->cand_limit : kCandOwnBytes;
-  ctx->cand_shared = !ctx->cand_limit && all > own;
+  ctx->cand_shared = !ctx->cand_limit && all > own && ctx->device < kMaxDevices;
   // larger when it has to be, or when the memory for it is free
   auto grows = [&](size_t bytes, size_t want) {
     return bytes < need || (bytes < want && cand_share(want) > bytes);

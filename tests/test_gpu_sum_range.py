@@ -59,3 +59,27 @@ def test_infinite_and_undefined_terms(tmp_path, engine_lib):
         got = ctx.run(inp.opts)
         assert np.isnan(got["e2vp"][0]) and np.isnan(got["psivp"][0])
         assert got["n_processed"] == base["n_processed"]
+
+
+def test_zero_denominators(tmp_path, engine_lib):
+    """A root whose MP energy is exactly a perturber's: infinite MP sums, EN sums
+    and the set of perturbers as they were."""
+    inp, roots = _load(tmp_path)
+    opts = engine.Opts.from_buffer_copy(inp.opts)
+    opts.tau, opts.ywdeg = -1.0, 0  # a record of every perturber
+    fmpb = np.round(roots["fmpb"] * 1024) / 1024  # sums of these are exact
+    with engine.Context(inp.dims) as ctx:
+        ctx.upload(inp)
+        ctx.set_roots(**dict(roots, fmpb=fmpb))
+        base = ctx.run(opts)
+        bits = ctx.selection_raw(base["n_selected"])["bits"]
+        norb, nocc = inp.dims.norb, inp.dims.noca
+        occ = np.unpackbits(np.ascontiguousarray(bits).view(np.uint8), axis=1, bitorder="little")
+        occ = np.concatenate([occ[:, :norb], occ[:, 64:64 + norb]], axis=1).astype(float)
+        hmp = (occ - np.tile(np.arange(norb) < nocc, 2)) @ fmpb
+        ctx.set_roots(**dict(roots, fmpb=fmpb, emp=hmp[len(hmp) // 2:][:1]))
+        got = ctx.run(opts)
+    assert np.isinf(got["e2mp"][0]) and np.isinf(got["psimp"][0])
+    assert got["n_processed"] == base["n_processed"] and got["n_selected"] == base["n_selected"]
+    for q in ("e2vp", "e2b", "psivp"):
+        np.testing.assert_allclose(got[q], base[q], rtol=2.0 ** -49, atol=0.0)
